@@ -47,17 +47,18 @@ __device__ __forceinline__ float warp_max_f32(float v) {
 // The reference's two-term fold (src/beam_search.c:43-47): certified fp32 evaluation first (same
 // interval argument as fast_lse.cuh: log1p(exp(-d)) in fp32 is within 2^-20.5 of the reference's
 // double value; if both ends of that interval round to the same float next to m, that float is
-// the reference's), value-exact routine otherwise.
-__device__ __forceinline__ float fold2(float x, float y, const ofx::TabRef t) {
+// the reference's).  Branch free; `sure` says whether the result is certain, and the caller goes to
+// the value-exact routine when it is not.
+__device__ __forceinline__ float fold2_fast(float x, float y, bool &sure) {
     const float d = fabsf(x - y);
     const float m = x > y ? x : y;
-    if (!(d < 17.0f)) return m;
     const float e = ofd::ex2_approx(-d * 1.4426950408889634f);
     const float l = ofd::lg2_approx(1.0f + e) * 0.6931471805599453f;
     const float eps = 6.75e-7f;  // 2^-20.5
     const float lo = m + (l - eps), hi = m + (l + eps);
-    if (lo == hi && fabsf(lo) < 3.0e38f) return lo;
-    return ofx::fold2_exact(x, y, t);
+    const bool adds = d < 17.0f;
+    sure = !adds || (lo == hi && fabsf(lo) < 3.0e38f);
+    return adds ? lo : m;
 }
 
 // CRC32C over two input bits, table form of src/beam_search.c:103-115:
@@ -84,37 +85,45 @@ __device__ __forceinline__ uint32_t crc32c_bits(uint32_t crc, uint32_t v, int n)
     return crc;
 }
 
-template <int NS, int RING>
+// Number of entries of the owner table; 32 elements land on distinct ones in all but 11 % of the timesteps.
+constexpr int kOwner = 4096;
+
+// GROUP timesteps share an mbarrier pair (fewer waits and releases on the beam warp's chain), STAGES
+// such groups make the ring.
+template <int NS, int STAGES, int GROUP>
 struct BeamSmem {
     static constexpr int kScoreRow = NS * 8;  // bytes of one fp16 score row
     static constexpr int kBwdRow = NS * 4;    // bytes of one fp32 backward row
-    alignas(16) uint4 rec[kBeam];
-    alignas(16) float cstep[kBeam * 4];
-    alignas(8) uint2 slot[2 * kBeam];  // compaction (+ one spare per lane): {score, parent slot | stay << 5 | base << 6}
-    unsigned char owner[8192 + 32];    // (+ one spare per lane) hash -> slot + 1 of the beam element owning it
+    static constexpr int kSlot = kScoreRow + kBwdRow;
+    // The beam: {score, hash, k-mer | back-pointer << 16, score before the subtraction}.  Only 32
+    // elements live on; the room behind them is for the survivors beyond the 32nd in a timestep that
+    // runs out of bisection guesses.
+    alignas(16) uint4 rec[5 * kBeam];
+    alignas(16) float4 step[kBeam];           // step scores of the timestep's candidates, by parent slot
+    unsigned char owner[kOwner + 32];         // (+ one spare per lane) hash -> slot + 1 of the beam element owning it
     int init_state[kBeam];
     double exp2_j[ofx::kExpTab];
     double rcp_c[ofx::kLogTab];
     double log_c[ofx::kLogTab];
-    alignas(8) uint64_t full[RING];
-    alignas(8) uint64_t empty[RING];
+    alignas(8) uint64_t full[STAGES];
+    alignas(8) uint64_t empty[STAGES];
     int abort_flag;
-    alignas(128) unsigned char score_ring[RING][kScoreRow];
-    alignas(128) unsigned char bwd_ring[RING][kBwdRow];
+    // slot of timestep t: score row t, then backward row t+1
+    alignas(128) unsigned char ring[STAGES * GROUP][kSlot];
 };
 
-template <int NS, int RING>
+template <int NS, int STAGES, int GROUP, bool SCALED>
 __global__ void __launch_bounds__(kBeamBlock)
 beam_search_kernel(const OfDecodeArgs a) {
     constexpr int BITS = (NS == 64) ? 6 : (NS == 256 ? 8 : 10);
     constexpr int MSB = NS / 4;
     constexpr int NT = kBeamBlock;
-    using Smem = BeamSmem<NS, RING>;
+    using Smem = BeamSmem<NS, STAGES, GROUP>;
     extern __shared__ unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (known to be the same for a whole warp)
     const int lane = tid & 31;
     const int chunk = blockIdx.x;
     const int T = a.T, N = a.N;
@@ -123,11 +132,10 @@ beam_search_kernel(const OfDecodeArgs a) {
         sm.rcp_c[i] = a.tables->rcp_c[i];
         sm.log_c[i] = a.tables->log_c[i];
     }
-    for (int i = tid; i < 2048 + 8; i += NT) reinterpret_cast<uint32_t *>(sm.owner)[i] = 0;
-    for (int i = tid; i < kBeam * 4; i += NT) sm.cstep[i] = __int_as_float(0x7fc00000);  // mailbox: NaN = empty
+    for (int i = tid; i < (kOwner + 32) / 4; i += NT) reinterpret_cast<uint32_t *>(sm.owner)[i] = 0;
     if (tid == 0) {
         sm.abort_flag = 0;
-        for (int r = 0; r < RING; ++r) {
+        for (int r = 0; r < STAGES; ++r) {
             ofd::mbar_init(&sm.full[r], 1);
             ofd::mbar_init(&sm.empty[r], 1);
         }
@@ -143,40 +151,45 @@ beam_search_kernel(const OfDecodeArgs a) {
         // ------------------------------------------------------------------ copy warp
         if (lane == 0) {
             // the beam search strides timesteps by N*C (src/decode_cpu.c:204,216)
-            const __half *beam_scores = a.scores + (size_t)chunk * NS * 4;
+            const __half *src = a.scores + (size_t)chunk * NS * 4;
+            const float *bwd_src = bwd_chunk + NS;
             const size_t beam_stride = (size_t)N * a.C;
-            int issued = 0;
-            for (int t = 0; t <= T; ++t, ++issued) {
-                const int slot = t % RING;
-                if (t >= RING)
-                    ofd::mbar_wait_bounded(&sm.empty[slot], (uint32_t)(t / RING - 1) & 1u,
-                                           &sm.abort_flag, a.status, a.wait_ns);
+            int issued = 0, stage = 0;
+            uint32_t parity = 1;  // (of the stage's previous release)
+            for (int t = 0; t < T; t += GROUP, ++issued) {
+                if (t >= STAGES * GROUP)
+                    ofd::mbar_wait_bounded(&sm.empty[stage], parity, &sm.abort_flag, a.status, a.wait_ns);
                 if (sm.abort_flag) break;
-                const uint32_t bytes = Smem::kBwdRow + (t < T ? Smem::kScoreRow : 0);
-                ofd::mbar_arrive_expect_tx(&sm.full[slot], bytes);
-                ofd::bulk_g2s(sm.bwd_ring[slot], bwd_chunk + (size_t)t * NS, Smem::kBwdRow, &sm.full[slot]);
-                if (t < T)
-                    ofd::bulk_g2s(sm.score_ring[slot], beam_scores + beam_stride * t, Smem::kScoreRow,
-                                  &sm.full[slot]);
+                const int rows = T - t < GROUP ? T - t : GROUP;
+                ofd::mbar_arrive_expect_tx(&sm.full[stage], rows * Smem::kSlot);
+                for (int r = 0; r < rows; ++r) {
+                    unsigned char *dst = sm.ring[stage * GROUP + r];
+                    ofd::bulk_g2s(dst + Smem::kScoreRow, bwd_src, Smem::kBwdRow, &sm.full[stage]);
+                    ofd::bulk_g2s(dst, src, Smem::kScoreRow, &sm.full[stage]);
+                    bwd_src += NS;
+                    src += beam_stride;
+                }
+                if (++stage == STAGES) {
+                    stage = 0;
+                    parity ^= 1u;
+                }
             }
             // after an abort: the newest copies get a bounded chance to land before the block retires
-            if (sm.abort_flag) ofd::mbar_drain_bounded(sm.full, RING, issued, a.wait_ns);
+            if (sm.abort_flag) ofd::mbar_drain_bounded(sm.full, STAGES, issued, a.wait_ns);
         }
         return;
     }
     // ------------------------------------------------------------------ beam warp
     const ofx::TabRef tr = {sm.exp2_j, 1, sm.rcp_c, sm.log_c};
     const uint32_t lt_mask = (1u << lane) - 1u;
-    ofd::mbar_wait_bounded(&sm.full[0], 0, &sm.abort_flag, a.status, a.wait_ns);
     // initial beam: first <= 32 states, in state order, reaching the 32nd largest bwd[0]
     // (src/beam_search.c:151-175).  Radix-select the 32nd largest key bit by bit.
     {
-        const float *b0 = reinterpret_cast<const float *>(sm.bwd_ring[0]);
         constexpr int PER = NS / 32;
         uint32_t key[PER];
 #pragma unroll
         for (int i = 0; i < PER; ++i)
-            key[i] = (uint32_t)ofd::float_order_key(b0[lane + 32 * i]) ^ 0x80000000u;
+            key[i] = (uint32_t)ofd::float_order_key(bwd_chunk[lane + 32 * i]) ^ 0x80000000u;
         uint32_t thr = 0;
         for (int bit = 31; bit >= 0; --bit) {
             const uint32_t cand = thr | (1u << bit);
@@ -197,130 +210,134 @@ beam_search_kernel(const OfDecodeArgs a) {
         }
         __syncwarp();
     }
-    int state = sm.init_state[lane];
-    uint32_t hash = crc32c_bits(0x12345678u, (uint32_t)state, 32);
-    float score = 0.f;
     int W = kBeam;
-    bp_chunk[lane] = (unsigned char)((state & 3) << 6);
+    {
+        const int state = sm.init_state[lane];
+        sm.rec[lane] = make_uint4(__float_as_uint(0.f), crc32c_bits(0x12345678u, (uint32_t)state, 32),
+                                  (uint32_t)state | (uint32_t)(state & 3) << 22, __float_as_uint(0.f));
+        a.init_kmers[(size_t)chunk * kBeam + lane] = state;  // for the traceback's benefit
+    }
+    __syncwarp();
 
+    // Bound: the chain of one timestep's dependent instructions in this one warp (two to three cycles
+    // an instruction), so the usual route is one long basic block up to the first count, and what
+    // happens in one timestep of six (a merge, two elements on one table entry) redoes the end of it.
+    unsigned char *bp = bp_chunk + lane;
+    const unsigned char *slot = sm.ring[0];
+    int stage = 0, in_group = 0;
+    uint32_t parity = 0;
+    ofd::mbar_wait_bounded(&sm.full[0], 0u, &sm.abort_flag, a.status, a.wait_ns);
     for (int t = 0; t < T; ++t) {
-        const int slot_a = t % RING, slot_b = (t + 1) % RING;
-        // row t was confirmed when it served as "next row" one step ago (or before the loop)
-        ofd::mbar_wait_bounded(&sm.full[slot_b], (uint32_t)((t + 1) / RING) & 1u, &sm.abort_flag, a.status, a.wait_ns);
-        const __half *srow = reinterpret_cast<const __half *>(sm.score_ring[slot_a]);
-        const float *brow = reinterpret_cast<const float *>(sm.bwd_ring[slot_b]);
+        const uint4 mine = sm.rec[lane];
         const bool act = lane < W;
+        // (idle slots hold a valid, stale k-mer: they read like everybody else, and a score of -inf
+        // voids their candidates)
+        const float score = act ? __uint_as_float(mine.x) : -INFINITY;
+        const uint32_t hash = mine.y;
+        const int state = (int)(mine.z & (uint32_t)(NS - 1));
         const int q = state & (MSB - 1);
         const int top = state >> (BITS - 2);
         const uint32_t b_own = (uint32_t)state & 3u;
 
         // duplicate-prefix detection (src/beam_search.c:281-316): a stay can only merge with a
         // step whose parent's hash is `need`.  Every element writes its slot number into an
-        // 8192-entry owner table indexed by its hash; a stay then finds the one candidate
-        // parent by a single look-up and confirms it by comparing the full hash.  If two
-        // elements landed on the same table entry the table cannot be trusted for this
-        // timestep and the exhaustive comparison below takes over.
-        const uint32_t need = crc_unstep2(hash, b_own);
-        // idle slots (lane >= W) use a private spare entry so that nothing here branches
-        const uint32_t own_at = act ? (hash & 8191u) : 8192u + lane;
+        // owner table indexed by its hash; a stay then finds the one candidate parent by a single
+        // look-up and confirms it by comparing the full hash.
+        // (idle slots use a private spare entry so that nothing here branches)
+        const uint32_t own_at = act ? (hash & (kOwner - 1)) : kOwner + lane;
         sm.owner[own_at] = (unsigned char)(lane + 1);
-        __syncwarp();
 
         // candidates: 4 steps (state' = 4q + b, column 16q + 4b + top) and the stay
+        const __half *sp = reinterpret_cast<const __half *>(slot) + 16 * q + top;
+        const float *brow = reinterpret_cast<const float *>(slot + Smem::kScoreRow);
+        const float4 bw = *reinterpret_cast<const float4 *>(brow + 4 * q);
+        const float bs = brow[state];
+        const __half s0 = sp[0], s1 = sp[4], s2 = sp[8], s3 = sp[12];
+        const uint32_t need = crc_unstep2(hash, b_own);
+        __syncwarp();
+        const int mine_back = sm.owner[own_at];
+        const int cand = sm.owner[need & (kOwner - 1)];
+        bp[0] = (unsigned char)(act ? mine.z >> 16 : 0u);  // back-pointer row t
+        bp += kBeam;
+        // the children's hashes (the CRC is linear: appending base b adds tab[b])
+        const uint32_t h0 = crc_step2(hash, 0u);
         float c0, c1, c2, c3, c4;
         {
-            // idle slots still hold a valid (stale) k-mer: they read like everybody else and
-            // their candidates are voided afterwards
-            const float4 bw = *reinterpret_cast<const float4 *>(brow + 4 * q);
-            const __half *sp = srow + 16 * q + top;
             // (float)score * score_scale, rounded before it is added (src/beam_search.c:233-234)
-            const float x0 = __fmul_rn(__half2float(sp[0]), a.score_scale), x1 = __fmul_rn(__half2float(sp[4]), a.score_scale);
-            const float x2 = __fmul_rn(__half2float(sp[8]), a.score_scale), x3 = __fmul_rn(__half2float(sp[12]), a.score_scale);
-            const float bs = brow[state];
-            c0 = __fadd_rn(__fadd_rn(score, x0), bw.x);
-            c1 = __fadd_rn(__fadd_rn(score, x1), bw.y);
-            c2 = __fadd_rn(__fadd_rn(score, x2), bw.z);
-            c3 = __fadd_rn(__fadd_rn(score, x3), bw.w);
+            auto scaled = [&](__half h) { return SCALED ? __fmul_rn(__half2float(h), a.score_scale) : __half2float(h); };
+            c0 = __fadd_rn(__fadd_rn(score, scaled(s0)), bw.x);
+            c1 = __fadd_rn(__fadd_rn(score, scaled(s1)), bw.y);
+            c2 = __fadd_rn(__fadd_rn(score, scaled(s2)), bw.z);
+            c3 = __fadd_rn(__fadd_rn(score, scaled(s3)), bw.w);
             c4 = __fadd_rn(__fadd_rn(score, a.stay), bs);
-            c0 = act ? c0 : -INFINITY;
-            c1 = act ? c1 : -INFINITY;
-            c2 = act ? c2 : -INFINITY;
-            c3 = act ? c3 : -INFINITY;
-            c4 = act ? c4 : -INFINITY;
         }
-        const int mine_back = sm.owner[own_at];
-        const int cand_raw = sm.owner[need & 8191u];
-        const int cand = act ? cand_raw : 0;
-        const uint32_t clash = __ballot_sync(0xffffffffu, mine_back != lane + 1);
+        // pruning threshold (src/beam_search.c:320-381): best - ln(beam_cut); if more than 32
+        // candidates pass, bisect towards 25..32 survivors for at most 9 further guesses.  The first
+        // of those guesses is known from the start and counted together with the threshold itself.
+        float best, cut, mid;
+        uint32_t both;
+        auto passing = [&](float th) {
+            return (uint32_t)((c0 >= th) + (c1 >= th) + (c2 >= th) + (c3 >= th) + (c4 >= th));
+        };
+        auto threshold = [&]() {
+            best = warp_max_f32(ofd::max3(ofd::max3(c0, c1, c2), c3, c4));
+            cut = __fsub_rn(best, a.log_beam_cut);
+            mid = __fmul_rn(__fadd_rn(cut, best), 0.5f);
+            both = __reduce_add_sync(0xffffffffu, passing(cut) + (passing(mid) << 16));
+        };
         const uint32_t cand_hash = __shfl_sync(0xffffffffu, hash, (cand - 1) & 31);
-        int mate = (cand > 0 && cand_hash == need) ? cand - 1 : -1;
-        __syncwarp();
+        int mate = (act && cand > 0 && cand_hash == need) ? cand - 1 : -1;
+        const bool odd = __any_sync(0xffffffffu, mate >= 0 || mine_back != lane + 1);
         sm.owner[own_at] = 0;
-
-        bool conflict = false;
-        if (clash) {
-            // exhaustive: for every stay that the table points anywhere, compare against
-            // all elements (the reference's semantics, all-pairs)
-            mate = -1;
-            unsigned long long claimed01 = 0ull, claimed23 = 0ull;
-            for (int i = 0; i < W; ++i) {
-                const uint32_t need_i = __shfl_sync(0xffffffffu, need, i);
-                const uint32_t b_i = __shfl_sync(0xffffffffu, b_own, i);
-                const uint32_t m = __ballot_sync(0xffffffffu, act && hash == need_i);
-                if (m) {
-                    if (m & (m - 1)) conflict = true;
-                    const int jj = __ffs(m) - 1;
-                    const unsigned long long bitpos = 1ull << (((b_i & 1u) << 5) + jj);
-                    unsigned long long &cl = (b_i & 2u) ? claimed23 : claimed01;
-                    if (cl & bitpos) conflict = true;
-                    cl |= bitpos;
-                    if (lane == i) mate = jj;
-                }
+        threshold();
+        if (__builtin_expect(odd, 0)) {
+            bool conflict = false;
+            // elements that found another on their table entry: the table does not know them, so
+            // every lane compares with each of them (one, nearly always)
+            for (uint32_t left = __ballot_sync(0xffffffffu, mine_back != lane + 1); left; left &= left - 1u) {
+                const int l = __ffs(left) - 1;
+                const uint32_t h = __shfl_sync(0xffffffffu, hash, l);
+                const uint32_t same = __ballot_sync(0xffffffffu, act && hash == h);
+                if (same & (same - 1u)) conflict = true;  // a hash that occurs twice in the beam
+                if (act && need == h) mate = l;
             }
-        }
-        if (__any_sync(0xffffffffu, mate >= 0)) {
-            if (!conflict) {
-                // every stay has at most one partner and no step has two: the folds are
-                // independent.  The stay fetches its partner's step score by shuffle, folds,
-                // and posts the partner's new score in a mailbox the partner reads.
-                const int src = mate >= 0 ? mate : lane;
-                const float y0 = __shfl_sync(0xffffffffu, c0, src), y1 = __shfl_sync(0xffffffffu, c1, src);
-                const float y2 = __shfl_sync(0xffffffffu, c2, src), y3 = __shfl_sync(0xffffffffu, c3, src);
+            const bool merges = __any_sync(0xffffffffu, mate >= 0);
+            if (merges) {
+                sm.step[lane] = make_float4(c0, c1, c2, c3);
+                __syncwarp();
+            }
+            if (merges && !conflict) {
+                // every stay has at most one partner and no step has two: the folds are independent.
+                // The stay reads its partner's step score, folds, and puts the partner's new score back.
+                float *theirs = reinterpret_cast<float *>(&sm.step[mate >= 0 ? mate : lane]) + b_own;
+                const float x = c4, y = *theirs;
+                bool sure;
+                float f = fold2_fast(x, y, sure);
                 if (mate >= 0) {
-                    const float x = c4;
-                    const float y = b_own == 0 ? y0 : (b_own == 1 ? y1 : (b_own == 2 ? y2 : y3));
-                    const float f = fold2(x, y, tr);
+                    if (!sure) f = ofx::fold2_exact(x, y, tr);
                     const bool stay_wins = x > y;
                     c4 = stay_wins ? f : -FLT_MAX;
-                    sm.cstep[4 * mate + b_own] = stay_wins ? -FLT_MAX : f;
+                    *theirs = stay_wins ? -FLT_MAX : f;
                 }
-                __syncwarp();
-                const float4 r = *reinterpret_cast<const float4 *>(&sm.cstep[4 * lane]);
-                c0 = isnan(r.x) ? c0 : r.x;
-                c1 = isnan(r.y) ? c1 : r.y;
-                c2 = isnan(r.z) ? c2 : r.z;
-                c3 = isnan(r.w) ? c3 : r.w;
-                __syncwarp();
-                if (mate >= 0) sm.cstep[4 * mate + b_own] = __int_as_float(0x7fc00000);
-            } else {
+            } else if (merges) {
                 // repeated hashes inside the beam (CRC collisions): replay the reference's
                 // nested loop, stay-major then slot-minor, on one lane
-                *reinterpret_cast<float4 *>(&sm.cstep[4 * lane]) = make_float4(c0, c1, c2, c3);
                 sm.rec[lane] = make_uint4(hash, b_own, __float_as_uint(c4), 0u);
                 __syncwarp();
                 if (lane == 0) {
+                    float *cstep = reinterpret_cast<float *>(sm.step);
                     for (int i = 0; i < W; ++i) {
                         const uint32_t h_i = sm.rec[i].x, b_i = sm.rec[i].y;
                         for (int jj = 0; jj < W; ++jj) {
                             if (h_i != crc_step2(sm.rec[jj].x, b_i)) continue;
                             const float x = __uint_as_float(sm.rec[i].z);
-                            const float y = sm.cstep[4 * jj + b_i];
+                            const float y = cstep[4 * jj + b_i];
                             const float f = ofx::fold2_exact(x, y, tr);
                             if (x > y) {
                                 sm.rec[i].z = __float_as_uint(f);
-                                sm.cstep[4 * jj + b_i] = -FLT_MAX;
+                                cstep[4 * jj + b_i] = -FLT_MAX;
                             } else {
-                                sm.cstep[4 * jj + b_i] = f;
+                                cstep[4 * jj + b_i] = f;
                                 sm.rec[i].z = __float_as_uint(-FLT_MAX);
                             }
                         }
@@ -328,124 +345,113 @@ beam_search_kernel(const OfDecodeArgs a) {
                 }
                 __syncwarp();
                 if (act) c4 = __uint_as_float(sm.rec[lane].z);
-                const float4 r = *reinterpret_cast<const float4 *>(&sm.cstep[4 * lane]);
-                c0 = r.x; c1 = r.y; c2 = r.z; c3 = r.w;
+            }
+            if (merges) {
                 __syncwarp();
-                *reinterpret_cast<float4 *>(&sm.cstep[4 * lane]) =
-                    make_float4(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000),
-                                __int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+                const float4 r = sm.step[lane];
+                c0 = r.x; c1 = r.y; c2 = r.z; c3 = r.w;
+                threshold();
             }
         }
-
-        // pruning threshold (src/beam_search.c:320-381): best - ln(beam_cut); if more than 32
-        // candidates pass, bisect towards 25..32 survivors for at most 9 further guesses
-        const float best = warp_max_f32(ofd::max3(ofd::max3(c0, c1, c2), c3, c4));
-        float cut = __fsub_rn(best, a.log_beam_cut);
-        auto count_at_least = [&](float th) {
-            const int n = (c0 >= th) + (c1 >= th) + (c2 >= th) + (c3 >= th) + (c4 >= th);
-            return __reduce_add_sync(0xffffffffu, n);
-        };
-        int kept = count_at_least(cut);
+        int kept = (int)(both & 0xffffu);
         if (kept > kBeam) {
             float lo = cut, hi = best;
-            int guesses = 1;
-            while ((kept > kBeam || kept < 25) && guesses < 10) {
-                if (kept > kBeam) {
-                    lo = cut;
-                    cut = __fmul_rn(__fadd_rn(cut, hi), 0.5f);
-                } else {
-                    hi = cut;
-                    cut = __fmul_rn(__fadd_rn(cut, lo), 0.5f);
-                }
-                kept = count_at_least(cut);
+            cut = mid;
+            kept = (int)(both >> 16);
+            // (unrolled: a vote or reduction inside a loop costs a hundred cycles of re-convergence)
+            int guesses = 2;
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                if (kept <= kBeam && kept >= 25) break;
+                const bool many = kept > kBeam;
+                lo = many ? cut : lo;
+                hi = many ? hi : cut;
+                cut = __fmul_rn(__fadd_rn(cut, many ? hi : lo), 0.5f);
+                kept = (int)__reduce_add_sync(0xffffffffu, passing(cut));
                 ++guesses;
             }
             if (guesses == 10) {
                 cut = hi;
-                kept = count_at_least(cut);
+                kept = (int)__reduce_add_sync(0xffffffffu, passing(cut));
             }
-            kept = min(kept, kBeam);
         }
-        const uint32_t B0 = __ballot_sync(0xffffffffu, c0 >= cut), B1 = __ballot_sync(0xffffffffu, c1 >= cut);
-        const uint32_t B2 = __ballot_sync(0xffffffffu, c2 >= cut), B3 = __ballot_sync(0xffffffffu, c3 >= cut);
-        const uint32_t B4 = __ballot_sync(0xffffffffu, c4 >= cut);
 
-        // survivors keep candidate order: steps (slot-major, base-minor), then stays.  Each
-        // survivor drops {score, parent slot | stay | base} at its new slot; the new owner
-        // fetches the parent's hash and k-mer by shuffle and extends them itself.
+        // survivors keep candidate order: steps (slot-major, base-minor), then stays.  Every
+        // survivor goes to its new slot complete: score less the backward score, hash, k-mer and
+        // back-pointer, so that the next timestep starts with one read.
         {
-            int p = (__popc(B0 & lt_mask) + __popc(B1 & lt_mask)) + (__popc(B2 & lt_mask) + __popc(B3 & lt_mask));
-            const int nsteps = (__popc(B0) + __popc(B1)) + (__popc(B2) + __popc(B3));
-            // a survivor beyond the 32nd, and every non-survivor, writes into a spare slot
-            // of its own instead of branching around the store
-            const uint32_t bit = 1u << lane;
-            const int spare = kBeam + lane;
-            const bool k0 = (B0 & bit) != 0, k1 = (B1 & bit) != 0, k2 = (B2 & bit) != 0, k3 = (B3 & bit) != 0;
-            const int p0 = p, p1 = p0 + k0, p2 = p1 + k1, p3 = p2 + k2;
-            sm.slot[(k0 && p0 < kBeam) ? p0 : spare] = make_uint2(__float_as_uint(c0), lane | (0u << 6));
-            sm.slot[(k1 && p1 < kBeam) ? p1 : spare] = make_uint2(__float_as_uint(c1), lane | (1u << 6));
-            sm.slot[(k2 && p2 < kBeam) ? p2 : spare] = make_uint2(__float_as_uint(c2), lane | (2u << 6));
-            sm.slot[(k3 && p3 < kBeam) ? p3 : spare] = make_uint2(__float_as_uint(c3), lane | (3u << 6));
-            const int ps = nsteps + __popc(B4 & lt_mask);
-            sm.slot[((B4 & bit) && ps < kBeam) ? ps : spare] = make_uint2(__float_as_uint(c4), lane | 32u | (b_own << 6));
+            const bool k0 = c0 >= cut, k1 = c1 >= cut, k2 = c2 >= cut, k3 = c3 >= cut, k4 = c4 >= cut;
+            const uint32_t B0 = __ballot_sync(0xffffffffu, k0), B1 = __ballot_sync(0xffffffffu, k1);
+            const uint32_t B2 = __ballot_sync(0xffffffffu, k2), B3 = __ballot_sync(0xffffffffu, k3);
+            const uint32_t B4 = __ballot_sync(0xffffffffu, k4);
+            uint4 *to = sm.rec + ((__popc(B0 & lt_mask) + __popc(B1 & lt_mask)) + (__popc(B2 & lt_mask) + __popc(B3 & lt_mask)));
+            uint4 *to4 = sm.rec + (kept - __popc(B4 & ~lt_mask));
+            const uint32_t word = (uint32_t)(4 * q) | (uint32_t)lane << 16;
+            if (k0) *to = make_uint4(__float_as_uint(__fsub_rn(c0, bw.x)), h0, word, __float_as_uint(c0));
+            to += k0;
+            if (k1) *to = make_uint4(__float_as_uint(__fsub_rn(c1, bw.y)), h0 ^ crc_tab2(1u), word | (1u | 1u << 22), __float_as_uint(c1));
+            to += k1;
+            if (k2) *to = make_uint4(__float_as_uint(__fsub_rn(c2, bw.z)), h0 ^ crc_tab2(2u), word | (2u | 2u << 22), __float_as_uint(c2));
+            to += k2;
+            if (k3) *to = make_uint4(__float_as_uint(__fsub_rn(c3, bw.w)), h0 ^ crc_tab2(3u), word | (3u | 3u << 22), __float_as_uint(c3));
+            if (k4) *to4 = make_uint4(__float_as_uint(__fsub_rn(c4, bs)), hash, (uint32_t)state | (uint32_t)(lane | 32) << 16 | b_own << 22, __float_as_uint(c4));
         }
+        W = min(kept, kBeam);
         __syncwarp();
-        W = kept;
-        const uint2 mine = sm.slot[lane];
-        uint32_t meta = lane < W ? mine.y : 0u;
-        const uint32_t ph = __shfl_sync(0xffffffffu, hash, meta & 31u);
-        const int pst = __shfl_sync(0xffffffffu, state, meta & 31u);
-        {
-            const bool live = lane < W, stayed = (meta & 32u) != 0;
-            const uint32_t h_step = crc_step2(ph, meta >> 6);
-            const int s_step = ((pst << 2) & (NS - 1)) | (int)(meta >> 6);
-            score = live ? __uint_as_float(mine.x) : score;
-            hash = live ? (stayed ? ph : h_step) : hash;
-            state = live ? (stayed ? pst : s_step) : state;
+        slot += Smem::kSlot;
+        if (++in_group == GROUP) {
+            // the group's rows have been read by every lane
+            in_group = 0;
+            ofd::mbar_arrive_if(lane == 0, &sm.empty[stage]);
+            if (++stage == STAGES) {
+                stage = 0;
+                slot = sm.ring[0];
+                parity ^= 1u;
+            }
+            if (t + 1 < T && !ofd::mbar_try_wait(&sm.full[stage], parity))
+                ofd::mbar_wait_slow(&sm.full[stage], parity, &sm.abort_flag, a.status, a.wait_ns);
         }
-        if (t == T - 1) {
-            // best survivor swaps into slot 0 (src/beam_search.c:398-414)
-            const float sc = lane < W ? score : -INFINITY;
-            const float top_s = warp_max_f32(sc);
-            const uint32_t eq = __ballot_sync(0xffffffffu, lane < W && sc == top_s && sc > -FLT_MAX);
-            const int at = eq ? __ffs(eq) - 1 : 0;
-            const uint32_t h0 = __shfl_sync(0xffffffffu, hash, 0), ha = __shfl_sync(0xffffffffu, hash, at);
-            const int s0 = __shfl_sync(0xffffffffu, state, 0), sa = __shfl_sync(0xffffffffu, state, at);
-            const float v0 = __shfl_sync(0xffffffffu, score, 0), va = __shfl_sync(0xffffffffu, score, at);
-            const uint32_t m0_ = __shfl_sync(0xffffffffu, meta, 0), ma = __shfl_sync(0xffffffffu, meta, at);
-            if (lane == at) { hash = h0; state = s0; score = v0; meta = m0_; }
-            if (lane == 0) { hash = ha; state = sa; score = va; meta = ma; }
-        }
-        {
-            const float back = brow[state];
-            score = lane < W ? __fsub_rn(score, back) : score;
-        }
-        bp_chunk[(size_t)(t + 1) * kBeam + lane] = (unsigned char)meta;
-        __syncwarp();
-        if (lane == 0) ofd::mbar_arrive(&sm.empty[slot_a]);
     }
-    // the initial k-mers, for the traceback's benefit
-    a.init_kmers[(size_t)chunk * kBeam + lane] = sm.init_state[lane];
+    if (T > 0) {
+        // best survivor swaps into slot 0 (src/beam_search.c:398-414); of the last row only the
+        // back-pointers matter any more
+        const uint4 mine = sm.rec[lane];
+        const float sc = lane < W ? __uint_as_float(mine.w) : -INFINITY;
+        const float top_s = warp_max_f32(sc);
+        const uint32_t eq = __ballot_sync(0xffffffffu, lane < W && sc == top_s && sc > -FLT_MAX);
+        const int at = eq ? __ffs(eq) - 1 : 0;
+        uint32_t meta = lane < W ? mine.z >> 16 : 0u;
+        const uint32_t m0 = __shfl_sync(0xffffffffu, meta, 0), ma = __shfl_sync(0xffffffffu, meta, at);
+        if (lane == at) meta = m0;
+        if (lane == 0) meta = ma;
+        bp[0] = (unsigned char)meta;
+    }
 }
 
-template <int NS, int RING>
+template <int NS, int STAGES, int GROUP, bool SCALED>
 cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
-    using Smem = BeamSmem<NS, RING>;
+    using Smem = BeamSmem<NS, STAGES, GROUP>;
     const size_t bytes = sizeof(Smem) + 128;
-    auto kern = beam_search_kernel<NS, RING>;
+    auto kern = beam_search_kernel<NS, STAGES, GROUP, SCALED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
     kern<<<a.N, kBeamBlock, bytes, stream>>>(a);
     return cudaGetLastError();
 }
 
+// (a scale of one leaves every score as it is: no multiplication then)
+template <int NS, int STAGES, int GROUP>
+cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
+    return a.score_scale == 1.0f ? launch_beam<NS, STAGES, GROUP, false>(a, stream) : launch_beam<NS, STAGES, GROUP, true>(a, stream);
+}
+
 }  // namespace
 
 cudaError_t of_launch_beam_search(const OfDecodeArgs &a, cudaStream_t stream) {
     switch (a.state_len) {
-        case 3: return launch_beam<64, 8>(a, stream);
-        case 4: return launch_beam<256, 4>(a, stream);
-        case 5: return launch_beam<1024, 4>(a, stream);
+        case 3: return launch_beam<64, 2, 4>(a, stream);
+        case 4: return launch_beam<256, 2, 2>(a, stream);
+        case 5: return launch_beam<1024, 4, 1>(a, stream);
         default: return cudaErrorInvalidValue;
     }
 }

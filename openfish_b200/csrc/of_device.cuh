@@ -33,6 +33,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The same by the threads whose flag is set, without a branch.
+__device__ __forceinline__ void mbar_arrive_if(bool flag, uint64_t *bar) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%1];\n\t}"
+                 ::"r"((int)flag), "r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -77,6 +82,13 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t *bar, uint32_t parity
             }
         }
     }
+}
+
+// For a wait that nearly always finds its phase complete: the caller tries once and comes here only if
+// that failed; out of line so that its loop stays out of the caller's.
+static __device__ __noinline__ void mbar_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status,
+                                            uint64_t limit_ns) {
+    mbar_wait_bounded(bar, parity, abort_flag, status, limit_ns);
 }
 
 // After an abort: give the copies this thread issued last (the newest into each ring slot; copy
