@@ -119,8 +119,8 @@ beam_search_kernel(const OfDecodeArgs a) {
     constexpr int MSB = NS / 4;
     constexpr int NT = kBeamBlock;
     using Smem = BeamSmem<NS, STAGES, GROUP>;
-    extern __shared__ unsigned char smem_raw[];
-    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (known to be the same for a whole warp)
@@ -431,7 +431,7 @@ beam_search_kernel(const OfDecodeArgs a) {
 template <int NS, int STAGES, int GROUP, bool SCALED>
 cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
     using Smem = BeamSmem<NS, STAGES, GROUP>;
-    const size_t bytes = sizeof(Smem) + 128;
+    const size_t bytes = sizeof(Smem);
     auto kern = beam_search_kernel<NS, STAGES, GROUP, SCALED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;

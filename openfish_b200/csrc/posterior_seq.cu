@@ -67,8 +67,8 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     constexpr int NT = kPostThreads;
     constexpr int NWARP = NT / 32;
     using Smem = PostSmem<NS>;
-    extern __shared__ unsigned char smem_raw[];
-    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -286,7 +286,7 @@ cudaError_t launch_post(const OfDecodeArgs &a, cudaStream_t stream) {
     using Smem = PostSmem<NS>;
     const int Tp = (a.T + 16) & ~15;
     const size_t tail = (size_t)kWin * kBeam + (kWin / 8) * (kBeam + 4) + 8 * (size_t)Tp + 64;
-    const size_t bytes = sizeof(Smem) + tail + 128;
+    const size_t bytes = sizeof(Smem) + tail;
     if (bytes > 227 * 1024) return cudaErrorInvalidValue;
     auto kern = posterior_seq_kernel<NS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

@@ -348,7 +348,7 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
     constexpr int NW = Smem::NW, PER = Smem::kPerWarp;
     static_assert(!POST || Topo::kForward, "the posterior rides on the forward scan");
     static_assert(TPC % 32 == 0, "scan warps must be full");
-    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < ofx::kExpTab * kExpCopies; i += blockDim.x)
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(NS / SPT + 64, (NS <= 64 ? 8 : NS <= 256 ? 4 :
 scan_spec_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd,
                  int T, int N, int n_bwd_blocks, float stay, const ofx::Tables *__restrict__ tables,
                  int *status, uint64_t wait_ns) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     if ((int)blockIdx.x < n_bwd_blocks)
         spec_body<BwdTopo<NS>, NS, SPT, RING, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
                                                      status, wait_ns);
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(NS / SPT + 96, (NS <= 256 ? 5 : 2))
 scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__restrict__ bwd,
                            float *__restrict__ post, int T, int N, float stay,
                            const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     spec_body<FwdTopo<NS>, NS, SPT, RING, true>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
 }
 
@@ -662,7 +662,7 @@ template <int NS, int SPT, int RING>
 cudaError_t launch_spec(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
                         const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
     using Smem = SpecSmem<NS, SPT, RING, false>;
-    const size_t bytes = sizeof(Smem) + 128;
+    const size_t bytes = sizeof(Smem);
     auto kern = scan_spec_kernel<NS, SPT, RING>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
@@ -675,7 +675,7 @@ template <int NS, int SPT, int RING>
 cudaError_t launch_spec_posterior(const __half *scores, const float *bwd, float *post, int T, int N, float stay,
                                   const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
     using Smem = SpecSmem<NS, SPT, RING, true>;
-    const size_t bytes = sizeof(Smem) + 128;
+    const size_t bytes = sizeof(Smem);
     auto kern = scan_spec_posterior_kernel<NS, SPT, RING>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
