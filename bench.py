@@ -141,7 +141,7 @@ class ClockSampler(threading.Thread):
 
 def measure_rotary(of, dev, cpu_too=False):
     """openfish_rotary_emb_gpu on fp16 [32][1666][3][8][64] (Q and K heads in one call): device time
-    by the library's CUDA events on the legacy default stream the kernel runs on, rotating over four tensors
+    by the device's clock, first block to last, rotating over four tensors
     (655 MB) so that no call finds its input in the 126 MB L2."""
     import numpy as np
     import torch
@@ -161,7 +161,7 @@ def measure_rotary(of, dev, cpu_too=False):
         w0 = time.perf_counter()
         of.rotary_emb_gpu(xs[i % 4], sin, cos, *args)
         wall += time.perf_counter() - w0
-        total += of.last_rotary_ms()  # the library's own events around the kernel
+        total += of.last_rotary_ms()  # taken by the kernel itself
     ms = total / reps
     nbytes = 2 * B * S * 2 * H * D * 2 + 2 * S * half * 4
     peak, _ = measured_peak()

@@ -109,8 +109,8 @@ void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]);
  * submitted through openfish_b200_decode_submit_5wide (0 otherwise; not part of ms[3]). */
 void openfish_b200_last_decode_detail_ms(const openfish_gpubuf_t *gpubuf, float ms[8]);
 
-/* Device time, in milliseconds, of the calling thread's last openfish_rotary_emb_gpu call (CUDA
- * events on the legacy default stream around the kernel). */
+/* Device time, in milliseconds, of the calling thread's last openfish_rotary_emb_gpu call: from the start
+ * of the kernel's first block to the end of its last, by the device's clock. */
 float openfish_b200_last_rotary_ms(void);
 
 /* Self-check of the arithmetic the scans rely on.  Backward scores are made bit-identical to the

@@ -112,9 +112,10 @@ def lib():
 
 
 def _check():
-    st = lib().openfish_b200_last_status()
+    L = _lib or lib()
+    st = L.openfish_b200_last_status()
     if st != 0:
-        raise OpenfishError(st, lib().openfish_b200_error_text().decode())
+        raise OpenfishError(st, L.openfish_b200_error_text().decode())
 
 
 class _DevView:
@@ -281,9 +282,9 @@ def decode_wait(gpubuf):
 def rotary_emb_gpu(x_gpu, sin_gpu, cos_gpu, batch_size, seqlen, nheads, head_dim, rotary_half,
                    stride_batch, stride_seq, stride_head):
     """openfish_rotary_emb_gpu on torch CUDA tensors (x float16 in place, sin/cos float32)."""
-    lib().openfish_rotary_emb_gpu(x_gpu.data_ptr(), sin_gpu.data_ptr(), cos_gpu.data_ptr(),
-                                  batch_size, seqlen, nheads, head_dim, rotary_half, stride_batch,
-                                  stride_seq, stride_head)
+    (_lib or lib()).openfish_rotary_emb_gpu(x_gpu.data_ptr(), sin_gpu.data_ptr(), cos_gpu.data_ptr(),
+                                            batch_size, seqlen, nheads, head_dim, rotary_half, stride_batch,
+                                            stride_seq, stride_head)
     _check()
 
 

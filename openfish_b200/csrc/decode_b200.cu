@@ -16,6 +16,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "backend.h"
 #include "scan.cuh"
 #include "exact_math.cuh"
@@ -380,38 +383,85 @@ extern "C" int ofb_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[8]) 
     return OPENFISH_B200_OK;
 }
 
-// Device time of this thread's last rotary call: two events per device, made on first use.
+// Rotary: where a call's kernel reports its end.  A record belongs to one thread at a time; a thread
+// that ends leaves its record for the next one that needs one, so there are never more of them than
+// there have been threads at work at once.
 namespace {
 constexpr int kMaxDevices = 64;
-struct RotaryClock {
-    cudaEvent_t ev[kMaxDevices][2] = {};
-    bool made[kMaxDevices] = {};
-    float last_ms = 0.f;
+struct RotaryRecord {
+    RotaryDone *done;  // page-locked, portable: any device may write it
+    unsigned calls;
+    RotaryRecord *next;
 };
-thread_local RotaryClock t_rotary;
+std::mutex g_rotary_lock;
+RotaryRecord *g_rotary_free = nullptr;
+std::atomic<int> g_sms[kMaxDevices];
+
+struct RotaryThread {
+    RotaryRecord *mine = nullptr;
+    float last_ms = 0.f;
+    ~RotaryThread() {
+        if (!mine) return;
+        std::lock_guard<std::mutex> hold(g_rotary_lock);
+        mine->next = g_rotary_free;
+        g_rotary_free = mine;
+    }
+};
+thread_local RotaryThread t_rotary;
+
+int rotary_record(RotaryRecord **out) {
+    if (!t_rotary.mine) {
+        std::lock_guard<std::mutex> hold(g_rotary_lock);
+        if (g_rotary_free) {
+            t_rotary.mine = g_rotary_free;
+            g_rotary_free = g_rotary_free->next;
+        } else {
+            RotaryDone *d = nullptr;
+            CU(cudaHostAlloc(&d, sizeof(RotaryDone), cudaHostAllocPortable | cudaHostAllocMapped));
+            memset(d, 0, sizeof(*d));
+            RotaryRecord *r = static_cast<RotaryRecord *>(calloc(1, sizeof(RotaryRecord)));
+            if (!r) {
+                cudaFreeHost(d);
+                return fail(OPENFISH_B200_ERR_ALLOC, "out of host memory");
+            }
+            r->done = d;
+            t_rotary.mine = r;
+        }
+    }
+    *out = t_rotary.mine;
+    return OPENFISH_B200_OK;
+}
 }  // namespace
 
 extern "C" int ofb_rotary(void *x, const void *sin_t, const void *cos_t, int batch, int seqlen,
                           int nheads, int rotary_half, long long stride_batch,
                           long long stride_seq, long long stride_head) {
-    int dev = 0, sms = 0;
-    CU(cudaGetDevice(&dev));
-    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const bool timed = dev >= 0 && dev < kMaxDevices;
-    if (timed && !t_rotary.made[dev]) {
-        CU(cudaEventCreate(&t_rotary.ev[dev][0]));
-        CU(cudaEventCreate(&t_rotary.ev[dev][1]));
-        t_rotary.made[dev] = true;
-    }
-    // the reference launches on the legacy default stream and waits for the device
-    // (src/nn_cuda.cu:27-39); same stream here, and a wait on that stream only
-    if (timed) CU(cudaEventRecord(t_rotary.ev[dev][0], 0));
-    CU(of_launch_rotary(x, sin_t, cos_t, batch, seqlen, nheads, rotary_half, stride_batch,
-                        stride_seq, stride_head, sms, 0));
-    if (timed) CU(cudaEventRecord(t_rotary.ev[dev][1], 0));
-    CU(cudaStreamSynchronize(0));
     t_rotary.last_ms = 0.f;
-    if (timed) CU(cudaEventElapsedTime(&t_rotary.last_ms, t_rotary.ev[dev][0], t_rotary.ev[dev][1]));
+    if ((long long)batch * seqlen * nheads * rotary_half <= 0) return OPENFISH_B200_OK;
+    int dev = 0;
+    CU(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) return fail(OPENFISH_B200_ERR_ARGUMENT, "device %d out of range", dev);
+    int sms = g_sms[dev].load(std::memory_order_relaxed);
+    if (!sms) {
+        CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        g_sms[dev].store(sms, std::memory_order_relaxed);
+    }
+    RotaryRecord *r = nullptr;
+    const int rc = rotary_record(&r);
+    if (rc != OPENFISH_B200_OK) return rc;
+    const unsigned call = ++r->calls;
+    // the reference launches on the legacy default stream and waits for the device
+    // (src/nn_cuda.cu:27-39); same stream here, and a wait for this kernel only
+    CU(of_launch_rotary(x, sin_t, cos_t, batch, seqlen, nheads, rotary_half, stride_batch,
+                        stride_seq, stride_head, sms, r->done, call, 0));
+    // The kernel's own report first (nothing is nearer); work queued before it may keep it for longer, and
+    // an error would keep it for good: then the stream is asked.
+    volatile unsigned *seen = &r->done->call;
+    for (int spin = 0; *seen != call && spin < 20000; ++spin) __builtin_ia32_pause();
+    if (*seen != call) CU(cudaStreamSynchronize(0));
+    if (*seen != call) return fail(OPENFISH_B200_ERR_CUDA, "the rotary kernel did not report its end");
+    std::atomic_thread_fence(std::memory_order_acquire);
+    t_rotary.last_ms = (float)((r->done->end_ns - r->done->start_ns) * 1e-6);
     return OPENFISH_B200_OK;
 }
 

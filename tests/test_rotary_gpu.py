@@ -58,6 +58,19 @@ def test_odd_shapes_take_the_scalar_path(native_lib, oracle_mod, B, S, H, D, hal
     assert close(out, ref)
 
 
+@pytest.mark.parametrize("B,S,H,D,half", [(3, 1999, 5, 80, 20), (1, 3, 1, 8, 4), (2, 700, 4, 40, 12)])
+def test_four_pairs_at_a_time(native_lib, oracle_mod, B, S, H, D, half):
+    # halves of a head that are no multiple of eight pairs but of four; more positions than one pass of
+    # the grid covers in the first case, a single thread's work in the second
+    rng = np.random.default_rng(B * 100 + S)
+    x = rng.standard_normal((B, S, H, D)).astype(np.float16)
+    sin, cos = tables(S, half)
+    out = run(native_lib, x, sin, cos, B, S, H, half, S * H * D, H * D, D)
+    ref = x.astype(np.float32).copy()
+    oracle_mod.rotary(ref.reshape(-1), sin, cos, half, S * H * D, H * D, D, B, S, H)
+    assert close(out, ref)
+
+
 def test_full_size_against_the_oracle(native_lib, oracle_mod):
     # the encoder's whole packed QKV tensor [32][1666][3][8][64] against
     # the CPU routine on the same fp16 values, every element
