@@ -98,15 +98,16 @@ void openfish_b200_decode_submit_5wide(void *cuda_stream, int T, int N, const vo
                                        char *qstring);
 
 /* Device time, in milliseconds, of the gpubuf's last completed decode, measured with CUDA
- * events on the streams the kernels ran on: ms[0] backward scan kernel, ms[1] everything between
- * it and the copies (the beam search kernel with the forward scan kernel beside it on a second
- * stream, then the posterior + traceback + sequence kernel), ms[2] device-to-host copies, ms[3]
- * all of it. */
+ * events on the streams the kernels ran on: ms[0] the scans that the beam search waits for (the
+ * backward one, in a small batch both), ms[1] everything between them and the copies (the beam search
+ * kernel with the rest of the way to the posterior beside it on a second stream, then the traceback
+ * + sequence kernel), ms[2] device-to-host copies, ms[3] all of it. */
 void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]);
 
-/* The same four numbers followed by: ms[4] beam search kernel, ms[5] forward scan kernel, ms[6]
- * posterior + traceback + sequence kernel, ms[7] the blank-column strip in front of a decode
- * submitted through openfish_b200_decode_submit_5wide (0 otherwise; not part of ms[3]). */
+/* The same four numbers followed by: ms[4] beam search kernel, ms[5] what ran beside it (forward scan
+ * and posterior, in a small batch the posterior alone), ms[6] traceback + sequence kernel, ms[7] the
+ * blank-column strip in front of a decode submitted through openfish_b200_decode_submit_5wide (0
+ * otherwise; not part of ms[3]). */
 void openfish_b200_last_decode_detail_ms(const openfish_gpubuf_t *gpubuf, float ms[8]);
 
 /* Device time, in milliseconds, of the calling thread's last openfish_rotary_emb_gpu call: from the start
@@ -137,7 +138,8 @@ int openfish_b200_selfcheck_arith(double err[2]);
  * the reference, whose kernels do not wait. */
 int openfish_b200_selfcheck_wait(const openfish_gpubuf_t *gpubuf, unsigned limit_us);
 
-/* Number of kernels one decode call launches (for benchmark bookkeeping). */
+/* Number of kernels one decode call launches (for benchmark bookkeeping; the 64-state model's larger
+ * batches launch one more). */
 int openfish_b200_kernels_per_decode(void);
 
 /* Decode without allocating anything, for callers that cannot let a library allocate once they

@@ -1,4 +1,4 @@
-// beam_post.cuh -- launchers of the beam search kernel (beam_search.cu) and of the posterior +
+// beam_post.cuh -- launchers of the beam search kernel (beam_search.cu) and of the
 // traceback + sequence kernel (posterior_seq.cu).
 #pragma once
 #include <cuda_fp16.h>
@@ -9,9 +9,7 @@ namespace ofx { struct Tables; }
 struct OfDecodeArgs {
     const __half *scores;      // [T][N][C] fp16, 16-byte aligned, C % 8 == 0, C >= 4*ns
     const float *bwd;          // [N][T+1][ns], from the backward scan
-    const float *fwd;          // [N][T+1][ns], from the forward scan (posterior kernel only); null when
-                               // the forward scan has already written the posterior into `post`
-    float *post;               // [N][T+1][ns] out
+    const float *post;         // [N][T+1][ns], from the forward scan
     unsigned char *bp;         // [N][T+1][32] packed back-pointers: beam search -> traceback
     int *init_kmers;           // [N][32] k-mers of the initial beam: beam search -> traceback
     uint8_t *moves;            // [N][T] out
@@ -31,5 +29,5 @@ struct OfDecodeArgs {
 
 // needs scores, bwd; writes bp, init_kmers
 cudaError_t of_launch_beam_search(const OfDecodeArgs &a, cudaStream_t stream);
-// needs bwd, fwd, bp, init_kmers; writes post and every output
+// needs post, bp, init_kmers; writes every output
 cudaError_t of_launch_posterior_seq(const OfDecodeArgs &a, cudaStream_t stream);

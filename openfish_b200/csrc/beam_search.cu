@@ -25,6 +25,7 @@
 #include "exact_math.cuh"
 #include "fast_lse.cuh"
 #include "of_device.cuh"
+#include "prepare.cuh"
 
 namespace {
 
@@ -429,29 +430,43 @@ beam_search_kernel(const OfDecodeArgs a) {
 }
 
 template <int NS, int STAGES, int GROUP, bool SCALED>
-cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
-    using Smem = BeamSmem<NS, STAGES, GROUP>;
-    const size_t bytes = sizeof(Smem);
-    auto kern = beam_search_kernel<NS, STAGES, GROUP, SCALED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    kern<<<a.N, kBeamBlock, bytes, stream>>>(a);
-    return cudaGetLastError();
-}
+struct Beam {
+    static constexpr auto kern = beam_search_kernel<NS, STAGES, GROUP, SCALED>;
+    static constexpr size_t bytes = sizeof(BeamSmem<NS, STAGES, GROUP>);
+    static cudaError_t launch(const OfDecodeArgs &a, cudaStream_t stream) {
+        kern<<<a.N, kBeamBlock, bytes, stream>>>(a);
+        return cudaGetLastError();
+    }
+};
+template <bool SCALED> using Beam64 = Beam<64, 2, 4, SCALED>;
+template <bool SCALED> using Beam256 = Beam<256, 2, 2, SCALED>;
+template <bool SCALED> using Beam1024 = Beam<1024, 4, 1, SCALED>;
 
 // (a scale of one leaves every score as it is: no multiplication then)
-template <int NS, int STAGES, int GROUP>
+template <template <bool> class B>
 cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
-    return a.score_scale == 1.0f ? launch_beam<NS, STAGES, GROUP, false>(a, stream) : launch_beam<NS, STAGES, GROUP, true>(a, stream);
+    return a.score_scale == 1.0f ? B<false>::launch(a, stream) : B<true>::launch(a, stream);
 }
 
 }  // namespace
 
 cudaError_t of_launch_beam_search(const OfDecodeArgs &a, cudaStream_t stream) {
     switch (a.state_len) {
-        case 3: return launch_beam<64, 2, 4>(a, stream);
-        case 4: return launch_beam<256, 2, 2>(a, stream);
-        case 5: return launch_beam<1024, 4, 1>(a, stream);
+        case 3: return launch_beam<Beam64>(a, stream);
+        case 4: return launch_beam<Beam256>(a, stream);
+        case 5: return launch_beam<Beam1024>(a, stream);
         default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t of_load_beam_search(int kernel) {
+    switch (kernel) {
+        case kBeam64: return of_load<Beam64<false>>();
+        case kBeam256: return of_load<Beam256<false>>();
+        case kBeam1024: return of_load<Beam1024<false>>();
+        case kBeam64Scaled: return of_load<Beam64<true>>();
+        case kBeam256Scaled: return of_load<Beam256<true>>();
+        case kBeam1024Scaled: return of_load<Beam1024<true>>();
+        default: return cudaSuccess;
     }
 }

@@ -3,9 +3,9 @@
 // Replaces gpubuf_init_cuda / gpubuf_free_cuda / decode_cuda (src/decode_cuda.cu:11-212).
 // Differences in design: the caller-visible openfish_gpubuf_t sits at the start of a private
 // record that also owns two streams, events, the arithmetic tables and a page-locked staging
-// area; one decode is four kernel launches -- backward scan; beam search with the forward scan
-// beside it on the second stream; posterior + traceback + sequence -- and one device-to-host
-// copy, all stream
+// area; one decode is four or five kernel launches -- the scans that the beam search waits for; beam
+// search with the rest of the way to the posterior beside it on the second stream; traceback +
+// sequence -- and one device-to-host copy, all stream
 // ordered, with a single host wait at the end (the reference launches five kernels and three
 // memsets with a device-wide synchronisation after each and copies with three blocking
 // pageable transfers).
@@ -24,6 +24,7 @@
 #include "exact_math.cuh"
 #include "beam_post.cuh"
 #include "of_device.cuh"
+#include "prepare.cuh"
 #include "openfish_b200.h"
 #include "rotary.cuh"
 
@@ -35,15 +36,13 @@ struct GpuBuf {
     openfish_gpubuf_t pub;  // must stay first: the public pointer is the record's address
     uint32_t magic;
     int T, N, state_len, device;
-    cudaStream_t stream;   // everything but the forward scan; blocking, see ofb_gpubuf_create
-    cudaStream_t stream2;  // the forward scan, ordered against `stream` by events only
+    cudaStream_t stream;   // the main one; blocking, see ofb_gpubuf_create
+    cudaStream_t stream2;  // what runs beside the beam search, ordered against `stream` by events only
     cudaEvent_t ev[9];     // 0 start, 1 bwd scan done, 2 beam search done, 3 sequence done, 4 copies done,
                            // 5 fwd scan start, 6 fwd scan done, 7 the caller's stream at submit time, 8 blank-column strip start
     uint64_t wait_ns;      // how long a kernel waits for an asynchronous copy before it raises d_status
     int *d_init_kmers;     // inside the beam_vector allocation, behind the back-pointers
     ofx::Tables *d_tables;
-    float *d_fwd;              // forward scores [N][T+1][ns]: scan kernel -> posterior kernel (64-state model
-                               // only; null otherwise: the forward scan kernel writes the posterior)
     int *d_status;
     void *d_scores4;           // 4-wide copy of 5-wide scores, made on the first 5-wide decode (null before)
     int sms;
@@ -104,7 +103,6 @@ int destroy(GpuBuf *g) {
     cudaFree(g->pub.base_probs);
     cudaFree(g->pub.total_probs);
     cudaFree(g->d_tables);
-    cudaFree(g->d_fwd);
     cudaFree(g->d_status);
     cudaFree(g->d_scores4);
     if (g->h_stage) cudaFreeHost(g->h_stage);
@@ -121,6 +119,27 @@ int destroy(GpuBuf *g) {
 
 }  // namespace
 
+// The kernels are loaded here, all at once and always in the same order, instead of each at its first
+// launch: kernels that run beside one another get in each other's way in the instruction caches according
+// to where their code has come to lie.  A 512-chunk decode of the 256-state model took 2.96 ms in a process
+// that began with one and 3.10 in one that had decoded 74 chunks before.
+cudaError_t of_prepare_device(int device) {
+    static std::mutex lock;
+    static bool loaded[64];
+    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> hold(lock);
+    if (loaded[device]) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < kKernels && e == cudaSuccess; ++k) {
+        e = of_load_scan(k);
+        if (e == cudaSuccess) e = of_load_ahead(k);
+        if (e == cudaSuccess) e = of_load_beam_search(k);
+        if (e == cudaSuccess) e = of_load_posterior_seq(k);
+    }
+    loaded[device] = e == cudaSuccess;
+    return e;
+}
+
 extern "C" const char *ofb_error_text(void) { return g_err; }
 
 extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t **out) {
@@ -133,6 +152,7 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
     const size_t tens = (size_t)N * (T + 1) * ns * sizeof(float);
     int rc = [&]() -> int {
         CU(cudaGetDevice(&g->device));
+        CU(of_prepare_device(g->device));
         CU(cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, g->device));
         // a blocking stream: ordered after work the caller queued on the legacy default
         // stream (where the reference runs), so freshly written scores are seen
@@ -144,8 +164,6 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
         // result arrays share one allocation so that one copy brings them back
         CU(cudaMalloc(&g->pub.bwd_NTC, tens));
         CU(cudaMalloc(&g->pub.post_NTC, tens));
-        // (models whose forward scan writes the posterior itself need no forward tensor)
-        if (!of_forward_posterior_fused(state_len)) CU(cudaMalloc(&g->d_fwd, tens));
         CU(cudaMalloc(&g->d_results, 3 * nt));
         g->pub.moves = g->d_results;
         g->pub.sequence = reinterpret_cast<char *>(g->d_results + nt);
@@ -219,7 +237,6 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     OfDecodeArgs a;
     a.scores = static_cast<const __half *>(scores);
     a.bwd = g->pub.bwd_NTC;
-    a.fwd = g->d_fwd;
     a.post = g->pub.post_NTC;
     a.bp = static_cast<unsigned char *>(g->pub.beam_vector);
     a.init_kmers = g->d_init_kmers;
@@ -240,9 +257,8 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     a.q_scale = q_scale;
     a.score_scale = params->score_scale;
 
-    // stream:  backward scan -> beam search ----------------------> posterior + sequence -> copies
-    // stream2:                  forward scan (beside the beam search) --^
-    // (for hac and sup the forward scan kernel also writes the posterior, and a.fwd is null)
+    // stream:  scans as far as the beam search needs them -> beam search -----> sequence -> copies
+    // stream2:                    the rest of the way to the posterior (beside it) --^
     // Ordering against the producer of the scores: the gpubuf's main stream is a blocking one, so it
     // runs after whatever the caller queued on the legacy default stream (the reference's stream);
     // a caller that works on a stream of its own names it, and the decode waits for that stream's
@@ -253,17 +269,14 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
         CU(cudaStreamWaitEvent(g->stream, g->ev[7], 0));
     }
     CU(cudaEventRecord(g->ev[0], g->stream));
-    CU(of_launch_scans(scores, g->pub.bwd_NTC, nullptr, T, N, state_len, blank_score, g->d_tables,
-                       g->d_status, g->wait_ns, g->stream));
+    const OfScanPlan plan = of_scan_plan(N, state_len, g->sms);
+    CU(of_launch_first_scans(plan, scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, g->sms, blank_score,
+                             g->d_tables, g->d_status, g->wait_ns, g->stream));
     CU(cudaEventRecord(g->ev[1], g->stream));
     CU(cudaStreamWaitEvent(g->stream2, g->ev[1], 0));
     CU(cudaEventRecord(g->ev[5], g->stream2));
-    if (of_forward_posterior_fused(state_len))
-        CU(of_launch_forward_posterior(scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, blank_score,
-                                       g->d_tables, g->d_status, g->wait_ns, g->stream2));
-    else
-        CU(of_launch_scans(scores, nullptr, g->d_fwd, T, N, state_len, blank_score, g->d_tables,
-                           g->d_status, g->wait_ns, g->stream2));
+    CU(of_launch_rest_of_posterior(plan, scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, g->sms, blank_score,
+                                   g->d_tables, g->d_status, g->wait_ns, g->stream2));
     CU(cudaEventRecord(g->ev[6], g->stream2));
     CU(of_launch_beam_search(a, g->stream));
     CU(cudaEventRecord(g->ev[2], g->stream));
@@ -339,10 +352,10 @@ extern "C" int ofb_decode_wait(const openfish_gpubuf_t *gpubuf) {
         memcpy(g->dst_sequence, g->h_stage + nt, nt);
         memcpy(g->dst_qstring, g->h_stage + 2 * nt, nt);
     }
-    // ms: 0 backward scan, 1 everything between it and the copies (beam search with the forward
-    // scan beside it, then posterior + sequence), 2 copies, 3 all of it; detail: 4 beam search,
-    // 5 forward scan, 6 posterior + sequence (from the later of its two inputs), 7 the blank-column
-    // strip in front of a 5-wide decode (0 otherwise)
+    // ms: 0 the scans before the beam search, 1 everything between them and the copies (beam search
+    // with the rest of the posterior beside it, then sequence), 2 copies, 3 all of it; detail: 4 beam
+    // search, 5 the rest of the posterior, 6 sequence (from the later of its two inputs), 7 the
+    // blank-column strip in front of a 5-wide decode (0 otherwise)
     cudaEventElapsedTime(&g->ms[0], g->ev[0], g->ev[1]);
     cudaEventElapsedTime(&g->ms[1], g->ev[1], g->ev[3]);
     cudaEventElapsedTime(&g->ms[2], g->ev[3], g->ev[4]);

@@ -30,6 +30,7 @@
 #include "exact_math.cuh"
 #include "beam_post.cuh"
 #include "of_device.cuh"
+#include "prepare.cuh"
 #include "openfish_b200.h"
 
 namespace {
@@ -65,10 +66,11 @@ int setup_device(int dev, unsigned char **base_out) {
         }
         ofx::Tables host_tables;
         ofx::fill_tables(&host_tables);
-        e = cudaMemcpy(p, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice);
+        e = of_prepare_device(dev);
+        if (e == cudaSuccess) e = cudaMemcpy(p, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             char msg[160];
-            snprintf(msg, sizeof(msg), "uploading the tables failed: %s", cudaGetErrorString(e));
+            snprintf(msg, sizeof(msg), "loading the kernels and uploading the tables failed: %s", cudaGetErrorString(e));
             return report(OPENFISH_B200_ERR_CUDA, msg);
         }
         g_base[dev] = p;
@@ -95,15 +97,15 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
     if (options->beam_width != 32)
         return report(OPENFISH_B200_ERR_OPTION, "beam_width must be 32");
 
-    // carve the array: tables | status | bwd | fwd | post | back-pointers | states | qual | probs
-    // (no forward tensor for the models whose forward scan forms the posterior itself)
-    const bool fused = of_forward_posterior_fused(state_len);
+    // carve the array: tables | status | bwd | post | back-pointers | states | qual | probs
+    // (the documented size of the 64-state model counts a third tensor, which nothing uses any more: the
+    // limit that callers were given stays)
     const size_t nt = (size_t)N * T, rows = (size_t)N * (T + 1);
     size_t off = 0;
     const size_t o_tables = off; off += align_up(sizeof(ofx::Tables));
     const size_t o_status = off; off += 256;
     const size_t o_bwd = off; off += align_up(rows * ns * sizeof(float));
-    const size_t o_fwd = off; off += fused ? 0 : align_up(rows * ns * sizeof(float));
+    if (state_len == 3) off += align_up(rows * ns * sizeof(float));
     const size_t o_post = off; off += align_up(rows * ns * sizeof(float));
     const size_t o_bp = off; off += align_up(rows * 32);
     const size_t o_init = off; off += align_up((size_t)N * 32 * sizeof(int));
@@ -130,21 +132,23 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
     const ofx::Tables *tables = reinterpret_cast<const ofx::Tables *>(base + o_tables);
     int *status = reinterpret_cast<int *>(base + o_status);
     float *bwd = reinterpret_cast<float *>(base + o_bwd);
-    float *fwd = fused ? nullptr : reinterpret_cast<float *>(base + o_fwd);
     float *post = reinterpret_cast<float *>(base + o_post);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return report(OPENFISH_B200_ERR_CUDA, "cudaDeviceGetAttribute failed");
+    const OfScanPlan plan = of_scan_plan(N, state_len, sms);
     cudaStream_t stream = 0;  // legacy default stream: nothing to create
     e = cudaMemsetAsync(status, 0, sizeof(int), stream);  // the one thing that must start at zero
     if (e == cudaSuccess)
-        e = of_launch_scans(scores_TNC, bwd, fwd, T, N, state_len, options->blank_score, tables,
-                            status, ofd::kDefaultWaitLimitNs, stream);
-    if (e == cudaSuccess && fused)
-        e = of_launch_forward_posterior(scores_TNC, bwd, post, T, N, state_len, options->blank_score,
-                                        tables, status, ofd::kDefaultWaitLimitNs, stream);
+        e = of_launch_first_scans(plan, scores_TNC, bwd, post, T, N, state_len, sms, options->blank_score, tables, status,
+                                  ofd::kDefaultWaitLimitNs, stream);
+    if (e == cudaSuccess)
+        e = of_launch_rest_of_posterior(plan, scores_TNC, bwd, post, T, N, state_len, sms, options->blank_score, tables,
+                                        status, ofd::kDefaultWaitLimitNs, stream);
     if (e == cudaSuccess) {
         OfDecodeArgs a;
         a.scores = static_cast<const __half *>(scores_TNC);
         a.bwd = bwd;
-        a.fwd = fwd;
         a.post = post;
         a.bp = base + o_bp;
         a.init_kmers = reinterpret_cast<int *>(base + o_init);

@@ -57,6 +57,8 @@ struct Tables {
     double exp2_j[kExpTab];
     double rcp_c[kLogTab];
     double log_c[kLogTab];
+    float rcp_f[kLogTab];  // for the fp32 logarithm of fast_lse.cuh: 1/c with log(c) = log_f to within 2^-26
+    float log_f[kLogTab];
 };
 
 inline void fill_tables(Tables *t) {
@@ -72,6 +74,26 @@ inline void fill_tables(Tables *t) {
     // tie whenever the maximum is a round number, as it is on the first timestep.
     t->rcp_c[0] = 1.0;
     t->log_c[0] = 0.0;
+    // c near the centre of the interval such that log(c) is a multiple of 2^-11 and 1/c hits a float
+    // closely (accurate tables in the manner of Gal): of the multiples around the centre's logarithm
+    // the nearest one whose exp(-.) lies within 2^-28 of a float, or the best of 32.
+    t->rcp_f[0] = 1.0f;
+    t->log_f[0] = 0.0f;
+    for (int i = 1; i < kLogTab; ++i) {
+        const double c = ldexp(1.0 + ((i & 63) + 0.5) / 64.0, i >> 6);
+        const double mid = rint(log(c) * 2048.0);
+        double best = 1.0;
+        for (int k = 0; k < 32 && best > 0x1p-28; ++k) {
+            const double g = (mid + ((k & 1) ? (k + 1) / 2 : -k / 2)) / 2048.0;
+            const float r = (float)exp(-g);
+            const double off = fabs(log((double)r) + g);
+            if (off < best) {
+                best = off;
+                t->rcp_f[i] = r;
+                t->log_f[i] = (float)g;
+            }
+        }
+    }
 }
 
 OFX_HD double d_fma(double a, double b, double c) {

@@ -1,56 +1,27 @@
-// posterior_seq.cu -- posterior, traceback, per-base quality and sequence/qstring generation for
+// posterior_seq.cu -- traceback, per-base quality and sequence/qstring generation for
 // one chunk per block, for sm_100a.
 //
-// Replaces the softmax half of the reference kernel fwd_post_scan (src/scan_cuda.cu:147-199),
-// the traceback at the end of beam_search (src/beam_search_cuda.cu:517-527) and the kernels
+// Replaces the traceback at the end of beam_search (src/beam_search_cuda.cu:517-527) and the kernels
 // compute_qual_data (:530-605) and generate_sequence (:52-121); semantics are those of the CPU
-// routines (src/decode_cpu.c:115,121-147; src/beam_search.c:430-496 and 49-99).
+// routines (src/beam_search.c:430-496 and 49-99).
 //
-// First (unless the forward scan kernel has done it already: a.fwd null) the posterior =
-// softmax over states of fwd + bwd: rows are independent, so each warp
-// takes rows of its own and streams them straight from and to HBM (this part is bound by HBM
-// bandwidth: it reads 2(T+1)ns and writes (T+1)ns floats per chunk).  No per-row maximum is
-// needed: the log partition function is the same for every row, so one offset taken from row 0
-// keeps every exponent in range.
-// Then the whole block walks the back-pointers the beam search left in HBM (staged through
-// shared memory in windows), rebuilds the k-mer of every path element from the emitted bases,
-// gathers the posterior of each path k-mer and its shifted neighbours, and emits moves,
-// sequence and qstring, zero-filling the unused tail of each row.
+// The whole block walks the back-pointers the beam search left in HBM (staged through shared memory
+// in windows), rebuilds the k-mer of every path element from the emitted bases, gathers the
+// posterior of each path k-mer and its shifted neighbours, and emits moves, sequence and qstring,
+// zero-filling the unused tail of each row.
 #include <float.h>
 
 #include "beam_post.cuh"
-#include "fast_lse.cuh"
 #include "of_device.cuh"
+#include "prepare.cuh"
 
 namespace {
 
 constexpr int kBeam = 32;
 constexpr int kWin = 256;  // traceback window, timesteps
-using ofd::ex2_approx;
-constexpr float kLog2e = 1.4426950408889634f;
 
-// SPT (1, 2 or 4) consecutive floats through one vector access.
-template <int SPT>
-__device__ __forceinline__ void load_floats(float (&d)[SPT], const float *p) {
-    if constexpr (SPT == 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(p);
-        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-    } else if constexpr (SPT == 2) {
-        const float2 v = *reinterpret_cast<const float2 *>(p);
-        d[0] = v.x; d[1] = v.y;
-    } else {
-        d[0] = *p;
-    }
-}
-template <int SPT>
-__device__ __forceinline__ void store_floats(float *p, const float (&d)[SPT]) {
-    if constexpr (SPT == 4) *reinterpret_cast<float4 *>(p) = make_float4(d[0], d[1], d[2], d[3]);
-    else if constexpr (SPT == 2) *reinterpret_cast<float2 *>(p) = make_float2(d[0], d[1]);
-    else *p = d[0];
-}
 template <int NS>
 struct PostSmem {
-    float m0;
     int part[256];  // block-scan partials of the tail phase
     // the tail phase's arrays start here and run into the dynamic shared memory behind
     alignas(128) unsigned char tail[128];
@@ -65,68 +36,16 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     constexpr int SL = BITS / 2;
     constexpr int MSB = NS / 4;
     constexpr int NT = kPostThreads;
-    constexpr int NWARP = NT / 32;
     using Smem = PostSmem<NS>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
-    const int lane = tid & 31;
     const int chunk = blockIdx.x;
     const int T = a.T;
-    const float *bwd_chunk = a.bwd + (size_t)chunk * (size_t)(T + 1) * NS;
-    const float *fwd_chunk = a.fwd + (size_t)chunk * (size_t)(T + 1) * NS;
-    float *post_chunk = a.post + (size_t)chunk * (size_t)(T + 1) * NS;
+    const float *post_chunk = a.post + (size_t)chunk * (size_t)(T + 1) * NS;
     const unsigned char *bp_chunk = a.bp + (size_t)chunk * (size_t)(T + 1) * kBeam;
 
-    // ---------------------------------------------------------------------- posterior
-    // Rows are independent: a warp takes a row, each lane NS/32 of its states (two lanes per
-    // 16 bytes for the 64-state model), one shuffle reduction for the row sum.  The softmax
-    // offset is the maximum of fwd+bwd at row 0 (= bwd row 0, fwd is zero there): the log
-    // partition function is the same for every row, so every exponent stays in range.
-    if (a.fwd != nullptr && warp == 0) {
-        float m = -FLT_MAX;
-        for (int s = lane; s < NS; s += 32) m = fmaxf(m, bwd_chunk[s]);
-        m = ofd::warp_max(m);
-        if (lane == 0) sm.m0 = m;
-    }
-    __syncthreads();
-    const float m0 = sm.m0;
-    constexpr int PER = NS / 32;              // states per lane: 2, 8 or 32
-    constexpr int VEC = PER >= 4 ? 4 : PER;   // floats per access
-    constexpr int NV = PER / VEC;
-    for (int t = warp; t <= T && a.fwd != nullptr; t += NWARP) {
-        const float *fr = fwd_chunk + (size_t)t * NS, *br = bwd_chunk + (size_t)t * NS;
-        float e[PER];
-        float part = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            float fv[VEC], bv[VEC];
-            load_floats<VEC>(fv, fr + (i * 32 + lane) * VEC);
-            load_floats<VEC>(bv, br + (i * 32 + lane) * VEC);
-#pragma unroll
-            for (int k = 0; k < VEC; ++k) {
-                e[i * VEC + k] = ex2_approx(((fv[k] + bv[k]) - m0) * kLog2e);
-                part += e[i * VEC + k];
-            }
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const float inv = 1.0f / part;
-        float *pr = post_chunk + (size_t)t * NS;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            float o[VEC];
-#pragma unroll
-            for (int k = 0; k < VEC; ++k) o[k] = e[i * VEC + k] * inv;
-            store_floats<VEC>(pr + (i * 32 + lane) * VEC, o);
-        }
-    }
-
-    // ---------------------------------------------------------------------- tail, whole block
-    __syncthreads();
-    // arrays laid over the rings (and the dynamic shared memory behind them)
     unsigned char *tail = sm.tail;
     const int Tp = (T + 16) & ~15;
     unsigned char *win = tail;                          // kWin * 32 bytes
@@ -281,17 +200,22 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     }
 }
 
+constexpr size_t kMostBytes = 227 * 1024;  // of dynamic shared memory: what a block can have
+
+template <int NS>
+struct Seq {
+    static constexpr auto kern = posterior_seq_kernel<NS>;
+    static constexpr size_t bytes = kMostBytes;
+};
+
 template <int NS>
 cudaError_t launch_post(const OfDecodeArgs &a, cudaStream_t stream) {
     using Smem = PostSmem<NS>;
     const int Tp = (a.T + 16) & ~15;
     const size_t tail = (size_t)kWin * kBeam + (kWin / 8) * (kBeam + 4) + 8 * (size_t)Tp + 64;
     const size_t bytes = sizeof(Smem) + tail;
-    if (bytes > 227 * 1024) return cudaErrorInvalidValue;
-    auto kern = posterior_seq_kernel<NS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    kern<<<a.N, kPostThreads, bytes, stream>>>(a);
+    if (bytes > kMostBytes) return cudaErrorInvalidValue;
+    posterior_seq_kernel<NS><<<a.N, kPostThreads, bytes, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -303,5 +227,14 @@ cudaError_t of_launch_posterior_seq(const OfDecodeArgs &a, cudaStream_t stream) 
         case 4: return launch_post<256>(a, stream);
         case 5: return launch_post<1024>(a, stream);
         default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t of_load_posterior_seq(int kernel) {
+    switch (kernel) {
+        case kSeq64: return of_load<Seq<64>>();
+        case kSeq256: return of_load<Seq<256>>();
+        case kSeq1024: return of_load<Seq<1024>>();
+        default: return cudaSuccess;
     }
 }

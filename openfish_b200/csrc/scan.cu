@@ -7,12 +7,12 @@
 //                                       for s = j + k*ns/4
 //   fwd[n][0][s] = 0,  fwd[n][t+1][s] = LSE5( fwd[n][t][s] + stay,   fwd[n][t][j + b*ns/4] + score[t][n][4s + b] )
 //                                       for s = 4j + k                         (b = 0..3 in both)
-// The two recursions do not depend on each other (only the posterior needs both).  The launcher
-// takes either or both; the decode runs the backward scan first (the beam search waits for it)
-// and the forward scan beside the beam search, which leaves most issue slots free.  For the 256-
-// and 1024-state models the forward scan also forms the posterior (a warp of its own per block,
-// see PosteriorRow) and its scores never leave the chip; for the 64-state model they go to HBM for
-// the kernel that forms the posterior.
+// The two recursions do not depend on each other (only the posterior needs both).  This file's kernels
+// are for batches that fill the GPU (scan_ahead.cu has one for small batches): the decode runs the
+// backward scan first (the beam search waits for it) and the forward scan beside the beam search,
+// which leaves most issue slots free.  For the 256- and 1024-state models the forward scan also
+// forms the posterior (a warp of its own per block, see PosteriorRow) and its scores never leave the
+// chip; for the 64-state model they go to HBM for the kernel that forms the posterior.
 //
 // Shape of a block.  In either direction the four states that share j also share their four
 // neighbour inputs, and their 16 transition scores are one contiguous 32-byte piece of the score
@@ -27,91 +27,12 @@
 #include "exact_math.cuh"
 #include "fast_lse.cuh"
 #include "of_device.cuh"
+#include "prepare.cuh"
+#include "scan_topo.cuh"
 
 namespace {
 
-constexpr int kExpCopies = 16;  // per-half-warp-lane copies of the 2^(j/64) table
-
-// One fp16 out of a 32-bit word, widened.  Going through __half2 lets the conversion pick its
-// half of the register directly instead of shifting it out first.
-__device__ __forceinline__ float half_of(uint32_t word, int odd) {
-    const __half2 h = *reinterpret_cast<const __half2 *>(&word);
-    return odd ? __high2float(h) : __low2float(h);
-}
-
-// ------------------------------------------------------------------------------------------
-// The two recursions differ only in which states a thread owns, which inputs they share, where
-// their scores sit inside the 32-byte piece, and in the direction of time.
-
-template <int NS>
-struct BwdTopo {
-    static constexpr int NJ = NS / 4;
-    static constexpr bool kForward = false;
-    // thread (j, slot k) owns state j + k*NJ; the four slots share the successors 4j..4j+3
-    __device__ static int state(int j, int k) { return j + k * NJ; }
-    __device__ static void shared_inputs(const float *in, int j, float (&x)[4]) {
-        const float4 v = *reinterpret_cast<const float4 *>(in + 4 * j);
-        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-    }
-    // score of (slot k, base b) is half number 4b + k of the piece
-    __device__ static int half_index(int k, int b) { return 4 * b + k; }
-    // the same out of the piece held as eight words, slot k0 + k with k0 (a multiple of SPT)
-    // known only at run time: selects instead of strided shared-memory reads
-    template <int SPT>
-    __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
-        if (SPT == 4) return half_of(w[2 * b + (k >> 1)], k & 1);
-        const uint32_t x = (k0 & 2) ? w[2 * b + 1] : w[2 * b];
-        return SPT == 2 ? half_of(x, k) : half_of(x, k0 & 1);
-    }
-    __device__ static int j_of(int s) { return s % NJ; }
-    __device__ static int k_of(int s) { return s / NJ; }
-    // the states of the next row to be computed that read state s of this row, d = 0..3
-    __device__ static int reader(int s, int d) { return (s >> 2) + d * NJ; }
-    // time: step i reads score row T-1-i and produces output row T-1-i; row T is the zero row
-    __device__ static int score_row(int i, int T) { return T - 1 - i; }
-    __device__ static int out_row(int i, int T) { return T - 1 - i; }
-    __device__ static int zero_row(int T) { return T; }
-};
-
-template <int NS>
-struct FwdTopo {
-    static constexpr int NJ = NS / 4;
-    static constexpr bool kForward = true;
-    // thread (j, slot k) owns state 4j + k; the four slots share the predecessors j + b*NJ
-    __device__ static int state(int j, int k) { return 4 * j + k; }
-    __device__ static void shared_inputs(const float *in, int j, float (&x)[4]) {
-#pragma unroll
-        for (int b = 0; b < 4; ++b) x[b] = in[j + b * NJ];
-    }
-    __device__ static int half_index(int k, int b) { return 4 * k + b; }
-    template <int SPT>
-    __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
-        const int c = b >> 1;
-        if (SPT == 4) return half_of(w[2 * k + c], b & 1);
-        if (SPT == 2) return half_of(k0 ? w[4 + 2 * k + c] : w[2 * k + c], b & 1);
-        const uint32_t x = (k0 & 2) ? ((k0 & 1) ? w[6 + c] : w[4 + c]) : ((k0 & 1) ? w[2 + c] : w[c]);
-        return half_of(x, b & 1);
-    }
-    __device__ static int j_of(int s) { return s >> 2; }
-    __device__ static int k_of(int s) { return s & 3; }
-    __device__ static int reader(int s, int d) { return 4 * (s % NJ) + d; }
-    __device__ static int score_row(int i, int) { return i; }
-    __device__ static int out_row(int i, int) { return i + 1; }
-    __device__ static int zero_row(int) { return 0; }
-};
-
-// The five terms of state s: inputs from row `in`, scores from the chunk's score row `row`.
-template <class Topo>
-__device__ __forceinline__ void terms_of(int s, const float *in, const unsigned char *row, float stay,
-                                         float (&v)[5]) {
-    const int j = Topo::j_of(s), k = Topo::k_of(s);
-    const __half *piece = reinterpret_cast<const __half *>(row) + 16 * j;
-    float x[4];
-    Topo::shared_inputs(in, j, x);
-    v[0] = in[s] + stay;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) v[b + 1] = x[b] + __half2float(piece[Topo::half_index(k, b)]);
-}
+using namespace scan_topo;
 
 // Terms of the SPT states (j, k0 .. k0+SPT-1) of one thread.  The 32-byte piece is read as two
 // 16-byte halves (a two-way bank conflict, which costs less than the selects that avoid it: the
@@ -161,7 +82,7 @@ __device__ __forceinline__ void thread_store(float *smem_row, float *gmem_row, i
 // during which it is needed; a load from HBM issued by this warp would put a microsecond of
 // latency into every timestep, which is more than the scan warps take).  Lane l
 // takes the states (q*32 + l)*VEC .. +VEC-1; the arithmetic and its order are those of the
-// stand-alone posterior loop in posterior_seq.cu (softmax offset m0 = the maximum of row 0, where
+// stand-alone posterior kernel in scan_ahead.cu (softmax offset m0 = the maximum of row 0, where
 // fwd is zero: the log partition function is the same for every row, so exponents stay in range).
 template <int NS>
 struct PosteriorRow {
@@ -236,8 +157,9 @@ struct PosteriorRow {
 // value, what the exact routine alone would have produced.  Three row buffers rotate so that the
 // inputs of a timestep are still there while it is being checked, and score rows are released
 // one timestep late.
-template <int NS, int SPT, int RING, bool POST>
+template <int NS, int SPT, int RING, int COPIES, bool POST>
 struct SpecSmem {
+    static constexpr int kExpCopies = COPIES;  // of the 2^(j/64) table, by lane: their reads rarely meet in a bank
     static constexpr int kRowBytes = NS * 4 * 2;
     static constexpr int NW = NS / SPT / 32;  // scan warps
     static constexpr int kPerWarp = 16;       // listed states per warp and timestep, at most
@@ -267,11 +189,11 @@ struct SpecSmem {
 // out of line on purpose.  v: the thread's terms, res: its guesses (in) and, where states were
 // settled, their exact values (out); bit k of okmask: state k was certified.  Returns the number of
 // states the warp put on the list, or -1 if it settled its uncertified states here (res changed).
-template <class Topo, int NS, int SPT, int RING, bool POST>
-__device__ __noinline__ int crowded_step(SpecSmem<NS, SPT, RING, POST> &sm, const float (*v)[5], float *res, uint32_t okmask,
+template <class Topo, int NS, int SPT, int RING, int COPIES, bool POST>
+__device__ __noinline__ int crowded_step(SpecSmem<NS, SPT, RING, COPIES, POST> &sm, const float (*v)[5], float *res, uint32_t okmask,
                                          int par, int j, int k0, const float *in, const unsigned char *row,
                                          float stay, const ofx::TabRef tr) {
-    constexpr int PER = SpecSmem<NS, SPT, RING, POST>::kPerWarp;
+    constexpr int PER = SpecSmem<NS, SPT, RING, COPIES, POST>::kPerWarp;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t bad[SPT];
@@ -336,16 +258,16 @@ __device__ __noinline__ int crowded_step(SpecSmem<NS, SPT, RING, POST> &sm, cons
 // that (`out` is then the posterior tensor and `bwd_in` the finished backward scores).  Row r is
 // final after the barrier that ends timestep r (its guesses have been checked by then) and its
 // buffer is written again during timestep r+2, so the posterior warp takes it during timestep
-// r+1; the last two rows are taken after the scan.  The arithmetic is that of the stand-alone
-// posterior loop in posterior_seq.cu, operation for operation.
-template <class Topo, int NS, int SPT, int RING, bool POST>
+// r+1; the last two rows are taken after the scan.
+template <class Topo, int NS, int SPT, int RING, int COPIES, bool POST>
 __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, const __half *scores,
                                           float *out, const float *bwd_in, int T, int N, float stay,
                                           const ofx::Tables *tables, int *status, uint64_t wait_ns) {
     constexpr int NJ = NS / 4;
     constexpr int TPC = NS / SPT;
-    using Smem = SpecSmem<NS, SPT, RING, POST>;
+    using Smem = SpecSmem<NS, SPT, RING, COPIES, POST>;
     constexpr int NW = Smem::NW, PER = Smem::kPerWarp;
+    constexpr int kExpCopies = Smem::kExpCopies;
     static_assert(!POST || Topo::kForward, "the posterior rides on the forward scan");
     static_assert(TPC % 32 == 0, "scan warps must be full");
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
@@ -606,7 +528,7 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
                 cres[k] = res[k];
                 okmask |= (uint32_t)ok[k] << k;
             }
-            total = crowded_step<Topo, NS, SPT, RING, POST>(sm, cv, cres, okmask, i & 1, j, k0, in, row, stay, tr);
+            total = crowded_step<Topo, NS, SPT, RING, COPIES, POST>(sm, cv, cres, okmask, i & 1, j, k0, in, row, stay, tr);
 #pragma unroll
             for (int k = 0; k < SPT; ++k) res[k] = cres[k];
             if (total < 0) {  // states were settled here and now: their values replace the guesses
@@ -634,81 +556,109 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
 // One grid for either or both directions: the first n_bwd_blocks blocks scan backwards, the
 // rest forwards.
 
-template <int NS, int SPT, int RING>
-__global__ void __launch_bounds__(NS / SPT + 64, (NS <= 64 ? 8 : NS <= 256 ? 4 : 2))
+template <int NS, int SPT, int RING, int COPIES, int MINB>
+__global__ void __launch_bounds__(NS / SPT + 64, MINB)
 scan_spec_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd,
                  int T, int N, int n_bwd_blocks, float stay, const ofx::Tables *__restrict__ tables,
                  int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     if ((int)blockIdx.x < n_bwd_blocks)
-        spec_body<BwdTopo<NS>, NS, SPT, RING, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
+        spec_body<BwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
                                                      status, wait_ns);
     else
-        spec_body<FwdTopo<NS>, NS, SPT, RING, false>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
+        spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
                                                      stay, tables, status, wait_ns);
 }
 
 // Forward scan with the posterior on top: one block per chunk, reads the finished backward scores.
-template <int NS, int SPT, int RING>
+template <int NS, int SPT, int RING, int COPIES>
 __global__ void __launch_bounds__(NS / SPT + 96, (NS <= 256 ? 5 : 2))
 scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__restrict__ bwd,
                            float *__restrict__ post, int T, int N, float stay,
                            const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    spec_body<FwdTopo<NS>, NS, SPT, RING, true>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
+    spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, true>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
 }
 
-template <int NS, int SPT, int RING>
-cudaError_t launch_spec(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
-                        const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
-    using Smem = SpecSmem<NS, SPT, RING, false>;
-    const size_t bytes = sizeof(Smem);
-    auto kern = scan_spec_kernel<NS, SPT, RING>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    const int n_bwd = bwd ? N : 0, n_fwd = fwd ? N : 0;
-    kern<<<n_bwd + n_fwd, NS / SPT + 64, bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
-    return cudaGetLastError();
-}
+// The kernels are described once, for loading (of_prepare_scans) and for launching.
+template <int NS, int SPT, int RING, int COPIES, int MINB>
+struct Spec {
+    static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB>;
+    static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, false>);
+    static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
+                              const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
+        const int n_bwd = bwd ? N : 0, n_fwd = fwd ? N : 0;
+        kern<<<n_bwd + n_fwd, NS / SPT + 64, bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
+        return cudaGetLastError();
+    }
+};
 
-template <int NS, int SPT, int RING>
-cudaError_t launch_spec_posterior(const __half *scores, const float *bwd, float *post, int T, int N, float stay,
-                                  const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
-    using Smem = SpecSmem<NS, SPT, RING, true>;
-    const size_t bytes = sizeof(Smem);
-    auto kern = scan_spec_posterior_kernel<NS, SPT, RING>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    kern<<<N, NS / SPT + 96, bytes, stream>>>(scores, bwd, post, T, N, stay, tables, status, wait_ns);
-    return cudaGetLastError();
-}
+template <int NS, int SPT, int RING, int COPIES>
+struct SpecPosterior {
+    static constexpr auto kern = scan_spec_posterior_kernel<NS, SPT, RING, COPIES>;
+    static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, true>);
+    static cudaError_t launch(const __half *scores, const float *bwd, float *post, int T, int N, float stay,
+                              const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
+        kern<<<N, NS / SPT + 96, bytes, stream>>>(scores, bwd, post, T, N, stay, tables, status, wait_ns);
+        return cudaGetLastError();
+    }
+};
+
+using Spec64 = Spec<64, 1, 8, 16, 8>;
+using Spec256 = Spec<256, 4, 6, 16, 4>;
+using Spec256Many = Spec<256, 4, 6, 4, 7>;
+using Spec1024 = Spec<1024, 4, 6, 16, 2>;
+using SpecPosterior256 = SpecPosterior<256, 4, 6, 16>;
+using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4>;
+using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 16>;
 
 }  // namespace
 
-// (Not for the 64-state model: a row is too little work there for a warp-wide reduction per
-// chunk and timestep to pay; its posterior is done by the stand-alone loop.)
-bool of_forward_posterior_fused(int state_len) { return state_len == 4 || state_len == 5; }
-
 cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bwd, float *post, int T, int N,
-                                        int state_len, float stay, const ofx::Tables *tables, int *status,
+                                        int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                         uint64_t wait_ns, cudaStream_t stream) {
     const __half *s = static_cast<const __half *>(scores_fp16);
     if (T < 1) return cudaErrorInvalidValue;
     switch (state_len) {
-        case 4: return launch_spec_posterior<256, 4, 6>(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
-        case 5: return launch_spec_posterior<1024, 4, 6>(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
+        // A block of 36 KB for batches that fit the GPU three and a half to the SM beside their beam
+        // searches; a larger batch takes one of 30 KB (fewer copies of a table), of which four go with
+        // four beam searches: 560 chunks of T = 800 in 1.64 ms instead of 1.96, 2048 of T = 1666 in 10.20
+        // instead of 10.31, but 512 in 3.00 instead of 2.96.
+        case 4:
+            if (2 * N <= 7 * sms) return SpecPosterior256::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
+            return SpecPosterior256Many::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
+        case 5: return SpecPosterior1024::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int T, int N,
-                            int state_len, float stay, const ofx::Tables *tables, int *status,
+                            int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                             uint64_t wait_ns, cudaStream_t stream) {
     const __half *s = static_cast<const __half *>(scores_fp16);
     switch (state_len) {
-        case 3: return launch_spec<64, 1, 8>(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        case 4: return launch_spec<256, 4, 6>(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        case 5: return launch_spec<1024, 4, 6>(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        // Four blocks to the SM (128 registers) as long as that is room enough, else seven (72): what a
+        // block loses is less than what a half empty second round of blocks costs.  740 chunks of T = 1666:
+        // 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28; 2048: 3.55 instead of 4.20; 512: 1.16 with
+        // four, 1.24 with seven.
+        case 4:
+            if (N <= 4 * sms) return Spec256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+            return Spec256Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        case 5: return Spec1024::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t of_load_scan(int kernel) {
+    switch (kernel) {
+        case kBwd256: return of_load<Spec256>();
+        case kFwd256: return of_load<SpecPosterior256>();
+        case kBwd256Many: return of_load<Spec256Many>();
+        case kFwd256Many: return of_load<SpecPosterior256Many>();
+        case kScan1024: return of_load<Spec1024>();
+        case kFwd1024: return of_load<SpecPosterior1024>();
+        case kFwd64: return of_load<Spec64>();
+        default: return cudaSuccess;
     }
 }

@@ -1,0 +1,542 @@
+// scan_ahead.cu -- the two scans of a small batch, side by side, for sm_100a.
+//
+// Same recursions and, value for value, the same results as scan.cu (src/decode_cpu.c:13-52, 54-119),
+// arranged for the case in which a GPU has fewer chunks than it could hold and a batch lasts as long as
+// one chunk's chain of T dependent timesteps.  One launch takes both directions (a block each for the
+// backward and the forward scan of a chunk; they do not depend on each other), the forward rows go to
+// HBM, and the posterior is formed by a kernel of its own while the beam search runs.
+//
+// A state whose rounding the fp32 evaluation cannot certify (two or three of a row's 256, once the
+// scores have grown) needs the value-exact routine, a chain of some 450 cycles on its own.  The scan
+// warps never wait for it: such a state gets the likelier of its two candidate floats, a bit in its
+// thread's mask says so, and the scan goes on.  Timesteps come in groups of E; while the scan warps work
+// on a group, E checker warps recompute the marked states of the group before, a timestep each, and
+// their verdict is looked at in the group after.  Was a guess wrong (one timestep in sixty), the scan
+// goes back to the group it was made in, takes that timestep with the exact routine for every state and
+// carries on from there.  What reaches HBM is what the exact routine alone would have produced.  While
+// the scores are small and the float grid fine, guesses are too many and too often wrong: every state
+// goes through the exact routine until the scores have passed kGuessFrom.
+//
+// What bounds it: the instructions of one timestep in one scan warp, issued two to three cycles apart.
+// So a thread has two states (four warps for 256 states; with four states a thread a timestep takes a
+// quarter longer), and everything that a timestep can do without sits elsewhere: waits for score rows,
+// verdicts and ring bookkeeping once a group, copies in, rows out and checks in warps of their own,
+// offsets inside a group as constants.
+#include <type_traits>
+
+#include "exact_math.cuh"
+#include "fast_lse.cuh"
+#include "of_device.cuh"
+#include "prepare.cuh"
+#include "scan.cuh"
+#include "scan_topo.cuh"
+
+namespace {
+
+using namespace scan_topo;
+
+// The 16 scores of the four states that share j: 32 consecutive bytes of the score row.
+struct Piece {
+    uint32_t w[8];
+    __device__ __forceinline__ Piece(const unsigned char *row, int j) { load(row, j); }
+    __device__ __forceinline__ void load(const unsigned char *row, int j) {
+        const uint4 lo = *reinterpret_cast<const uint4 *>(row + 32 * j);
+        const uint4 hi = *reinterpret_cast<const uint4 *>(row + 32 * j + 16);
+        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
+        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
+    }
+};
+
+// Terms of the SPT states (j, k0 .. k0+SPT-1) of one thread; `own` holds those states of row `in`
+// (what the thread computed a timestep ago).
+template <class Topo, int SPT>
+__device__ __forceinline__ void thread_terms(const float *in, const Piece &piece, int j, int k0, float stay,
+                                             float (*v)[5], const float *own) {
+    float x[4];
+    Topo::shared_inputs(in, j, x);
+#pragma unroll
+    for (int k = 0; k < SPT; ++k) {
+        v[k][0] = own[k] + stay;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) v[k][b + 1] = x[b] + Topo::template score<SPT>(piece.w, k0, k, b);
+    }
+}
+
+template <class Topo, int SPT>
+__device__ __forceinline__ void thread_store(float *dst, int j, int k0, const float *res) {
+    if constexpr (Topo::kForward && SPT == 4) {
+        *reinterpret_cast<float4 *>(dst + 4 * j) = make_float4(res[0], res[1], res[2], res[3]);
+    } else if constexpr (Topo::kForward && SPT == 2) {
+        *reinterpret_cast<float2 *>(dst + 4 * j + k0) = make_float2(res[0], res[1]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < SPT; ++k) dst[Topo::state(j, k0 + k)] = res[k];
+    }
+}
+
+template <int NS, int W, int E, int S>
+struct AheadSmem {
+    static constexpr int kRowBytes = NS * 4 * 2;
+    static constexpr int H = E * (S + 1);  // rows kept: a row is overwritten only after it has gone out
+    alignas(128) unsigned char ring[S][E][kRowBytes];
+    alignas(16) float rows[H][NS];
+    alignas(8) ofd::LogPair log_f[ofd::kLogPairs];
+    uint32_t mask[2][W][32];          // by group parity and scan thread: bit SPT*q + k, timestep q, state k
+    int verdict[2][E];                // by group parity and timestep: a guess was wrong
+    unsigned short marked[E][64];     // a timestep's marked states, when a lane has more than one
+    int back;                         // barriers minus groups: two more for every time the scan has gone back
+    double exp2_j[ofx::kExpTab];
+    double rcp_c[ofx::kLogTab];
+    double log_c[ofx::kLogTab];
+    alignas(8) uint64_t full[S];      // score rows landed
+    alignas(8) uint64_t done[S];      // group verified, its input rows final
+    alignas(8) uint64_t empty[S];     // those rows gone out
+    int abort_flag;
+};
+
+// Scores from which on guesses are made: one in twelve states is then marked, one in a thousand wrong.
+constexpr float kGuessFrom = 512.f;
+
+// All states of a thread by the exact routine; out of line (the first hundred timesteps and redone
+// ones come here), so everything is passed in registers.
+template <class Topo, int SPT>
+__device__ __noinline__ float4 exact_step(const float *in, const unsigned char *row, int j, int k0, float stay,
+                                          float4 own, const double *exp2_j, const double *rcp_c, const double *log_c) {
+    float v[SPT][5], out[SPT];
+    const float o[4] = {own.x, own.y, own.z, own.w};
+    thread_terms<Topo, SPT>(in, Piece(row, j), j, k0, stay, v, o);
+    const ofx::TabRef tr = {exp2_j, 1, rcp_c, log_c};
+    ofx::lse5_batch_exact<SPT>(v, out, tr);
+    return make_float4(out[0], SPT > 1 ? out[1 % SPT] : 0.f, SPT > 2 ? out[2 % SPT] : 0.f, SPT > 2 ? out[3 % SPT] : 0.f);
+}
+
+template <int ID, int THREADS>
+__device__ __forceinline__ void named_sync() {
+    if constexpr (THREADS == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+
+// One direction of one chunk by one block: W scan warps, E checker warps, a copy warp and an output warp.
+// `out` gets the T+1 rows of the chunk.
+template <class Topo, int NS, int W, int E, int S>
+__device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, const __half *scores, float *out,
+                                           int T, int N, float stay, const ofx::Tables *tables, int *status,
+                                           uint64_t wait_ns) {
+    constexpr int SPT = NS / (32 * W);  // states per scan thread
+    static_assert(SPT == 2 || SPT == 4, "a thread's states share one j");
+    static_assert(E * SPT <= 32 && E >= 2 && S >= 4, "a mask word per group; three groups are under way");
+    constexpr int NT = 32 * (W + E + 2);
+    constexpr int kSync = 32 * (W + E);  // threads at a group's end
+    using Smem = AheadSmem<NS, W, E, S>;
+    constexpr int H = Smem::H;
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (known to be the same for a whole warp)
+    for (int i = tid; i < ofx::kExpTab; i += NT) sm.exp2_j[i] = tables->exp2_j[i];
+    for (int i = tid; i < ofx::kLogTab; i += NT) {
+        sm.rcp_c[i] = tables->rcp_c[i];
+        sm.log_c[i] = tables->log_c[i];
+        sm.log_f[i] = {tables->rcp_f[i], tables->log_f[i]};
+    }
+    for (int i = tid; i < NS; i += NT) sm.rows[0][i] = 0.f;
+    for (int i = tid; i < 2 * W * 32; i += NT) (&sm.mask[0][0][0])[i] = 0;
+    if (tid < 2 * E) (&sm.verdict[0][0])[tid] = 0;
+    if (tid == 0) {
+        sm.abort_flag = 0;
+        sm.back = 0;
+        for (int r = 0; r < S; ++r) {
+            ofd::mbar_init(&sm.full[r], 1);
+            ofd::mbar_init(&sm.done[r], 1);
+            ofd::mbar_init(&sm.empty[r], 1);
+        }
+        ofd::mbar_fence_init();
+    }
+    __syncthreads();
+
+    float *out_chunk = out + (size_t)chunk * (size_t)(T + 1) * NS;
+    const int groups = (T + E - 1) / E;
+
+    if (warp == W + E) {
+        // ------------------------------------------------------------------ copy warp
+        if (lane == 0) {
+            const size_t t_stride = (size_t)N * NS * 4;
+            const __half *src = scores + (size_t)chunk * NS * 4 + t_stride * (size_t)Topo::score_row(0, T);
+            const ptrdiff_t step = Topo::kForward ? (ptrdiff_t)t_stride : -(ptrdiff_t)t_stride;
+            int issued = 0, stage = 0;
+            uint32_t parity = 1;  // (of the stage's previous release)
+            for (; issued < groups; ++issued) {
+                if (issued >= S) ofd::mbar_wait_bounded(&sm.empty[stage], parity, &sm.abort_flag, status, wait_ns);
+                if (*(volatile int *)&sm.abort_flag) break;
+                const int n = min(E, T - issued * E);
+                ofd::mbar_arrive_expect_tx(&sm.full[stage], n * Smem::kRowBytes);
+                for (int q = 0; q < n; ++q) {
+                    ofd::bulk_g2s(sm.ring[stage][q], src, Smem::kRowBytes, &sm.full[stage]);
+                    src += step;
+                }
+                if (++stage == S) {
+                    stage = 0;
+                    parity ^= 1u;
+                }
+            }
+            // after an abort the newest copies get a bounded chance to land before the block retires
+            if (*(volatile int *)&sm.abort_flag) ofd::mbar_drain_bounded(sm.full, S, issued, wait_ns);
+        }
+        return;
+    }
+
+    if (warp == W + E + 1) {
+        // ------------------------------------------------------------------ output warp
+        // rows of a group leave once the group is verified; row T at the end
+        constexpr int PERL = NS / 32, V = PERL >= 4 ? 4 : PERL;  // floats per lane, per access
+        float *dst = out_chunk + (size_t)Topo::zero_row(T) * NS;
+        const float *row = sm.rows[0];
+        auto row_out = [&]() {
+#pragma unroll
+            for (int q = 0; q < PERL / V; ++q) {
+                if constexpr (V == 4)
+                    reinterpret_cast<float4 *>(dst)[q * 32 + lane] = reinterpret_cast<const float4 *>(row)[q * 32 + lane];
+                else
+                    reinterpret_cast<float2 *>(dst)[q * 32 + lane] = reinterpret_cast<const float2 *>(row)[q * 32 + lane];
+            }
+            dst += Topo::kForward ? NS : -NS;
+            row = row == sm.rows[H - 1] ? sm.rows[0] : row + NS;
+        };
+        int stage = 0;
+        uint32_t parity = 0;
+        for (int g = 0; g < groups; ++g) {
+            ofd::mbar_wait_bounded(&sm.done[stage], parity, &sm.abort_flag, status, wait_ns);
+            const int n = min(E, T - g * E);
+            for (int q = 0; q < n; ++q) row_out();
+            __syncwarp();
+            ofd::mbar_arrive_if(lane == 0, &sm.empty[stage]);
+            if (++stage == S) {
+                stage = 0;
+                parity ^= 1u;
+            }
+        }
+        row_out();
+        return;
+    }
+
+    if (warp >= W) {
+        // ------------------------------------------------------------------ checker warps
+        // checker q takes timestep q of every group
+        const ofx::TabRef tr = {sm.exp2_j, 1, sm.rcp_c, sm.log_c};
+        const int q = warp - W;
+        const uint32_t lt_mask = (1u << lane) - 1u;
+        for (int at = 0;; ++at) {
+            named_sync<2, kSync>();
+            // the group that has just ended (when the scan is going back right now, `back` may show it
+            // already or not: this check is void either way)
+            const int g = at - *(volatile int *)&sm.back;
+            if (g > groups) return;
+            const int par = at & 1;
+            uint32_t m = 0;  // marks of this lane's W scan threads, SPT bits each
+#pragma unroll
+            for (int w = 0; w < W; ++w) m |= ((sm.mask[par][w][lane] >> (q * SPT)) & ((1u << SPT) - 1u)) << (w * SPT);
+            if (g < 0 || g >= groups) m = 0;
+            const int g0 = g < 0 ? 0 : g;
+            const int h0 = (g0 * E + q) % H;
+            const float *in = sm.rows[h0], *res = sm.rows[h0 + 1 == H ? 0 : h0 + 1];
+            const unsigned char *row = sm.ring[g0 % S][q];
+            bool wrong = false;
+            // bit `bit` of lane l's marks
+            auto check = [&](bool mine, int l, int bit) {
+                const int t = (bit / SPT) * 32 + l;  // the scan thread
+                const int s = Topo::state(t % Topo::NJ, (t / Topo::NJ) * SPT + bit % SPT);
+                float v[5];
+                terms_of<Topo>(s, in, row, stay, v);
+                const float guess = res[s];
+                const float x = ofx::lse5_exact(v, tr);
+                wrong = wrong || (mine && __float_as_uint(x) != __float_as_uint(guess));
+            };
+            uint32_t owners = __ballot_sync(0xffffffffu, m != 0);
+            if (owners) {
+                if (__any_sync(0xffffffffu, (m & (m - 1u)) != 0)) {
+                    int n = 0;
+                    do {
+                        const int to = n + __popc(owners & lt_mask);
+                        if (m && to < 64) sm.marked[q][to] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
+                        n += __popc(owners);
+                        m &= m - 1u;
+                        owners = __ballot_sync(0xffffffffu, m != 0);
+                    } while (owners);
+                    __syncwarp();
+                    if (n > 64) {
+                        wrong = true;  // (not worth checking: exactly for all states, then)
+                    } else {
+                        for (int first = 0; first < n; first += 32) {
+                            const bool mine = first + lane < n;
+                            const int e = sm.marked[q][mine ? first + lane : 0];
+                            check(mine, e & 31, e >> 5);
+                        }
+                    }
+                } else {
+                    check(m != 0, lane, m ? __ffs(m) - 1 : 0);
+                }
+            }
+            wrong = __any_sync(0xffffffffu, wrong);
+            if (lane == 0) sm.verdict[par][q] = wrong;
+        }
+    }
+
+    // ---------------------------------------------------------------------- scan warps
+    const int j = tid % Topo::NJ, k0 = (tid / Topo::NJ) * SPT;
+    float res[SPT];  // the thread's states of the current row: its stay terms for the next timestep
+#pragma unroll
+    for (int k = 0; k < SPT; ++k) res[k] = 0.f;
+    float *rows = sm.rows[0], *rows_next = sm.rows[E % H];  // row g*E, row (g+1)*E
+    const unsigned char *ring = sm.ring[0][0];
+    int g = 0, stage = 0;
+    uint32_t parity = 0;
+    int ignore = 2;  // verdicts to come that are about nothing
+    // timesteps of group `exact_of` that go through the exact routine for all states: those found wrong
+    // so far (they add up, or two wrong guesses in one group would take turns for ever)
+    uint32_t exact = 0;
+    int exact_of = -1;
+    bool small = true;  // the scores were small a group ago
+    ofd::mbar_wait_bounded(&sm.full[0], 0u, &sm.abort_flag, status, wait_ns);
+    Piece piece(ring, j);
+    // (one group past the end for the last verdict, one more for the checkers to leave)
+    for (int par = 0; g <= groups + 1; par ^= 1) {
+        // The verdict on the group before the last was handed over at the barrier just passed (it stays
+        // until the check of this group).  Nothing waits for it here: it is looked at when the first
+        // timestep of this group has been computed.
+        uint32_t wrong = 0;
+#pragma unroll
+        for (int q = 0; q < E; ++q) wrong |= *(volatile int *)&sm.verdict[par][q] ? 1u << q : 0u;
+        const int next = stage + 1 == S ? 0 : stage + 1;
+        const uint32_t next_parity = next ? parity : parity ^ 1u;
+        const unsigned char *ring_next = next ? ring + E * Smem::kRowBytes : sm.ring[0][0];
+        const float probe = rows[0];
+        const uint32_t how = small ? ~0u : (g == exact_of ? exact : 0u);
+        const int n = T - g * E;  // timesteps left
+        const bool ready = g + 1 >= groups || ofd::mbar_try_wait(&sm.full[next], next_parity);
+        const bool back = ignore == 0 && wrong != 0;
+        uint32_t bad = 0;
+        if (g < groups) {
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const float *in = rows + q * NS;
+                float *nxt = q + 1 < E ? rows + (q + 1) * NS : rows_next;
+                if (__builtin_expect((how >> q) & 1u, 0)) {
+                    const float4 own = make_float4(res[0], res[1], SPT > 2 ? res[2 % SPT] : 0.f, SPT > 2 ? res[3 % SPT] : 0.f);
+                    const float4 x = exact_step<Topo, SPT>(in, ring + q * Smem::kRowBytes, j, k0, stay, own, sm.exp2_j, sm.rcp_c, sm.log_c);
+                    res[0] = x.x;
+                    res[1] = x.y;
+                    if constexpr (SPT > 2) {
+                        res[2] = x.z;
+                        res[3] = x.w;
+                    }
+                } else {
+                    float v[SPT][5];
+                    thread_terms<Topo, SPT>(in, piece, j, k0, stay, v, res);
+                    bad |= ofd::lse5_guess_pairs<SPT, (NS > 64)>(v, res, sm.log_f) << (q * SPT);
+                }
+                if (q == 0 && back) break;
+                // (timesteps past the end are taken like any other, on leftover scores: their rows lie
+                // behind row T, and nothing reads them)
+                thread_store<Topo, SPT>(nxt, j, k0, res);
+                if (q + 1 < E) {
+                    piece.load(ring + (q + 1) * Smem::kRowBytes, j);
+                    named_sync<1, 32 * W>();
+                }
+            }
+        }
+        if (__builtin_expect(back, 0)) {
+            // back to the group before the last (only the first wrong timestep is known to be wrong for
+            // certain: what follows it followed from it)
+            g -= 2;
+            exact = (g == exact_of ? exact : 0u) | (wrong & (0u - wrong));
+            exact_of = g;
+            ignore = 2;
+            par ^= 1;  // (no barrier has been passed)
+            if (tid == 0) *(volatile int *)&sm.back = sm.back + 2;
+            rows = sm.rows[(g * E) % H];
+            rows_next = sm.rows[(g * E + E) % H];
+            stage = g % S;
+            parity = (uint32_t)(g / S) & 1u;
+            ring = sm.ring[stage][0];
+#pragma unroll
+            for (int k = 0; k < SPT; ++k) res[k] = rows[Topo::state(j, k0 + k)];
+            piece.load(ring, j);
+            small = fabsf(rows[0]) < kGuessFrom;
+            continue;
+        }
+        // the group before the last is verified
+        ofd::mbar_arrive_if(tid == 0 && ignore == 0 && g <= groups + 1, &sm.done[stage >= 2 ? stage - 2 : stage - 2 + S]);
+        ignore -= ignore > 0;
+        if (n < E) bad &= n > 0 ? (1u << (n * SPT)) - 1u : 0u;
+        sm.mask[par][warp][lane] = bad;
+        if (!ready) ofd::mbar_wait_slow(&sm.full[next], next_parity, &sm.abort_flag, status, wait_ns);
+        piece.load(ring_next, j);
+        small = fabsf(probe) < kGuessFrom;
+        named_sync<2, kSync>();
+        ++g;
+        stage = next;
+        parity = next_parity;
+        ring = ring_next;
+        rows = rows_next;
+        rows_next = rows_next == sm.rows[H - E] ? sm.rows[0] : rows_next + E * NS;
+    }
+}
+
+// The first n_bwd blocks scan backwards, the others forwards.
+template <int NS, int W, int E, int S, int MINB>
+__global__ void __launch_bounds__(32 * (W + E + 2), MINB)
+scan_ahead_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd, int T, int N,
+                  int n_bwd, float stay, const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    if ((int)blockIdx.x < n_bwd)
+        scan_chunk<BwdTopo<NS>, NS, W, E, S>(smem_raw, blockIdx.x, scores, bwd, T, N, stay, tables, status, wait_ns);
+    else
+        scan_chunk<FwdTopo<NS>, NS, W, E, S>(smem_raw, blockIdx.x - n_bwd, scores, fwd, T, N, stay, tables, status, wait_ns);
+}
+
+template <int NS, int W, int E, int S, int MINB>
+struct Ahead {
+    static constexpr auto kern = scan_ahead_kernel<NS, W, E, S, MINB>;
+    static constexpr size_t bytes = sizeof(AheadSmem<NS, W, E, S>);
+    static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
+                              const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
+        const int n_bwd = bwd ? N : 0, n_fwd = fwd ? N : 0;
+        kern<<<n_bwd + n_fwd, 32 * (W + E + 2), bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
+        return cudaGetLastError();
+    }
+};
+using Ahead64 = Ahead<64, 1, 2, 6, 8>;
+using Ahead256 = Ahead<256, 4, 2, 6, 2>;
+
+// ------------------------------------------------------------------------------------------
+// post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,
+// a warp takes a row straight from and to HBM.  No per-row maximum: the log partition function is the same
+// for every row, so one offset, the maximum of row 0 (where the forward scores are zero), keeps every
+// exponent in range.  Bound by HBM (12 bytes a state and row); it runs beside the beam search.
+constexpr int kPostRows = 32;  // rows a block takes, eight warps
+
+template <int NS>
+__global__ void __launch_bounds__(256) posterior_kernel(const float *__restrict__ bwd, float *post, int T) {
+    constexpr int PER = NS / 32, VEC = PER >= 4 ? 4 : PER, NV = PER / VEC;
+    constexpr float kLog2e = 1.4426950408889634f;
+    typedef typename std::conditional<VEC == 4, float4, float2>::type vec;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t base = (size_t)blockIdx.y * (size_t)(T + 1) * NS;
+    float m0 = -3.0e38f;
+    for (int s = lane; s < NS; s += 32) m0 = fmaxf(m0, bwd[base + s]);
+    m0 = ofd::warp_max(m0);
+    const int last = min(T + 1, (int)(blockIdx.x + 1) * kPostRows);
+    for (int t = blockIdx.x * kPostRows + warp; t < last; t += 8) {
+        const vec *br = reinterpret_cast<const vec *>(bwd + base + (size_t)t * NS);
+        vec *pr = reinterpret_cast<vec *>(post + base + (size_t)t * NS);
+        vec f[NV], b[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            f[q] = pr[q * 32 + lane];
+            b[q] = br[q * 32 + lane];
+        }
+        float part = 0.f;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            float *e = reinterpret_cast<float *>(&f[q]);
+            const float *d = reinterpret_cast<const float *>(&b[q]);
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) {
+                e[k] = ofd::ex2_approx(((e[k] + d[k]) - m0) * kLog2e);
+                part += e[k];
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        const float inv = 1.0f / part;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            float *e = reinterpret_cast<float *>(&f[q]);
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) e[k] *= inv;
+            pr[q * 32 + lane] = f[q];
+        }
+    }
+}
+
+template <int NS>
+struct Posterior {
+    static constexpr auto kern = posterior_kernel<NS>;
+    static constexpr size_t bytes = 0;
+};
+
+}  // namespace
+
+cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, float stay,
+                            const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
+    const __half *s = static_cast<const __half *>(scores_fp16);
+    if (T < 1) return cudaErrorInvalidValue;
+    switch (state_len) {
+        case 3: return Ahead64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        case 4: return Ahead256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int state_len, cudaStream_t stream) {
+    // (65535 chunks are the most that a grid's second dimension holds)
+    for (int first = 0; first < N; first += 65535) {
+        const int n = N - first < 65535 ? N - first : 65535;
+        const size_t skip = (size_t)first * (size_t)(T + 1) << (2 * state_len);
+        const dim3 grid((T + 1 + kPostRows - 1) / kPostRows, n);
+        switch (state_len) {
+            case 3: posterior_kernel<64><<<grid, 256, 0, stream>>>(bwd + skip, post + skip, T); break;
+            case 4: posterior_kernel<256><<<grid, 256, 0, stream>>>(bwd + skip, post + skip, T); break;
+            case 5: posterior_kernel<1024><<<grid, 256, 0, stream>>>(bwd + skip, post + skip, T); break;
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    return cudaGetLastError();
+}
+
+// Where the lines lie (decodes of T = 800, ms, by plan: together / ahead then forward / backward then forward):
+//   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;  320: 1.73 / 1.61 / 1.48
+//   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;  592: 1.16 / 1.01 / 1.05
+//   1024 states: 74 chunks 1.42 /  -   / 1.81;  222: 2.69 /  -   / 2.79;  240: 2.98 /  -   / 2.80
+// Two directions on one SM are in each other's way beyond their number (their code is more than an
+// instruction cache holds), which is why "together" ends where every block has an SM to itself, except for
+// the 1024-state model, where one block is half an SM's work.
+OfScanPlan of_scan_plan(int N, int state_len, int sms) {
+    if (state_len == 5) return 2 * N <= 3 * sms ? OfScanPlan::kTogether : OfScanPlan::kBackwardThenForward;
+    if (2 * N <= sms) return OfScanPlan::kTogether;
+    if (state_len == 3 || N <= 2 * sms) return OfScanPlan::kAheadThenForward;
+    return OfScanPlan::kBackwardThenForward;
+}
+
+cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bwd, float *post, int T, int N,
+                                  int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
+                                  uint64_t wait_ns, cudaStream_t stream) {
+    float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
+    if (plan == OfScanPlan::kBackwardThenForward || state_len == 5)
+        return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
+    return of_launch_ahead(scores, bwd, fwd, T, N, state_len, stay, tables, status, wait_ns, stream);
+}
+
+cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, const float *bwd, float *post, int T,
+                                        int N, int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
+                                        uint64_t wait_ns, cudaStream_t stream) {
+    if (plan != OfScanPlan::kTogether) {
+        // (a row of the 64-state model is too little work for a warp-wide reduction per chunk and timestep)
+        if (state_len != 3)
+            return of_launch_forward_posterior(scores, bwd, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
+        const cudaError_t e = of_launch_scans(scores, nullptr, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return of_launch_posterior(bwd, post, T, N, state_len, stream);
+}
+
+cudaError_t of_load_ahead(int kernel) {
+    switch (kernel) {
+        case kAhead256: return of_load<Ahead256>();
+        case kAhead64: return of_load<Ahead64>();
+        case kPosterior64: return of_load<Posterior<64>>();
+        case kPosterior256: return of_load<Posterior<256>>();
+        case kPosterior1024: return of_load<Posterior<1024>>();
+        default: return cudaSuccess;
+    }
+}

@@ -132,6 +132,16 @@ def test_long_chunks(native_lib, oracle_mod):
     check(native_lib, oracle_mod, synth.make_scores(6000, 5, 3, 98), 3, min_identical=1.0)
 
 
+@pytest.mark.parametrize("sl,T,N", [(3, 900, 74), (3, 33, 75), (3, 2, 149), (4, 300, 74), (4, 41, 75), (4, 260, 148),
+                                    (4, 24, 297), (4, 8, 519), (4, 5, 593), (5, 9, 222), (5, 8, 223), (4, 700, 2)])
+def test_batches_on_either_side_of_a_change_of_kernels(native_lib, oracle_mod, sl, T, N):
+    # the scans of a batch are run together, one ahead of the other or one after the other according to how
+    # many chunks there are for the GPU's 148 multiprocessors; odd and even T (groups of two timesteps),
+    # T long enough for guesses to be made and to be wrong
+    from openfish_b200 import synth
+    check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 300 + N, p_step=0.6), sl, min_identical=1.0)
+
+
 @pytest.mark.parametrize("okw", [dict(beam_cut=0.0), dict(beam_cut=1.5), dict(beam_cut=1e6),
                                  dict(q_scale=0.95, q_shift=-0.2), dict(q_scale=3.0, q_shift=10.0)])
 def test_options(native_lib, oracle_mod, okw):
