@@ -359,9 +359,8 @@ beam_search_kernel(const OfDecodeArgs a) {
             float lo = cut, hi = best;
             cut = mid;
             kept = (int)(both >> 16);
-            // (unrolled: a vote or reduction inside a loop costs a hundred cycles of re-convergence)
             int guesses = 2;
-#pragma unroll
+#pragma unroll 2
             for (int g = 0; g < 8; ++g) {
                 if (kept <= kBeam && kept >= 25) break;
                 const bool many = kept > kBeam;
