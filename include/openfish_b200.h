@@ -101,7 +101,8 @@ void openfish_b200_decode_submit_5wide(void *cuda_stream, int T, int N, const vo
  * events on the streams the kernels ran on: ms[0] the scans that the beam search waits for (the
  * backward one, in a small batch both), ms[1] everything between them and the copies (the beam search
  * kernel with the rest of the way to the posterior beside it on a second stream, then the traceback
- * + sequence kernel), ms[2] device-to-host copies, ms[3] all of it. */
+ * + sequence kernel, which also writes the results to the host), ms[2] zero (there are no copies
+ * behind the kernels), ms[3] all of it. */
 void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]);
 
 /* The same four numbers followed by: ms[4] beam search kernel, ms[5] what ran beside it (forward scan

@@ -8,6 +8,7 @@ module's native half raises.
 """
 import ctypes as C
 import os
+import weakref
 
 import numpy as np
 
@@ -176,9 +177,16 @@ def _scores_args(scores_TNC, state_len, options, gpubuf):
     return (T, N, Cc, scores_TNC.data_ptr(), state_len, C.byref(options or decoder_init()), gpubuf.ptr)
 
 
+def _own(ptr, N, T):
+    """uint8 array [N][T] on malloc'ed memory, which is freed when the last view of it is gone."""
+    mem = (C.c_uint8 * (N * T)).from_address(ptr)
+    weakref.finalize(mem, _lib.libc_free, ptr).atexit = False
+    return np.frombuffer(mem, dtype=np.uint8).reshape(N, T)
+
+
 def decode_gpu(scores_TNC, state_len, options=None, gpubuf=None):
-    """openfish_decode_gpu: returns dict(moves, sequence, qstring) of uint8 arrays [N][T]
-    (copies of the library's malloc'ed results, which are freed here)."""
+    """openfish_decode_gpu: returns dict(moves, sequence, qstring) of uint8 arrays [N][T] (the
+    library's malloc'ed results themselves, freed with the arrays)."""
     own = gpubuf is None
     if own:
         gpubuf = GpuBuf(scores_TNC.shape[0], scores_TNC.shape[1], state_len)
@@ -187,12 +195,7 @@ def decode_gpu(scores_TNC, state_len, options=None, gpubuf=None):
         out = [C.c_void_p() for _ in range(3)]
         lib().openfish_decode_gpu(*args, *[C.byref(o) for o in out])
         _check()
-        T, N = args[0], args[1]
-        res = {}
-        for k, p in zip(("moves", "sequence", "qstring"), out):
-            res[k] = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_uint8)), shape=(N, T)).copy()
-            lib().libc_free(p)
-        return res
+        return {k: _own(p.value, args[1], args[0]) for k, p in zip(("moves", "sequence", "qstring"), out)}
     finally:
         if own:
             gpubuf.free()

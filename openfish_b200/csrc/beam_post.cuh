@@ -15,6 +15,10 @@ struct OfDecodeArgs {
     uint8_t *moves;            // [N][T] out
     char *sequence;            // [N][T] out
     char *qstring;             // [N][T] out
+    // moves, sequence and qstring once more, in host memory that the device can write, and the status word
+    // (null: no copies)
+    unsigned char *host_results[3];
+    int *host_status;
     int *states;               // [N][T] out (base per timestep)
     float *qual;               // [N][T][4] out
     float *base_probs;         // [N][T] out

@@ -5,10 +5,9 @@
 // record that also owns two streams, events, the arithmetic tables and a page-locked staging
 // area; one decode is four or five kernel launches -- the scans that the beam search waits for; beam
 // search with the rest of the way to the posterior beside it on the second stream; traceback +
-// sequence -- and one device-to-host copy, all stream
-// ordered, with a single host wait at the end (the reference launches five kernels and three
-// memsets with a device-wide synchronisation after each and copies with three blocking
-// pageable transfers).
+// sequence, which also writes the results to the host -- all stream ordered, with a single host
+// wait at the end (the reference launches five kernels and three memsets with a device-wide
+// synchronisation after each and copies with three blocking pageable transfers).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdarg.h>
@@ -38,24 +37,29 @@ struct GpuBuf {
     int T, N, state_len, device;
     cudaStream_t stream;   // the main one; blocking, see ofb_gpubuf_create
     cudaStream_t stream2;  // what runs beside the beam search, ordered against `stream` by events only
-    cudaEvent_t ev[9];     // 0 start, 1 bwd scan done, 2 beam search done, 3 sequence done, 4 copies done,
-                           // 5 fwd scan start, 6 fwd scan done, 7 the caller's stream at submit time, 8 blank-column strip start
+    // 0 start, 1 first scans done, 2 beam search done, 3 all done, 4 and 5 start and end of what runs beside the
+    // beam search, 6 blank-column strip start; two sets, so that the times of the last decode can be
+    // worked out when somebody asks for them, whether or not another is in flight
+    cudaEvent_t ev[2][7];
+    cudaEvent_t caller_ev;  // the caller's stream at submit time
+    int set;                // of the decode in flight, or else of the last one
+    int done_set;           // of the last completed decode, -1 before the first
     uint64_t wait_ns;      // how long a kernel waits for an asynchronous copy before it raises d_status
     int *d_init_kmers;     // inside the beam_vector allocation, behind the back-pointers
     ofx::Tables *d_tables;
     int *d_status;
     void *d_scores4;           // 4-wide copy of 5-wide scores, made on the first 5-wide decode (null before)
     int sms;
-    unsigned char *d_results;  // moves | sequence | qstring, N*T bytes each
-    unsigned char *h_stage;    // page-locked, 3*N*T bytes + one status word
+    unsigned char *d_results;  // moves | sequence | qstring, N*T bytes each, on 16-byte boundaries
+    unsigned char *h_stage;    // page-locked, three results of N*T bytes, each on a 16-byte boundary, and a status word
+    unsigned char *d_stage;    // the same for the device
     int *h_status;
     // decode in flight
     bool pending;
     uint8_t *dst_moves;
     char *dst_sequence, *dst_qstring;
     bool via_stage;
-    float ms[8];
-    bool stripped = false;  // the decode in flight began with the blank-column strip
+    bool stripped[2];  // the decode of this set of events began with the blank-column strip
 };
 
 thread_local char g_err[512] = "";
@@ -77,17 +81,21 @@ int fail(int code, const char *fmt, ...) {
                         "%s failed: %s", #call, cudaGetErrorString(e_));                      \
     } while (0)
 
+// Bytes from one result to the next, in the staging area and on the device.
+size_t stage_pitch(const GpuBuf *g) { return ((size_t)g->N * g->T + 15) & ~(size_t)15; }
+
 GpuBuf *priv(const openfish_gpubuf_t *g) {
     return reinterpret_cast<GpuBuf *>(const_cast<openfish_gpubuf_t *>(g));
 }
 
-bool host_is_pinned(const void *p) {
+// Where the device can write a page-locked host buffer; null if it cannot.
+unsigned char *device_view(void *p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return nullptr;
     }
-    return at.type == cudaMemoryTypeHost;
+    return at.type == cudaMemoryTypeHost ? static_cast<unsigned char *>(at.devicePointer) : nullptr;
 }
 
 int destroy(GpuBuf *g) {
@@ -106,8 +114,9 @@ int destroy(GpuBuf *g) {
     cudaFree(g->d_status);
     cudaFree(g->d_scores4);
     if (g->h_stage) cudaFreeHost(g->h_stage);
-    for (int i = 0; i < 9; ++i)
-        if (g->ev[i]) cudaEventDestroy(g->ev[i]);
+    for (int i = 0; i < 14; ++i)
+        if (g->ev[i / 7][i % 7]) cudaEventDestroy(g->ev[i / 7][i % 7]);
+    if (g->caller_ev) cudaEventDestroy(g->caller_ev);
     if (g->stream2) cudaStreamDestroy(g->stream2);
     if (g->stream) cudaStreamDestroy(g->stream);
     g->magic = 0;
@@ -158,16 +167,17 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
         // stream (where the reference runs), so freshly written scores are seen
         CU(cudaStreamCreateWithFlags(&g->stream, cudaStreamDefault));
         CU(cudaStreamCreateWithFlags(&g->stream2, cudaStreamNonBlocking));
-        for (int i = 0; i < 9; ++i) CU(cudaEventCreate(&g->ev[i]));
+        for (int i = 0; i < 14; ++i) CU(cudaEventCreate(&g->ev[i / 7][i % 7]));
+        CU(cudaEventCreateWithFlags(&g->caller_ev, cudaEventDisableTiming));
+        g->done_set = -1;
         g->wait_ns = ofd::kDefaultWaitLimitNs;
-        // same ten buffers and sizes as the reference (src/decode_cuda.cu:22-45); the three
-        // result arrays share one allocation so that one copy brings them back
+        // same ten buffers and sizes as the reference (src/decode_cuda.cu:22-45)
         CU(cudaMalloc(&g->pub.bwd_NTC, tens));
         CU(cudaMalloc(&g->pub.post_NTC, tens));
-        CU(cudaMalloc(&g->d_results, 3 * nt));
+        CU(cudaMalloc(&g->d_results, 3 * stage_pitch(g)));
         g->pub.moves = g->d_results;
-        g->pub.sequence = reinterpret_cast<char *>(g->d_results + nt);
-        g->pub.qstring = reinterpret_cast<char *>(g->d_results + 2 * nt);
+        g->pub.sequence = reinterpret_cast<char *>(g->d_results + stage_pitch(g));
+        g->pub.qstring = reinterpret_cast<char *>(g->d_results + 2 * stage_pitch(g));
         // reference-sized (8 bytes per beam slot and timestep); this library uses 1 byte of the 8
         // for its packed back-pointers and 128 bytes per chunk behind them for the initial k-mers
         CU(cudaMalloc(&g->pub.beam_vector, (size_t)8 * N * 32 * (T + 1)));
@@ -179,8 +189,10 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
         CU(cudaMalloc(&g->pub.total_probs, sizeof(float) * nt));
         CU(cudaMalloc(&g->d_tables, sizeof(ofx::Tables)));
         CU(cudaMalloc(&g->d_status, sizeof(int)));
-        CU(cudaMallocHost(&g->h_stage, 3 * nt + 16));
-        g->h_status = reinterpret_cast<int *>(g->h_stage + ((3 * nt + 7) & ~(size_t)7));
+        CU(cudaHostAlloc(&g->h_stage, 3 * stage_pitch(g) + 16, cudaHostAllocMapped));
+        CU(cudaHostGetDevicePointer(&g->d_stage, g->h_stage, 0));
+        g->h_status = reinterpret_cast<int *>(g->h_stage + 3 * stage_pitch(g));
+        *g->h_status = ofd::kStatusOk;
         ofx::Tables host_tables;
         ofx::fill_tables(&host_tables);
         CU(cudaMemcpy(g->d_tables, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice));
@@ -232,9 +244,19 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     int dev = -1;
     CU(cudaGetDevice(&dev));
     if (dev != g->device) return fail(OPENFISH_B200_ERR_ARGUMENT, "gpubuf belongs to device %d, current device is %d", g->device, dev);
-    const size_t nt = (size_t)N * T;
 
     OfDecodeArgs a;
+    // the last kernel writes the results to the host itself: into the caller's buffers if they are
+    // page-locked (and start on 16-byte boundaries, as the device's do), else into the staging area
+    void *const dst[3] = {moves, sequence, qstring};
+    g->via_stage = false;
+    for (int i = 0; i < 3; ++i) {
+        a.host_results[i] = device_view(dst[i]);
+        if (!a.host_results[i] || ((uintptr_t)a.host_results[i] & 15u)) g->via_stage = true;
+    }
+    if (g->via_stage)
+        for (int i = 0; i < 3; ++i) a.host_results[i] = g->d_stage + i * stage_pitch(g);
+    a.host_status = reinterpret_cast<int *>(g->d_stage + 3 * stage_pitch(g));
     a.scores = static_cast<const __half *>(scores);
     a.bwd = g->pub.bwd_NTC;
     a.post = g->pub.post_NTC;
@@ -257,7 +279,7 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     a.q_scale = q_scale;
     a.score_scale = params->score_scale;
 
-    // stream:  scans as far as the beam search needs them -> beam search -----> sequence -> copies
+    // stream:  scans as far as the beam search needs them -> beam search -----> sequence
     // stream2:                    the rest of the way to the posterior (beside it) --^
     // Ordering against the producer of the scores: the gpubuf's main stream is a blocking one, so it
     // runs after whatever the caller queued on the legacy default stream (the reference's stream);
@@ -265,45 +287,36 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     // work as of now.
     if (params->on_caller_stream) {
         cudaStream_t caller = static_cast<cudaStream_t>(params->caller_stream);
-        CU(cudaEventRecord(g->ev[7], caller));
-        CU(cudaStreamWaitEvent(g->stream, g->ev[7], 0));
+        CU(cudaEventRecord(g->caller_ev, caller));
+        CU(cudaStreamWaitEvent(g->stream, g->caller_ev, 0));
     }
-    CU(cudaEventRecord(g->ev[0], g->stream));
+    // (one decode is in flight at a time: the other set is free)
+    cudaEvent_t *const ev = g->ev[g->set = g->done_set == 0 ? 1 : 0];
+    CU(cudaEventRecord(ev[0], g->stream));
     const OfScanPlan plan = of_scan_plan(N, state_len, g->sms);
     CU(of_launch_first_scans(plan, scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, g->sms, blank_score,
                              g->d_tables, g->d_status, g->wait_ns, g->stream));
-    CU(cudaEventRecord(g->ev[1], g->stream));
-    CU(cudaStreamWaitEvent(g->stream2, g->ev[1], 0));
-    CU(cudaEventRecord(g->ev[5], g->stream2));
+    CU(cudaEventRecord(ev[1], g->stream));
+    CU(cudaStreamWaitEvent(g->stream2, ev[1], 0));
+    CU(cudaEventRecord(ev[4], g->stream2));
     CU(of_launch_rest_of_posterior(plan, scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, g->sms, blank_score,
                                    g->d_tables, g->d_status, g->wait_ns, g->stream2));
-    CU(cudaEventRecord(g->ev[6], g->stream2));
+    CU(cudaEventRecord(ev[5], g->stream2));
     CU(of_launch_beam_search(a, g->stream));
-    CU(cudaEventRecord(g->ev[2], g->stream));
-    CU(cudaStreamWaitEvent(g->stream, g->ev[6], 0));
+    CU(cudaEventRecord(ev[2], g->stream));
+    CU(cudaStreamWaitEvent(g->stream, ev[5], 0));
     CU(of_launch_posterior_seq(a, g->stream));
-    CU(cudaEventRecord(g->ev[3], g->stream));
-
-    // results: straight into page-locked caller memory, else through the staging area
-    g->via_stage = !(host_is_pinned(moves) && host_is_pinned(sequence) && host_is_pinned(qstring));
-    if (g->via_stage) {
-        CU(cudaMemcpyAsync(g->h_stage, g->d_results, 3 * nt, cudaMemcpyDeviceToHost, g->stream));
-    } else {
-        CU(cudaMemcpyAsync(moves, g->pub.moves, nt, cudaMemcpyDeviceToHost, g->stream));
-        CU(cudaMemcpyAsync(sequence, g->pub.sequence, nt, cudaMemcpyDeviceToHost, g->stream));
-        CU(cudaMemcpyAsync(qstring, g->pub.qstring, nt, cudaMemcpyDeviceToHost, g->stream));
-    }
-    CU(cudaMemcpyAsync(g->h_status, g->d_status, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-    CU(cudaEventRecord(g->ev[4], g->stream));
+    CU(cudaEventRecord(ev[3], g->stream));
     g->dst_moves = moves;
     g->dst_sequence = sequence;
     g->dst_qstring = qstring;
+    g->stripped[g->set] = false;
     g->pending = true;
     return OPENFISH_B200_OK;
 }
 
 namespace {
-// Waits for the gpubuf's main stream, then looks at the status word its kernels share (copied to
+// Waits for the gpubuf's main stream, then looks at the status word its kernels share (brought to
 // the host by the last operation queued): a raised status is reported and cleared on the device.
 int stream_done_and_status(GpuBuf *g) {
     CU(cudaStreamSynchronize(g->stream));
@@ -329,15 +342,17 @@ extern "C" int ofb_decode_submit_5wide(int T, int N, const void *scores5, int st
     if (!g->d_scores4) CU(cudaMalloc(&g->d_scores4, (size_t)T * N * 4 * ns * sizeof(__half)));
     if (params->on_caller_stream) {
         cudaStream_t caller = static_cast<cudaStream_t>(params->caller_stream);
-        CU(cudaEventRecord(g->ev[7], caller));
-        CU(cudaStreamWaitEvent(g->stream, g->ev[7], 0));
+        CU(cudaEventRecord(g->caller_ev, caller));
+        CU(cudaStreamWaitEvent(g->stream, g->caller_ev, 0));
     }
-    CU(cudaEventRecord(g->ev[8], g->stream));
+    const int set = g->done_set == 0 ? 1 : 0;  // (what the submit below takes)
+    CU(cudaEventRecord(g->ev[set][6], g->stream));
     CU(of_launch_strip_blank(scores5, g->d_scores4, (long long)T * N, state_len, clamp, g->sms, g->stream));
-    g->stripped = true;
     ofb_decode_params_t p = *params;
     p.on_caller_stream = 0;  // (already ordered: the copy above runs on the gpubuf's stream)
-    return ofb_decode_submit(T, N, (int)(4 * ns), g->d_scores4, state_len, &p, gpubuf, moves, sequence, qstring);
+    const int rc = ofb_decode_submit(T, N, (int)(4 * ns), g->d_scores4, state_len, &p, gpubuf, moves, sequence, qstring);
+    g->stripped[set] = true;
+    return rc;
 }
 
 extern "C" int ofb_decode_wait(const openfish_gpubuf_t *gpubuf) {
@@ -346,36 +361,20 @@ extern "C" int ofb_decode_wait(const openfish_gpubuf_t *gpubuf) {
     g->pending = false;
     const int rc = stream_done_and_status(g);
     if (rc != OPENFISH_B200_OK) return rc;
-    const size_t nt = (size_t)g->N * g->T;
     if (g->via_stage) {
+        const size_t nt = (size_t)g->N * g->T;
         memcpy(g->dst_moves, g->h_stage, nt);
-        memcpy(g->dst_sequence, g->h_stage + nt, nt);
-        memcpy(g->dst_qstring, g->h_stage + 2 * nt, nt);
+        memcpy(g->dst_sequence, g->h_stage + stage_pitch(g), nt);
+        memcpy(g->dst_qstring, g->h_stage + 2 * stage_pitch(g), nt);
     }
-    // ms: 0 the scans before the beam search, 1 everything between them and the copies (beam search
-    // with the rest of the posterior beside it, then sequence), 2 copies, 3 all of it; detail: 4 beam
-    // search, 5 the rest of the posterior, 6 sequence (from the later of its two inputs), 7 the
-    // blank-column strip in front of a 5-wide decode (0 otherwise)
-    cudaEventElapsedTime(&g->ms[0], g->ev[0], g->ev[1]);
-    cudaEventElapsedTime(&g->ms[1], g->ev[1], g->ev[3]);
-    cudaEventElapsedTime(&g->ms[2], g->ev[3], g->ev[4]);
-    cudaEventElapsedTime(&g->ms[3], g->ev[0], g->ev[4]);
-    cudaEventElapsedTime(&g->ms[4], g->ev[1], g->ev[2]);
-    cudaEventElapsedTime(&g->ms[5], g->ev[5], g->ev[6]);
-    float from_beam = 0.f, from_fwd = 0.f;
-    cudaEventElapsedTime(&from_beam, g->ev[2], g->ev[3]);
-    cudaEventElapsedTime(&from_fwd, g->ev[6], g->ev[3]);
-    g->ms[6] = from_beam < from_fwd ? from_beam : from_fwd;
-    g->ms[7] = 0.f;
-    if (g->stripped) cudaEventElapsedTime(&g->ms[7], g->ev[8], g->ev[0]);
-    g->stripped = false;
+    g->done_set = g->set;
     return OPENFISH_B200_OK;
 }
 
 extern "C" int ofb_stream_wait_decode(void *stream, const openfish_gpubuf_t *gpubuf) {
     GpuBuf *g = priv(gpubuf);
     if (!g->pending) return OPENFISH_B200_OK;  // nothing in flight: nothing to wait for
-    CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->ev[4], 0));
+    CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->ev[g->set][3], 0));
     return OPENFISH_B200_OK;
 }
 
@@ -390,9 +389,25 @@ extern "C" int ofb_selfcheck_wait(const openfish_gpubuf_t *gpubuf, unsigned limi
     return stream_done_and_status(g);
 }
 
+// 0 the scans before the beam search, 1 everything after them (beam search with the rest of the posterior
+// beside it, then sequence), 2 zero (the last kernel writes the results to the host), 3 all of it; detail:
+// 4 beam search, 5 the rest of the posterior, 6 sequence (from the later of its two inputs), 7 the
+// blank-column strip in front of a 5-wide decode (0 otherwise)
 extern "C" int ofb_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[8]) {
     const GpuBuf *g = priv(gpubuf);
-    for (int i = 0; i < 8; ++i) ms[i] = g->ms[i];
+    for (int i = 0; i < 8; ++i) ms[i] = 0.f;
+    if (g->done_set < 0) return OPENFISH_B200_OK;
+    const cudaEvent_t *ev = g->ev[g->done_set];
+    float from_beam = 0.f, from_rest = 0.f;
+    CU(cudaEventElapsedTime(&ms[0], ev[0], ev[1]));
+    CU(cudaEventElapsedTime(&ms[1], ev[1], ev[3]));
+    CU(cudaEventElapsedTime(&ms[3], ev[0], ev[3]));
+    CU(cudaEventElapsedTime(&ms[4], ev[1], ev[2]));
+    CU(cudaEventElapsedTime(&ms[5], ev[4], ev[5]));
+    CU(cudaEventElapsedTime(&from_beam, ev[2], ev[3]));
+    CU(cudaEventElapsedTime(&from_rest, ev[5], ev[3]));
+    ms[6] = from_beam < from_rest ? from_beam : from_rest;
+    if (g->stripped[g->done_set]) CU(cudaEventElapsedTime(&ms[7], ev[6], ev[0]));
     return OPENFISH_B200_OK;
 }
 

@@ -155,6 +155,8 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
         a.moves = moves_gpu;
         a.sequence = sequence_gpu;
         a.qstring = qstring_gpu;
+        a.host_results[0] = a.host_results[1] = a.host_results[2] = nullptr;
+        a.host_status = nullptr;
         a.states = reinterpret_cast<int *>(base + o_states);
         a.qual = reinterpret_cast<float *>(base + o_qual);
         a.base_probs = reinterpret_cast<float *>(base + o_base);

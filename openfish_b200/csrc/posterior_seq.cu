@@ -20,6 +20,18 @@ namespace {
 constexpr int kBeam = 32;
 constexpr int kWin = 256;  // traceback window, timesteps
 
+// A chunk's row of n bytes to host memory.  Source and destination rows start at the same distance from a
+// 16-byte boundary (a row is chunk * n bytes behind its aligned array).
+__device__ __forceinline__ void row_to_host(unsigned char *to, const unsigned char *from, int n, int tid, int threads) {
+    const int head = min(n, (int)((16u - ((uintptr_t)to & 15u)) & 15u));
+    if (tid < head) to[tid] = from[tid];
+    const int pieces = (n - head) >> 4;
+    for (int i = tid; i < pieces; i += threads)
+        reinterpret_cast<uint4 *>(to + head)[i] = *reinterpret_cast<const uint4 *>(from + head + 16 * i);
+    const int done = head + 16 * pieces;
+    if (tid < n - done) to[done + tid] = from[done + tid];
+}
+
 template <int NS>
 struct PostSmem {
     int part[256];  // block-scan partials of the tail phase
@@ -197,6 +209,17 @@ posterior_seq_kernel(const OfDecodeArgs a) {
         a.qstring[ct + i] = 0;
         a.base_probs[ct + i] = 0.f;
         a.total_probs[ct + i] = 0.f;
+    }
+
+    // The results' way to the host, while other blocks are still at work (a copy after the kernel took
+    // 65 us for 512 chunks, 400 for 4096, 18 for one).
+    if (a.host_status != nullptr) {
+        __syncthreads();
+        row_to_host(a.host_results[0] + ct, a.moves + ct, T, tid, NT);
+        row_to_host(a.host_results[1] + ct, reinterpret_cast<const unsigned char *>(a.sequence) + ct, T, tid, NT);
+        row_to_host(a.host_results[2] + ct, reinterpret_cast<const unsigned char *>(a.qstring) + ct, T, tid, NT);
+        // (every kernel that waits for anything has ended)
+        if (chunk == 0 && tid == 0) *a.host_status = *a.status;
     }
 }
 
