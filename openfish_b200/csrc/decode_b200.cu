@@ -50,7 +50,7 @@ struct GpuBuf {
     int *d_status;
     void *d_scores4;           // 4-wide copy of 5-wide scores, made on the first 5-wide decode (null before)
     int sms;
-    unsigned char *d_results;  // moves | sequence | qstring, N*T bytes each, on 16-byte boundaries
+    unsigned char *d_small;    // the allocation of all device buffers but the two large tensors
     unsigned char *h_stage;    // page-locked, three results of N*T bytes, each on a 16-byte boundary, and a status word
     unsigned char *d_stage;    // the same for the device
     int *h_status;
@@ -104,14 +104,7 @@ int destroy(GpuBuf *g) {
     if (g->pending && g->stream2) cudaStreamSynchronize(g->stream2);
     cudaFree(g->pub.bwd_NTC);
     cudaFree(g->pub.post_NTC);
-    cudaFree(g->d_results);
-    cudaFree(g->pub.beam_vector);
-    cudaFree(g->pub.states);
-    cudaFree(g->pub.qual_data);
-    cudaFree(g->pub.base_probs);
-    cudaFree(g->pub.total_probs);
-    cudaFree(g->d_tables);
-    cudaFree(g->d_status);
+    cudaFree(g->d_small);
     cudaFree(g->d_scores4);
     if (g->h_stage) cudaFreeHost(g->h_stage);
     for (int i = 0; i < 14; ++i)
@@ -174,27 +167,42 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
         // same ten buffers and sizes as the reference (src/decode_cuda.cu:22-45)
         CU(cudaMalloc(&g->pub.bwd_NTC, tens));
         CU(cudaMalloc(&g->pub.post_NTC, tens));
-        CU(cudaMalloc(&g->d_results, 3 * stage_pitch(g)));
-        g->pub.moves = g->d_results;
-        g->pub.sequence = reinterpret_cast<char *>(g->d_results + stage_pitch(g));
-        g->pub.qstring = reinterpret_cast<char *>(g->d_results + 2 * stage_pitch(g));
+        // (everything but the two large tensors in one allocation)
+        size_t bytes = 0;
+        auto piece = [&](size_t n) {
+            const size_t at = bytes;
+            bytes += (n + 255) & ~(size_t)255;
+            return at;
+        };
+        const size_t o_results = piece(3 * stage_pitch(g));
         // reference-sized (8 bytes per beam slot and timestep); this library uses 1 byte of the 8
         // for its packed back-pointers and 128 bytes per chunk behind them for the initial k-mers
-        CU(cudaMalloc(&g->pub.beam_vector, (size_t)8 * N * 32 * (T + 1)));
-        g->d_init_kmers = reinterpret_cast<int *>(static_cast<unsigned char *>(g->pub.beam_vector) +
-                                                  (((size_t)N * 32 * (T + 1) + 255) & ~(size_t)255));
-        CU(cudaMalloc(&g->pub.states, sizeof(int32_t) * nt));
-        CU(cudaMalloc(&g->pub.qual_data, sizeof(float) * nt * 4));
-        CU(cudaMalloc(&g->pub.base_probs, sizeof(float) * nt));
-        CU(cudaMalloc(&g->pub.total_probs, sizeof(float) * nt));
-        CU(cudaMalloc(&g->d_tables, sizeof(ofx::Tables)));
-        CU(cudaMalloc(&g->d_status, sizeof(int)));
+        const size_t o_beam = piece((size_t)8 * N * 32 * (T + 1));
+        const size_t o_states = piece(sizeof(int32_t) * nt), o_qual = piece(sizeof(float) * nt * 4);
+        const size_t o_base = piece(sizeof(float) * nt), o_total = piece(sizeof(float) * nt);
+        const size_t o_tables = piece(sizeof(ofx::Tables)), o_status = piece(sizeof(int));
+        CU(cudaMalloc(&g->d_small, bytes));
+        unsigned char *const d = g->d_small;
+        g->pub.moves = d + o_results;
+        g->pub.sequence = reinterpret_cast<char *>(d + o_results + stage_pitch(g));
+        g->pub.qstring = reinterpret_cast<char *>(d + o_results + 2 * stage_pitch(g));
+        g->pub.beam_vector = d + o_beam;
+        g->d_init_kmers = reinterpret_cast<int *>(d + o_beam + (((size_t)N * 32 * (T + 1) + 255) & ~(size_t)255));
+        g->pub.states = d + o_states;
+        g->pub.qual_data = reinterpret_cast<float *>(d + o_qual);
+        g->pub.base_probs = reinterpret_cast<float *>(d + o_base);
+        g->pub.total_probs = reinterpret_cast<float *>(d + o_total);
+        g->d_tables = reinterpret_cast<ofx::Tables *>(d + o_tables);
+        g->d_status = reinterpret_cast<int *>(d + o_status);
         CU(cudaHostAlloc(&g->h_stage, 3 * stage_pitch(g) + 16, cudaHostAllocMapped));
         CU(cudaHostGetDevicePointer(&g->d_stage, g->h_stage, 0));
         g->h_status = reinterpret_cast<int *>(g->h_stage + 3 * stage_pitch(g));
         *g->h_status = ofd::kStatusOk;
-        ofx::Tables host_tables;
-        ofx::fill_tables(&host_tables);
+        static const ofx::Tables host_tables = [] {
+            ofx::Tables t;
+            ofx::fill_tables(&t);
+            return t;
+        }();
         CU(cudaMemcpy(g->d_tables, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice));
         CU(cudaMemset(g->d_status, 0, sizeof(int)));
         return OPENFISH_B200_OK;
