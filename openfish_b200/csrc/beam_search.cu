@@ -103,9 +103,6 @@ struct BeamSmem {
     alignas(16) float4 step[kBeam];           // step scores of the timestep's candidates, by parent slot
     unsigned char owner[kOwner + 32];         // (+ one spare per lane) hash -> slot + 1 of the beam element owning it
     int init_state[kBeam];
-    double exp2_j[ofx::kExpTab];
-    double rcp_c[ofx::kLogTab];
-    double log_c[ofx::kLogTab];
     alignas(8) uint64_t full[STAGES];
     alignas(8) uint64_t empty[STAGES];
     int abort_flag;
@@ -128,11 +125,6 @@ beam_search_kernel(const OfDecodeArgs a) {
     const int lane = tid & 31;
     const int chunk = blockIdx.x;
     const int T = a.T, N = a.N;
-    for (int i = tid; i < ofx::kExpTab; i += NT) sm.exp2_j[i] = a.tables->exp2_j[i];
-    for (int i = tid; i < ofx::kLogTab; i += NT) {
-        sm.rcp_c[i] = a.tables->rcp_c[i];
-        sm.log_c[i] = a.tables->log_c[i];
-    }
     for (int i = tid; i < (kOwner + 32) / 4; i += NT) reinterpret_cast<uint32_t *>(sm.owner)[i] = 0;
     if (tid == 0) {
         sm.abort_flag = 0;
@@ -181,7 +173,8 @@ beam_search_kernel(const OfDecodeArgs a) {
         return;
     }
     // ------------------------------------------------------------------ beam warp
-    const ofx::TabRef tr = {sm.exp2_j, 1, sm.rcp_c, sm.log_c};
+    // (so seldom needed that the tables stay where they are: a smaller block leaves the forward scan more room)
+    const ofx::TabRef tr = {a.tables->exp2_j, 1, a.tables->rcp_c, a.tables->log_c};
     const uint32_t lt_mask = (1u << lane) - 1u;
     // initial beam: first <= 32 states, in state order, reaching the 32nd largest bwd[0]
     // (src/beam_search.c:151-175).  Radix-select the 32nd largest key bit by bit.
