@@ -406,7 +406,7 @@ struct Ahead {
     }
 };
 using Ahead64 = Ahead<64, 1, 2, 6, 8>;
-using Ahead256 = Ahead<256, 4, 2, 6, 2>;
+using Ahead256 = Ahead<256, 4, 2, 6, 3>;
 
 // ------------------------------------------------------------------------------------------
 // post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,
@@ -495,7 +495,8 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 }
 
 // Where the lines lie (decodes of T = 800, ms, by plan: together / ahead then forward / backward then forward):
-//   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;  320: 1.73 / 1.61 / 1.48
+//   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;
+//                at T = 1666 440: - / 2.59 / 2.65;  512: - / 2.92 / 2.82
 //   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;  592: 1.16 / 1.01 / 1.05
 //   1024 states: 74 chunks 1.42 /  -   / 1.81;  222: 2.69 /  -   / 2.79;  240: 2.98 /  -   / 2.80
 // Two directions on one SM are in each other's way beyond their number (their code is more than an
@@ -504,7 +505,7 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 OfScanPlan of_scan_plan(int N, int state_len, int sms) {
     if (state_len == 5) return 2 * N <= 3 * sms ? OfScanPlan::kTogether : OfScanPlan::kBackwardThenForward;
     if (2 * N <= sms) return OfScanPlan::kTogether;
-    if (state_len == 3 || N <= 2 * sms) return OfScanPlan::kAheadThenForward;
+    if (state_len == 3 || N <= 3 * sms) return OfScanPlan::kAheadThenForward;
     return OfScanPlan::kBackwardThenForward;
 }
 
