@@ -4,7 +4,8 @@
 
 // The decode's kernels, in the order in which they are loaded.
 enum OfKernel : int {
-    kFwd256, kBwd256, kBeam256, kFwd256Many, kSeq256, kBwd256Many, kAhead256, kPosterior256, kBeam256Scaled,
+    kFwd256, kBwd256, kBeam256, kFwd256Many, kFwd256Most, kSeq256, kBwd256Many, kBwd256Most, kAhead256,
+    kPosterior256, kBeam256Scaled,
     kScan1024, kFwd1024, kBeam1024, kSeq1024, kPosterior1024, kBeam1024Scaled, kScan1024Both,
     kAhead64, kFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
     kKernels

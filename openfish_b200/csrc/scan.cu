@@ -615,8 +615,8 @@ scan_spec_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, flo
 }
 
 // Forward scan with the posterior on top: one block per chunk, reads the finished backward scores.
-template <int NS, int SPT, int RING, int COPIES, bool PACKED>
-__global__ void __launch_bounds__(NS / SPT + 96, (NS <= 256 ? 5 : 2))
+template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
+__global__ void __launch_bounds__(NS / SPT + 96, MINB)
 scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__restrict__ bwd,
                            float *__restrict__ post, int T, int N, float stay,
                            const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
@@ -637,9 +637,9 @@ struct Spec {
     }
 };
 
-template <int NS, int SPT, int RING, int COPIES, bool PACKED>
+template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
 struct SpecPosterior {
-    static constexpr auto kern = scan_spec_posterior_kernel<NS, SPT, RING, COPIES, PACKED>;
+    static constexpr auto kern = scan_spec_posterior_kernel<NS, SPT, RING, COPIES, MINB, PACKED>;
     static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, true>);
     static cudaError_t launch(const __half *scores, const float *bwd, float *post, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
@@ -651,11 +651,13 @@ struct SpecPosterior {
 using Spec64 = Spec<64, 2, 8, 4, 12, true>;
 using Spec256 = Spec<256, 4, 6, 16, 4, true>;
 using Spec256Many = Spec<256, 4, 6, 4, 7, true>;
+using Spec256Most = Spec<256, 4, 6, 4, 8, true>;
 using Spec1024 = Spec<1024, 4, 6, 16, 2, false>;
 using Spec1024Both = Spec<1024, 4, 6, 16, 2, true>;
-using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, true>;
-using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, true>;
-using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 16, false>;
+using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, 5, true>;
+using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, 5, true>;
+using SpecPosterior256Most = SpecPosterior<256, 4, 6, 4, 6, true>;
+using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 16, 2, false>;
 
 }  // namespace
 
@@ -668,10 +670,13 @@ cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bw
         // A block of 36 KB for batches that fit the GPU three and a half to the SM beside their beam
         // searches; a larger batch takes one of 30 KB (fewer copies of a table), of which four go with
         // four beam searches: 560 chunks of T = 800 in 1.64 ms instead of 1.96, 2048 of T = 1666 in 10.20
-        // instead of 10.31, but 512 in 3.00 instead of 2.96.
+        // instead of 10.31, but 512 in 3.00 instead of 2.96.  Six of them to the SM instead of five (64
+        // registers) when there are several rounds of blocks: 4096 chunks of T = 800 5.60 instead of 5.75 ms,
+        // 601 of T = 1201 1.65 instead of 1.63.
         case 4:
             if (2 * N <= 7 * sms) return SpecPosterior256::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
-            return SpecPosterior256Many::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
+            if (N <= 10 * sms) return SpecPosterior256Many::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
+            return SpecPosterior256Most::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
         case 5: return SpecPosterior1024::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
     }
@@ -686,11 +691,13 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
         // all of 1024 forward scans found room beside their beam searches (3.06 ms a decode instead of 2.68)
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // Four blocks to the SM (128 registers) as long as that is room enough, else seven (72): what a
-        // block loses is less than what a half empty second round of blocks costs.  740 chunks of T = 1666:
+        // block loses is less than what a half empty second round of blocks costs; eight (64) when there are
+        // several rounds anyway (4096 chunks of T = 800: 3.45 ms instead of 3.54, 601 of T = 1201: 1.09 instead of 1.06).  740 chunks of T = 1666:
         // 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28; 2048: 3.55 instead of 4.20; 512: 1.16 with
         // four, 1.24 with seven.
         case 4:
             if (N <= 4 * sms) return Spec256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+            if (N > 10 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Spec256Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         case 5:  // (both directions: a batch that leaves the GPU room)
             if (bwd && fwd) return Spec1024Both::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
@@ -705,6 +712,8 @@ cudaError_t of_load_scan(int kernel) {
         case kFwd256: return of_load<SpecPosterior256>();
         case kBwd256Many: return of_load<Spec256Many>();
         case kFwd256Many: return of_load<SpecPosterior256Many>();
+        case kFwd256Most: return of_load<SpecPosterior256Most>();
+        case kBwd256Most: return of_load<Spec256Most>();
         case kScan1024: return of_load<Spec1024>();
         case kScan1024Both: return of_load<Spec1024Both>();
         case kFwd1024: return of_load<SpecPosterior1024>();
