@@ -133,7 +133,7 @@ def test_long_chunks(native_lib, oracle_mod):
 
 
 @pytest.mark.parametrize("sl,T,N", [(3, 900, 74), (3, 33, 75), (3, 2, 149), (4, 300, 74), (4, 41, 75), (4, 260, 148),
-                                    (4, 24, 297), (4, 20, 444), (4, 11, 445), (4, 8, 519), (4, 5, 593), (4, 4, 1481), (5, 9, 222), (5, 8, 223), (4, 700, 2)])
+                                    (4, 24, 297), (4, 20, 444), (4, 11, 445), (4, 8, 519), (4, 5, 593), (4, 4, 1481), (5, 9, 222), (5, 8, 223), (5, 7, 297), (4, 700, 2)])
 def test_batches_on_either_side_of_a_change_of_kernels(native_lib, oracle_mod, sl, T, N):
     # the scans of a batch are run together, one ahead of the other or one after the other according to how
     # many chunks there are for the GPU's 148 multiprocessors; odd and even T (groups of two timesteps),
