@@ -151,11 +151,12 @@ posterior_seq_kernel(const OfDecodeArgs a) {
             nb[2 * b] = (st >> 2) + MSB * b;
             nb[2 * b + 1] = ((st << 2) & (NS - 1)) + b;
         }
-        // all nine posteriors are fetched before any is used: one memory round trip, not nine
-        float pv[8];
+        // all nine posteriors are fetched before any is used, the four that lie together at once: one memory
+        // round trip of six requests
         float prob = __ldcg(pr + st);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) pv[k] = __ldcg(pr + nb[k]);
+        const float4 next = __ldcg(reinterpret_cast<const float4 *>(pr + nb[1]));
+        const float pv[8] = {__ldcg(pr + nb[0]), next.x, __ldcg(pr + nb[2]), next.y,
+                             __ldcg(pr + nb[4]), next.z, __ldcg(pr + nb[6]), next.w};
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             bool fresh = nb[k] != st;
