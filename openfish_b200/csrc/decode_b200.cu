@@ -313,7 +313,7 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     CU(of_launch_beam_search(a, g->stream));
     CU(cudaEventRecord(ev[2], g->stream));
     CU(cudaStreamWaitEvent(g->stream, ev[5], 0));
-    CU(of_launch_posterior_seq(a, g->stream));
+    CU(of_launch_posterior_seq(a, g->sms, g->stream));
     CU(cudaEventRecord(ev[3], g->stream));
     g->dst_moves = moves;
     g->dst_sequence = sequence;

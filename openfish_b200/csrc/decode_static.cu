@@ -171,7 +171,7 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
         a.q_scale = options->q_scale;
         a.score_scale = options->temperature;
         e = of_launch_beam_search(a, stream);
-        if (e == cudaSuccess) e = of_launch_posterior_seq(a, stream);
+        if (e == cudaSuccess) e = of_launch_posterior_seq(a, sms, stream);
     }
     int dev_status = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&dev_status, status, sizeof(int), cudaMemcpyDeviceToHost);

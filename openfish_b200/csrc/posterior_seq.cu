@@ -18,7 +18,6 @@
 namespace {
 
 constexpr int kBeam = 32;
-constexpr int kWin = 256;  // traceback window, timesteps
 
 // A chunk's row of n bytes to host memory.  Source and destination rows start at the same distance from a
 // 16-byte boundary (a row is chunk * n bytes behind its aligned array).
@@ -32,23 +31,26 @@ __device__ __forceinline__ void row_to_host(unsigned char *to, const unsigned ch
     if (tid < n - done) to[done + tid] = from[done + tid];
 }
 
-template <int NS>
+template <int NS, int NT>
 struct PostSmem {
-    int part[256];  // block-scan partials of the tail phase
+    int part[NT / 32];  // steps in each warp's timesteps
+    int init_kmers[kBeam];
     // the tail phase's arrays start here and run into the dynamic shared memory behind
     alignas(128) unsigned char tail[128];
 };
 
-constexpr int kPostThreads = 256;
-
-template <int NS>
-__global__ void __launch_bounds__(kPostThreads)
+// What bounds it: in a large batch the posterior's gather, whose 32-byte pieces use half of what a read of
+// the memory brings; in a small one the chain of phases.  1024 threads to a chunk, with the next window's
+// rows on their way: 0.133 ms for 512 chunks of T = 1666 instead of 0.162 with 256 threads that fetch as they
+// go, 0.032 instead of 0.048 for 16, 0.153 instead of 0.217 for 1024 of the 64-state model.
+template <int NS, int NT>
+__global__ void __launch_bounds__(NT)
 posterior_seq_kernel(const OfDecodeArgs a) {
     constexpr int BITS = (NS == 64) ? 6 : (NS == 256 ? 8 : 10);
     constexpr int SL = BITS / 2;
     constexpr int MSB = NS / 4;
-    constexpr int NT = kPostThreads;
-    using Smem = PostSmem<NS>;
+    constexpr int kWin = NT / 2;  // traceback window, timesteps: a thread stages one 16-byte piece of it
+    using Smem = PostSmem<NS, NT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
@@ -73,15 +75,22 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     // shortened eightfold: for every block of 8 rows and each of the 32 slots one could enter it
     // with, all threads first work out where one leaves it (independent short walks); one thread
     // then hops block to block; finally all threads replay their block with the known entry.
+    // The next window's rows are on their way while this one is walked.
+    if (tid < kBeam) sm.init_kmers[tid] = a.init_kmers[(size_t)chunk * kBeam + tid];
+    uint4 piece = make_uint4(0, 0, 0, 0);
+    auto fetch = [&](int hi_r) {
+        const int lo_r = max(1, hi_r - kWin + 1);
+        if (tid < 2 * (hi_r - lo_r + 1)) piece = __ldcg(reinterpret_cast<const uint4 *>(bp_chunk + (size_t)lo_r * kBeam) + tid);
+    };
+    fetch(T);
     int at = 0;
     for (int hi_r = T; hi_r >= 1; hi_r -= kWin) {
         const int lo_r = max(1, hi_r - kWin + 1);
         const int rows = hi_r - lo_r + 1;
         const int nblk = (rows + 7) >> 3;
-        const int n16 = rows * 2;  // 16-byte pieces
-        const uint4 *src = reinterpret_cast<const uint4 *>(bp_chunk + (size_t)lo_r * kBeam);
-        for (int i = tid; i < n16; i += NT) reinterpret_cast<uint4 *>(win)[i] = __ldcg(src + i);
+        if (tid < 2 * rows) reinterpret_cast<uint4 *>(win)[tid] = piece;
         __syncthreads();
+        fetch(hi_r - kWin);
         for (int w = tid; w < nblk * kBeam; w += NT) {
             const int g = w >> 5;
             int e = w & 31;
@@ -109,7 +118,7 @@ posterior_seq_kernel(const OfDecodeArgs a) {
         __syncthreads();
     }
     if (tid == 0) {
-        const int st0 = a.init_kmers[(size_t)chunk * kBeam + at];
+        const int st0 = sm.init_kmers[at];
 #pragma unroll
         for (int i = 0; i < SL; ++i) ext[i] = (unsigned char)((st0 >> (2 * (SL - 1 - i))) & 3);
     }
@@ -120,10 +129,16 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     const int r_lo = 1 + tid * seg, r_hi = min(T, r_lo + seg - 1);
     int local = 0;
     for (int r = r_lo; r <= r_hi; ++r) local += !((path[r] >> 5) & 1);
-    sm.part[tid] = local;
+    int run = local;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const int below = __shfl_up_sync(0xffffffffu, run, d);
+        run += (tid & 31) >= d ? below : 0;
+    }
+    if ((tid & 31) == 31) sm.part[tid >> 5] = run;
     __syncthreads();
-    int run = 0;
-    for (int i = 0; i < tid; ++i) run += sm.part[i];
+    run -= local;
+    for (int w = 0; w < tid >> 5; ++w) run += sm.part[w];
     for (int r = r_lo; r <= r_hi; ++r) {
         const unsigned char b = path[r];
         if (!((b >> 5) & 1)) {
@@ -216,9 +231,12 @@ posterior_seq_kernel(const OfDecodeArgs a) {
     // 65 us for 512 chunks, 400 for 4096, 18 for one).
     if (a.host_status != nullptr) {
         __syncthreads();
-        row_to_host(a.host_results[0] + ct, a.moves + ct, T, tid, NT);
-        row_to_host(a.host_results[1] + ct, reinterpret_cast<const unsigned char *>(a.sequence) + ct, T, tid, NT);
-        row_to_host(a.host_results[2] + ct, reinterpret_cast<const unsigned char *>(a.qstring) + ct, T, tid, NT);
+        constexpr int part = NT / 4;
+        const unsigned char *rows[3] = {a.moves, reinterpret_cast<const unsigned char *>(a.sequence),
+                                        reinterpret_cast<const unsigned char *>(a.qstring)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (tid / part == k) row_to_host(a.host_results[k] + ct, rows[k] + ct, T, tid % part, part);
         // (every kernel that waits for anything has ended)
         if (chunk == 0 && tid == 0) *a.host_status = *a.status;
     }
@@ -226,39 +244,48 @@ posterior_seq_kernel(const OfDecodeArgs a) {
 
 constexpr size_t kMostBytes = 227 * 1024;  // of dynamic shared memory: what a block can have
 
-template <int NS>
+template <int NS, int NT>
 struct Seq {
-    static constexpr auto kern = posterior_seq_kernel<NS>;
+    static constexpr auto kern = posterior_seq_kernel<NS, NT>;
     static constexpr size_t bytes = kMostBytes;
+    static size_t bytes_for(int T) {
+        constexpr size_t win = NT / 2;
+        const size_t Tp = (T + 16) & ~15;
+        return sizeof(PostSmem<NS, NT>) + win * kBeam + (win / 8) * (kBeam + 4) + 8 * Tp + 64;
+    }
+    static cudaError_t launch(const OfDecodeArgs &a, cudaStream_t stream) {
+        const size_t need = bytes_for(a.T);
+        if (need > kMostBytes) return cudaErrorInvalidValue;
+        kern<<<a.N, NT, need, stream>>>(a);
+        return cudaGetLastError();
+    }
 };
 
+// 512 threads for many rounds of blocks: 4096 chunks 0.733 ms instead of 0.748.
 template <int NS>
-cudaError_t launch_post(const OfDecodeArgs &a, cudaStream_t stream) {
-    using Smem = PostSmem<NS>;
-    const int Tp = (a.T + 16) & ~15;
-    const size_t tail = (size_t)kWin * kBeam + (kWin / 8) * (kBeam + 4) + 8 * (size_t)Tp + 64;
-    const size_t bytes = sizeof(Smem) + tail;
-    if (bytes > kMostBytes) return cudaErrorInvalidValue;
-    posterior_seq_kernel<NS><<<a.N, kPostThreads, bytes, stream>>>(a);
-    return cudaGetLastError();
+cudaError_t launch_seq(const OfDecodeArgs &a, int sms, cudaStream_t stream) {
+    return a.N > 14 * sms ? Seq<NS, 512>::launch(a, stream) : Seq<NS, 1024>::launch(a, stream);
 }
 
 }  // namespace
 
-cudaError_t of_launch_posterior_seq(const OfDecodeArgs &a, cudaStream_t stream) {
+cudaError_t of_launch_posterior_seq(const OfDecodeArgs &a, int sms, cudaStream_t stream) {
     switch (a.state_len) {
-        case 3: return launch_post<64>(a, stream);
-        case 4: return launch_post<256>(a, stream);
-        case 5: return launch_post<1024>(a, stream);
+        case 3: return launch_seq<64>(a, sms, stream);
+        case 4: return launch_seq<256>(a, sms, stream);
+        case 5: return launch_seq<1024>(a, sms, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t of_load_posterior_seq(int kernel) {
     switch (kernel) {
-        case kSeq64: return of_load<Seq<64>>();
-        case kSeq256: return of_load<Seq<256>>();
-        case kSeq1024: return of_load<Seq<1024>>();
+        case kSeq64: return of_load<Seq<64, 1024>>();
+        case kSeq64Many: return of_load<Seq<64, 512>>();
+        case kSeq256: return of_load<Seq<256, 1024>>();
+        case kSeq256Many: return of_load<Seq<256, 512>>();
+        case kSeq1024: return of_load<Seq<1024, 1024>>();
+        case kSeq1024Many: return of_load<Seq<1024, 512>>();
         default: return cudaSuccess;
     }
 }

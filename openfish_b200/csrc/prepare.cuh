@@ -8,6 +8,7 @@ enum OfKernel : int {
     kPosterior256, kBeam256Scaled,
     kScan1024, kFwd1024, kFwd1024Many, kBeam1024, kSeq1024, kPosterior1024, kBeam1024Scaled, kScan1024Both, kScan1024Many,
     kAhead64, kFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
+    kSeq256Many, kSeq1024Many, kSeq64Many,
     kKernels
 };
 

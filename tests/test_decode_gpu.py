@@ -142,6 +142,14 @@ def test_batches_on_either_side_of_a_change_of_kernels(native_lib, oracle_mod, s
     check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 300 + N, p_step=0.6), sl, min_identical=1.0)
 
 
+@pytest.mark.parametrize("sl,T,N", [(3, 511, 3), (3, 512, 2), (4, 513, 2), (5, 1025, 2), (3, 16384, 1),
+                                    (3, 256, 2073), (3, 257, 2080)])
+def test_windows_of_the_traceback(native_lib, oracle_mod, sl, T, N):
+    # the traceback goes through its rows in windows of 512, and of 256 in a batch of many rounds
+    from openfish_b200 import synth
+    check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 400 + T, p_step=0.6), sl, min_identical=1.0)
+
+
 @pytest.mark.parametrize("okw", [dict(beam_cut=0.0), dict(beam_cut=1.5), dict(beam_cut=1e6),
                                  dict(q_scale=0.95, q_shift=-0.2), dict(q_scale=3.0, q_shift=10.0)])
 def test_options(native_lib, oracle_mod, okw):
