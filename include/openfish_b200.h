@@ -45,16 +45,17 @@ int openfish_b200_last_status(void);
 const char *openfish_b200_error_text(void);
 
 /* Same work as openfish_decode_gpu, but the results land in buffers the caller owns: three host
- * buffers of N*T bytes each (page-locked memory avoids a staging copy; pageable memory works
- * too).  Nothing is malloc'ed. */
+ * buffers of N*T bytes each.  The last kernel writes them itself if all three are page-locked from
+ * their first byte to their last, each inside one registration or allocation, and start on a 16-byte
+ * boundary; any other memory works too and takes a staging copy.  Nothing is malloc'ed. */
 void openfish_b200_decode_into(int T, int N, int C, const void *scores_TNC, int state_len,
                                const openfish_opt_t *options, const openfish_gpubuf_t *gpubuf,
                                uint8_t *moves, char *sequence, char *qstring);
 
-/* The same split in two: submit enqueues the kernels and the device-to-host copies on the
- * gpubuf's stream and returns at once; wait blocks until they are done and reports the status.
- * One decode may be in flight per gpubuf.  The three host buffers must be page-locked for the
- * copies to be asynchronous. */
+/* The same split in two: submit enqueues the kernels on the gpubuf's streams and returns at once;
+ * wait blocks until they are done, makes the staging copy where the buffers need one, and reports the
+ * status.  One decode may be in flight per gpubuf.  The three host buffers must stay what they were
+ * at submit until wait has returned. */
 void openfish_b200_decode_submit(int T, int N, int C, const void *scores_TNC, int state_len,
                                  const openfish_opt_t *options, const openfish_gpubuf_t *gpubuf,
                                  uint8_t *moves, char *sequence, char *qstring);
