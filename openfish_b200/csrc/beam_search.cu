@@ -147,13 +147,9 @@ beam_search_kernel(const OfDecodeArgs a) {
             const __half *src = a.scores + (size_t)chunk * NS * 4;
             const float *bwd_src = bwd_chunk + NS;
             const size_t beam_stride = (size_t)N * a.C;
-            int issued = 0, stage = 0;
-            uint32_t parity = 1;  // (of the stage's previous release)
-            for (int t = 0; t < T; t += GROUP, ++issued) {
-                if (t >= STAGES * GROUP)
-                    ofd::mbar_wait_bounded(&sm.empty[stage], parity, &sm.abort_flag, a.status, a.wait_ns);
-                if (sm.abort_flag) break;
-                const int rows = T - t < GROUP ? T - t : GROUP;
+            ofd::fill_ring_by_mbar<STAGES>((T + GROUP - 1) / GROUP, sm.full, sm.empty, &sm.abort_flag, a.status, a.wait_ns,
+                                           [&](int g, int stage) {
+                const int rows = min(GROUP, T - g * GROUP);
                 ofd::mbar_arrive_expect_tx(&sm.full[stage], rows * Smem::kSlot);
                 for (int r = 0; r < rows; ++r) {
                     unsigned char *dst = sm.ring[stage * GROUP + r];
@@ -162,13 +158,7 @@ beam_search_kernel(const OfDecodeArgs a) {
                     bwd_src += NS;
                     src += beam_stride;
                 }
-                if (++stage == STAGES) {
-                    stage = 0;
-                    parity ^= 1u;
-                }
-            }
-            // after an abort: the newest copies get a bounded chance to land before the block retires
-            if (sm.abort_flag) ofd::mbar_drain_bounded(sm.full, STAGES, issued, a.wait_ns);
+            });
         }
         return;
     }

@@ -5,6 +5,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "copy_ring.h"
+
 namespace ofd {
 
 // Status codes a kernel can raise in the gpubuf's status word (0 = fine).
@@ -103,6 +105,30 @@ __device__ __forceinline__ void mbar_drain_bounded(uint64_t *bars, int ring, int
             if (global_timer_ns() - t0 > limit_ns) return;
         }
     }
+}
+
+// Wait for copies whether or not the block has given up; `since` (zero before the first look) starts the limit
+// for all of them.
+static __device__ __noinline__ uint64_t mbar_land(uint64_t *bar, uint32_t parity, uint64_t since, uint64_t limit_ns) {
+    while (!mbar_try_wait(bar, parity)) {
+        const uint64_t now = global_timer_ns();
+        if (since == 0) since = now;
+        else if (now - since > limit_ns) break;
+        __nanosleep(64);
+    }
+    return since;
+}
+
+// copy_ring.h's fill_ring by one thread and two mbarriers a stage: full (the copies' bytes) and empty (the
+// readers' release).
+template <int RING, class Issue>
+__device__ __forceinline__ void fill_ring_by_mbar(int groups, uint64_t *full, uint64_t *empty, volatile int *abort_flag,
+                                                  int *status, uint64_t limit_ns, Issue issue) {
+    uint64_t since = 0;  // the first look at copies that had not landed
+    fill_ring(
+        groups, RING, [&](int stage, uint32_t parity) { mbar_wait_bounded(&empty[stage], parity, abort_flag, status, limit_ns); },
+        [&]() { return *abort_flag != 0; }, issue,
+        [&](int stage, uint32_t parity) { since = mbar_land(&full[stage], parity, since, limit_ns); });
 }
 
 // 1-D bulk asynchronous copy global -> this CTA's shared memory, completion counted in bytes

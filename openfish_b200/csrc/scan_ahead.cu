@@ -163,24 +163,14 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             const size_t t_stride = (size_t)N * NS * 4;
             const __half *src = scores + (size_t)chunk * NS * 4 + t_stride * (size_t)Topo::score_row(0, T);
             const ptrdiff_t step = Topo::kForward ? (ptrdiff_t)t_stride : -(ptrdiff_t)t_stride;
-            int issued = 0, stage = 0;
-            uint32_t parity = 1;  // (of the stage's previous release)
-            for (; issued < groups; ++issued) {
-                if (issued >= S) ofd::mbar_wait_bounded(&sm.empty[stage], parity, &sm.abort_flag, status, wait_ns);
-                if (*(volatile int *)&sm.abort_flag) break;
-                const int n = min(E, T - issued * E);
+            ofd::fill_ring_by_mbar<S>(groups, sm.full, sm.empty, &sm.abort_flag, status, wait_ns, [&](int g, int stage) {
+                const int n = min(E, T - g * E);
                 ofd::mbar_arrive_expect_tx(&sm.full[stage], n * Smem::kRowBytes);
                 for (int q = 0; q < n; ++q) {
                     ofd::bulk_g2s(sm.ring[stage][q], src, Smem::kRowBytes, &sm.full[stage]);
                     src += step;
                 }
-                if (++stage == S) {
-                    stage = 0;
-                    parity ^= 1u;
-                }
-            }
-            // after an abort the newest copies get a bounded chance to land before the block retires
-            if (*(volatile int *)&sm.abort_flag) ofd::mbar_drain_bounded(sm.full, S, issued, wait_ns);
+            });
         }
         return;
     }
