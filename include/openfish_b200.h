@@ -46,8 +46,8 @@ const char *openfish_b200_error_text(void);
 
 /* Same work as openfish_decode_gpu, but the results land in buffers the caller owns: three host
  * buffers of N*T bytes each.  The last kernel writes them itself if all three are page-locked from
- * their first byte to their last, each inside one registration or allocation, and start on a 16-byte
- * boundary; any other memory works too and takes a staging copy.  Nothing is malloc'ed. */
+ * their first byte to their last, each inside one registration or allocation; any other memory works
+ * too and takes a staging copy.  Nothing is malloc'ed. */
 void openfish_b200_decode_into(int T, int N, int C, const void *scores_TNC, int state_len,
                                const openfish_opt_t *options, const openfish_gpubuf_t *gpubuf,
                                uint8_t *moves, char *sequence, char *qstring);

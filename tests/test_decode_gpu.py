@@ -217,6 +217,27 @@ def test_results_into_memory_that_is_page_locked_only_in_part(native_lib):
         gb.free()
 
 
+@pytest.mark.parametrize("T,N,offset", [(501, 7, 0), (333, 5, 3), (16, 3, 8), (5, 3, 13), (1, 2, 15)])
+def test_page_locked_results_may_start_anywhere(native_lib, T, N, offset):
+    # three results one behind the other in one page-locked block: the last kernel writes them itself (they are
+    # there when the GPU is done, before decode_wait would copy anything), and nothing next to them
+    import torch
+    from openfish_b200 import synth
+    of = native_lib
+    sc = torch.from_numpy(synth.make_scores(T, N, 3, 93)).cuda()
+    gb = of.gpubuf_init(T, N, 3)
+    base = of.decode_gpu(sc, 3, gpubuf=gb)
+    block = torch.full((offset + 3 * N * T + 16,), 0xA5, dtype=torch.uint8).pin_memory()
+    rows = [block[offset + k * N * T:offset + (k + 1) * N * T].view(N, T) for k in range(3)]
+    of.decode_into(sc, 3, gb, *rows, wait=False)
+    torch.cuda.synchronize()
+    for k, r in zip(("moves", "sequence", "qstring"), rows):
+        assert np.array_equal(r.numpy(), base[k]), k
+    assert bool((block[:offset] == 0xA5).all()) and bool((block[offset + 3 * N * T:] == 0xA5).all())
+    of.decode_wait(gb)
+    gb.free()
+
+
 def test_decodes_from_several_host_threads_and_in_flight(native_lib):
     # a gpubuf per host thread, as the reference's driver does it (src/main.c:23,207): decodes of
     # different batches running at the same time must not disturb each other; nor must two
