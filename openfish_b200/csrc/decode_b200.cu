@@ -146,12 +146,11 @@ int destroy(GpuBuf *g) {
 // launch: kernels that run beside one another get in each other's way in the instruction caches according
 // to where their code has come to lie.  A 512-chunk decode of the 256-state model took 2.96 ms in a process
 // that began with one and 3.10 in one that had decoded 74 chunks before.
-cudaError_t of_prepare_device(int device) {
+// What is loaded and how much shared memory a kernel may have belongs to the current context and ends with it
+// (cudaDeviceReset), so nothing is remembered here: every set of device buffers asks again (2 us).
+cudaError_t of_prepare_device() {
     static std::mutex lock;
-    static bool loaded[64];
-    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> hold(lock);
-    if (loaded[device]) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < kKernels && e == cudaSuccess; ++k) {
         e = of_load_scan(k);
@@ -159,7 +158,6 @@ cudaError_t of_prepare_device(int device) {
         if (e == cudaSuccess) e = of_load_beam_search(k);
         if (e == cudaSuccess) e = of_load_posterior_seq(k);
     }
-    loaded[device] = e == cudaSuccess;
     return e;
 }
 
@@ -175,7 +173,7 @@ extern "C" int ofb_gpubuf_create(int T, int N, int state_len, openfish_gpubuf_t 
     const size_t tens = (size_t)N * (T + 1) * ns * sizeof(float);
     int rc = [&]() -> int {
         CU(cudaGetDevice(&g->device));
-        CU(of_prepare_device(g->device));
+        CU(of_prepare_device());
         CU(cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, g->device));
         // a blocking stream: ordered after work the caller queued on the legacy default
         // stream (where the reference runs), so freshly written scores are seen

@@ -66,7 +66,7 @@ int setup_device(int dev, unsigned char **base_out) {
         }
         ofx::Tables host_tables;
         ofx::fill_tables(&host_tables);
-        e = of_prepare_device(dev);
+        e = of_prepare_device();
         if (e == cudaSuccess) e = cudaMemcpy(p, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             char msg[160];

@@ -25,5 +25,5 @@ cudaError_t of_load_ahead(int kernel);          // scan_ahead.cu
 cudaError_t of_load_beam_search(int kernel);    // beam_search.cu
 cudaError_t of_load_posterior_seq(int kernel);  // posterior_seq.cu
 
-// All of them, once per device (decode_b200.cu); before the first launch on that device.
-cudaError_t of_prepare_device(int device);
+// All of them on the current device (decode_b200.cu); before the first launch in its present context.
+cudaError_t of_prepare_device();
