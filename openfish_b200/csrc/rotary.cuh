@@ -5,6 +5,7 @@
 // What a rotary kernel leaves in page-locked memory when its last block is through: `call` last.
 struct RotaryDone {
     unsigned long long start_ns, end_ns;  // of the kernel, by the device's clock
+    const void *owner;                    // the host's record of this memory (the kernel leaves it alone)
     unsigned call;
 };
 

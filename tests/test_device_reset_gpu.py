@@ -67,6 +67,19 @@ def decode():
     return got
 
 
+def rotary():
+    B, S, H, D, half = 2, 33, 4, 32, 16
+    rng = np.random.default_rng(62)
+    x = rng.standard_normal((B, S, H, D)).astype(np.float16)
+    angle = rng.standard_normal((S, half))
+    p = to_device(x)
+    args = (p, to_device(np.sin(angle).astype(np.float32)), to_device(np.cos(angle).astype(np.float32)), B, S, H, D, half,
+            S * H * D, H * D, D)
+    lib.openfish_rotary_emb_gpu(*args)
+    of._check()
+    return from_device(p, x).tobytes()
+
+
 first = %(case)s()
 ok(rt.cudaDeviceReset())
 assert %(case)s() == first
@@ -76,7 +89,7 @@ print("the same after a reset")
 """
 
 
-@pytest.mark.parametrize("case", ["decode"])
+@pytest.mark.parametrize("case", ["decode", "rotary"])
 def test_calls_before_and_after_a_reset(native_lib, case):
     r = subprocess.run([sys.executable, "-c", CHILD % {"root": ROOT, "case": case}], capture_output=True,
                        text=True, timeout=300)
