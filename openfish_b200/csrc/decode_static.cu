@@ -4,8 +4,8 @@
 // process that hands all free device memory to its own arena at start-up (a later cudaMalloc
 // from a library then fails or fragments the arena), or a pipeline that must not hit the
 // device-wide synchronisation a cudaMalloc / cudaFree implies in the middle of its steady
-// state.  openfish_gpubuf_init does ten cudaMallocs, a cudaMallocHost, a stream and four events,
-// and openfish_decode_gpu three host mallocs per call.  The entry point below needs none of
+// state.  openfish_gpubuf_init does three cudaMallocs and a cudaHostAlloc and makes two streams and
+// fifteen events, and openfish_decode_gpu does three host mallocs per call.  The entry point below needs none of
 // that: every intermediate of the decode (backward scores, posteriors, back-pointers, path
 // states, per-timestep qualities, the arithmetic tables, the status word) lives in ONE
 // file-scope device array of fixed size, the results go to device buffers the caller owns, the
@@ -18,8 +18,8 @@
 //   * all calls on a device share the array: it keeps the previous call's contents (whatever
 //     must start from zero is cleared by the call itself), and two calls that overlap on the
 //     same GPU -- from two host threads -- race.  Serialise them.
-//   * the first call on each device looks up the array's device address and uploads the tables.
-//     Make that first call before starting any stream capture.
+//   * the first call on each device (and after a cudaDeviceReset) loads the kernels and uploads the
+//     tables.  Make that first call before starting any stream capture.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -40,9 +40,13 @@ constexpr size_t kStaticScratchBytes = OPENFISH_B200_STATIC_SCRATCH_BYTES;
 // address; kernels receive the address cudaGetSymbolAddress returns for the current device.
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
-constexpr int kMaxDevices = 64;
-unsigned char *g_base[kMaxDevices];  // device address of the array, per device; null = not set up
 std::mutex g_setup_lock;
+
+// Never launched.  An attribute of it is set once the array of the current context has its tables: the runtime
+// forgets the attribute together with the array's contents when the context ends (cudaDeviceReset), and keeps
+// one for each context, so nothing about a device has to be remembered here.
+__global__ void tables_are_there() {}
+constexpr int kTablesMark = 4096;  // bytes of dynamic shared memory; the default is 48 KB
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -52,30 +56,32 @@ int report(int code, const char *text) {
     return code;
 }
 
-// Once per device, with that device current: resolve the array's address, put the tables at its
-// start.  No allocation: the tables travel from this function's stack.
-int setup_device(int dev, unsigned char **base_out) {
+// The array's address in the current context; the first time there, puts the tables at its start.  No
+// allocation: the tables travel from this function's stack.
+int setup_device(unsigned char **base_out) {
     std::lock_guard<std::mutex> hold(g_setup_lock);
-    if (!g_base[dev]) {
-        unsigned char *p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_static_scratch);
-        if (e != cudaSuccess || !p) {
-            char msg[160];
-            snprintf(msg, sizeof(msg), "cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
-            return report(OPENFISH_B200_ERR_CUDA, msg);
-        }
+    unsigned char *p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_static_scratch);
+    if (e != cudaSuccess || !p) {
+        char msg[160];
+        snprintf(msg, sizeof(msg), "cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+        return report(OPENFISH_B200_ERR_CUDA, msg);
+    }
+    cudaFuncAttributes mark;
+    e = cudaFuncGetAttributes(&mark, tables_are_there);
+    if (e == cudaSuccess && mark.maxDynamicSharedSizeBytes != kTablesMark) {
         ofx::Tables host_tables;
         ofx::fill_tables(&host_tables);
         e = of_prepare_device();
         if (e == cudaSuccess) e = cudaMemcpy(p, &host_tables, sizeof(host_tables), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            char msg[160];
-            snprintf(msg, sizeof(msg), "loading the kernels and uploading the tables failed: %s", cudaGetErrorString(e));
-            return report(OPENFISH_B200_ERR_CUDA, msg);
-        }
-        g_base[dev] = p;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(tables_are_there, cudaFuncAttributeMaxDynamicSharedMemorySize, kTablesMark);
     }
-    *base_out = g_base[dev];
+    if (e != cudaSuccess) {
+        char msg[160];
+        snprintf(msg, sizeof(msg), "loading the kernels and uploading the tables failed: %s", cudaGetErrorString(e));
+        return report(OPENFISH_B200_ERR_CUDA, msg);
+    }
+    *base_out = p;
     return OPENFISH_B200_OK;
 }
 
@@ -123,10 +129,10 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
 
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+    if (e != cudaSuccess || dev < 0)
         return report(OPENFISH_B200_ERR_CUDA, "no usable current CUDA device");
     unsigned char *base = nullptr;
-    const int rc = setup_device(dev, &base);
+    const int rc = setup_device(&base);
     if (rc != OPENFISH_B200_OK) return rc;
 
     const ofx::Tables *tables = reinterpret_cast<const ofx::Tables *>(base + o_tables);

@@ -67,6 +67,14 @@ def decode():
     return got
 
 
+def static():
+    n = 1  # (of the 1024-state model, what the array holds at this length)
+    out = [to_device(np.zeros((n, T), np.uint8)) for _ in range(3)]
+    d = to_device(np.ascontiguousarray(scores[:, :n]))
+    ok(lib.openfish_b200_decode_static(T, n, 4 * 4 ** SL, d, SL, C.byref(opt), *out))
+    return [from_device(o, np.zeros((n, T), np.uint8)).tobytes() for o in out]
+
+
 def rotary():
     B, S, H, D, half = 2, 33, 4, 32, 16
     rng = np.random.default_rng(62)
@@ -89,7 +97,7 @@ print("the same after a reset")
 """
 
 
-@pytest.mark.parametrize("case", ["decode", "rotary"])
+@pytest.mark.parametrize("case", ["decode", "rotary", "static"])
 def test_calls_before_and_after_a_reset(native_lib, case):
     r = subprocess.run([sys.executable, "-c", CHILD % {"root": ROOT, "case": case}], capture_output=True,
                        text=True, timeout=300)
