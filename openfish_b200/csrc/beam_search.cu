@@ -272,6 +272,7 @@ beam_search_kernel(const OfDecodeArgs a) {
         const uint32_t cand_hash = __shfl_sync(0xffffffffu, hash, (cand - 1) & 31);
         int mate = (act && cand > 0 && cand_hash == need) ? cand - 1 : -1;
         const bool odd = __any_sync(0xffffffffu, mate >= 0 || mine_back != lane + 1);
+        __syncwarp();  // (a vote orders no memory: the entries are cleared only after every lane's look-ups)
         sm.owner[own_at] = 0;
         threshold();
         if (__builtin_expect(odd, 0)) {
