@@ -142,6 +142,35 @@ def test_batches_on_either_side_of_a_change_of_kernels(native_lib, oracle_mod, s
     check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 300 + N, p_step=0.6), sl, min_identical=1.0)
 
 
+@pytest.mark.parametrize("sl,many", [(3, 160), (4, 450)])
+def test_an_infinite_score_is_taken_alike_by_every_scan_kernel_and_at_a_bearable_cost(native_lib, sl, many):
+    # from the score on (in either direction) no state's rounding can be certified.  The kernels for small and
+    # for large batches leave the same bits, and the one for small batches takes the exact routine's time for
+    # such rows (1.4 times that of ordinary ones over these timesteps; 3.7 times while it kept going back)
+    import torch
+    from openfish_b200 import synth
+    of = native_lib
+    T = 600
+    sc = torch.from_numpy(synth.make_scores(T, 4, sl, 94)).cuda()
+    inf = sc.clone()
+    inf[T // 2, :, 7] = float("inf")
+
+    def scans(scores):
+        gb = of.gpubuf_init(T, scores.shape[1], sl)
+        ms = []
+        for _ in range(5):
+            of.decode_gpu(scores, sl, gpubuf=gb)
+            ms.append(gb.last_decode_ms()["bwd_scan"])
+        bits = [gb.tensor(n)[:4].view(torch.int32).cpu().numpy() for n in ("bwd_NTC", "post_NTC")]
+        gb.free()
+        return min(ms), bits
+
+    few, few_bits = scans(inf)
+    _, many_bits = scans(inf.repeat(1, (many + 3) // 4, 1).contiguous())
+    assert all(np.array_equal(a, b) for a, b in zip(few_bits, many_bits))
+    assert few < 2.2 * scans(sc)[0]
+
+
 @pytest.mark.parametrize("sl,T,N", [(3, 511, 3), (3, 512, 2), (4, 513, 2), (5, 1025, 2), (3, 16384, 1),
                                     (3, 256, 2073), (3, 257, 2080)])
 def test_windows_of_the_traceback(native_lib, oracle_mod, sl, T, N):
