@@ -103,7 +103,8 @@ void openfish_b200_decode_submit_5wide(void *cuda_stream, int T, int N, const vo
  * backward one, in a small batch both), ms[1] everything between them and the copies (the beam search
  * kernel with the rest of the way to the posterior beside it on a second stream, then the traceback
  * + sequence kernel, which also writes the results to the host), ms[2] zero (there are no copies
- * behind the kernels), ms[3] all of it. */
+ * behind the kernels), ms[3] all of it.  If the events cannot be read the call fails like any other and
+ * the times are zero. */
 void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]);
 
 /* The same four numbers followed by: ms[4] beam search kernel, ms[5] what ran beside it (forward scan

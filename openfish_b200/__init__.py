@@ -155,6 +155,7 @@ class GpuBuf:
     def last_decode_ms(self):
         ms = (C.c_float * 8)()
         lib().openfish_b200_last_decode_detail_ms(self.ptr, ms)
+        _check()
         return dict(bwd_scan=ms[0], rest=ms[1], d2h=ms[2], total=ms[3], beam_search=ms[4],
                     fwd_scan=ms[5], posterior_seq=ms[6], strip_blank=ms[7])
 

@@ -248,8 +248,8 @@ void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]) 
         raise_error(__func__, OPENFISH_B200_ERR_ARGUMENT, "gpubuf and ms must not be NULL");
         return;
     }
-    float all[8];
-    ofb_last_decode_ms(gpubuf, all);
+    float all[8] = {0};
+    if (backend_failed(__func__, ofb_last_decode_ms(gpubuf, all))) memset(all, 0, sizeof(all));
     memcpy(ms, all, 4 * sizeof(float));
 }
 
@@ -259,7 +259,7 @@ void openfish_b200_last_decode_detail_ms(const openfish_gpubuf_t *gpubuf, float 
         raise_error(__func__, OPENFISH_B200_ERR_ARGUMENT, "gpubuf and ms must not be NULL");
         return;
     }
-    ofb_last_decode_ms(gpubuf, ms);
+    if (backend_failed(__func__, ofb_last_decode_ms(gpubuf, ms))) memset(ms, 0, 8 * sizeof(float));
 }
 
 int openfish_b200_kernels_per_decode(void) { return 4; }
