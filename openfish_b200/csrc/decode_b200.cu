@@ -23,6 +23,7 @@
 #include "scan.cuh"
 #include "exact_math.cuh"
 #include "beam_post.cuh"
+#include "cpu_relax.h"
 #include "host_view.h"
 #include "of_device.cuh"
 #include "prepare.cuh"
@@ -526,7 +527,7 @@ extern "C" int ofb_rotary(void *x, const void *sin_t, const void *cos_t, int bat
     // The kernel's own report first (nothing is nearer); work queued before it may keep it for longer, and
     // an error would keep it for good: then the stream is asked.
     volatile unsigned *seen = &r->done->call;
-    for (int spin = 0; *seen != call && spin < 20000; ++spin) __builtin_ia32_pause();
+    for (int spin = 0; *seen != call && spin < 20000; ++spin) cpu_relax();
     if (*seen != call) CU(cudaStreamSynchronize(0));
     if (*seen != call) return fail(OPENFISH_B200_ERR_CUDA, "the rotary kernel did not report its end");
     std::atomic_thread_fence(std::memory_order_acquire);
