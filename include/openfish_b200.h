@@ -114,7 +114,9 @@ void openfish_b200_last_decode_ms(const openfish_gpubuf_t *gpubuf, float ms[4]);
 void openfish_b200_last_decode_detail_ms(const openfish_gpubuf_t *gpubuf, float ms[8]);
 
 /* Device time, in milliseconds, of the calling thread's last openfish_rotary_emb_gpu call: from the start
- * of the kernel's first block to the end of its last, by the device's clock. */
+ * of the kernel's block 0 to the end of its last block, by the device's clock, which a B200 advances in
+ * steps of 32 ns.  The launch and the way from the last block to the host are not in it: a pair of CUDA
+ * events around the call shows 10 to 20 us more.  Zero if the call had nothing to do. */
 float openfish_b200_last_rotary_ms(void);
 
 /* Self-check of the arithmetic the scans rely on.  Backward scores are made bit-identical to the

@@ -71,6 +71,25 @@ def test_four_pairs_at_a_time(native_lib, oracle_mod, B, S, H, D, half):
     assert close(out, ref)
 
 
+@pytest.mark.parametrize("B,S,H,D,half", [(1, 1, 1, 8, 3), (2, 64, 16, 64, 32), (8, 1666, 16, 64, 32)])
+def test_the_kernels_own_time_lies_within_the_call(native_lib, B, S, H, D, half):
+    # by the device's clock: longer than nothing, no longer than the call as the host sees it, and a call with
+    # nothing to do leaves no time behind
+    import time
+
+    import torch
+    x = torch.randn((B, S, H, D), device="cuda").half()
+    sin, cos = (torch.from_numpy(t).cuda() for t in tables(S, half))
+    for _ in range(4):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        native_lib.rotary_emb_gpu(x, sin, cos, B, S, H, D, half, S * H * D, H * D, D)
+        wall = 1e3 * (time.perf_counter() - t0)
+        assert 0.0 < native_lib.last_rotary_ms() < wall
+    native_lib.rotary_emb_gpu(x, sin, cos, 0, S, H, D, half, S * H * D, H * D, D)
+    assert native_lib.last_rotary_ms() == 0.0
+
+
 def test_full_size_against_the_oracle(native_lib, oracle_mod):
     # the encoder's whole packed QKV tensor [32][1666][3][8][64] against
     # the CPU routine on the same fp16 values, every element
