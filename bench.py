@@ -140,9 +140,11 @@ class ClockSampler(threading.Thread):
 
 
 def measure_rotary(of, dev, cpu_too=False):
-    """openfish_rotary_emb_gpu on fp16 [32][1666][3][8][64] (Q and K heads in one call): device time
-    by the device's clock, first block to last, rotating over four tensors
-    (655 MB) so that no call finds its input in the 126 MB L2."""
+    """openfish_rotary_emb_gpu on fp16 [32][1666][3][8][64] (Q and K heads in one call), rotating over
+    four tensors (655 MB) so that no call finds its input in the 126 MB L2.  Two times: `ms` by a pair of
+    CUDA events around the whole call, as the comparator's is taken (launch and the host's wait included),
+    and `kernel_ms` by the kernel itself, from the start of its first block to the end of its last
+    (launch and drain left out, read in steps of 32 ns)."""
     import numpy as np
     import torch
     B, S, H, D = 32, 1666, 8, 64
@@ -155,19 +157,27 @@ def measure_rotary(of, dev, cpu_too=False):
     args = (B, S, 2 * H, D, half, S * 3 * H * D, 3 * H * D, D)
     for x in xs:
         of.rotary_emb_gpu(x, sin, cos, *args)
-    reps, total, wall = 20, 0.0, 0.0
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    reps, wall, by_events, kernel = 20, 0.0, [], 0.0
     for i in range(reps):
         torch.cuda.synchronize()
+        ev[0].record()  # on the legacy default stream, where the call launches
         w0 = time.perf_counter()
         of.rotary_emb_gpu(xs[i % 4], sin, cos, *args)
         wall += time.perf_counter() - w0
-        total += of.last_rotary_ms()  # taken by the kernel itself
-    ms = total / reps
+        ev[1].record()
+        torch.cuda.synchronize()
+        by_events.append(ev[0].elapsed_time(ev[1]))
+        kernel += of.last_rotary_ms()
+    ms, kernel_ms = statistics.median(by_events), kernel / reps
     nbytes = 2 * B * S * 2 * H * D * 2 + 2 * S * half * 4
     peak, _ = measured_peak()
-    out = {"shape": "fp16 [32][1666][3][8][64], nheads=16", "ms": ms, "algorithmic_bytes": nbytes,
-            "achieved_gbs": nbytes / (ms * 1e-3) / 1e9, "frac_of_measured_hbm": nbytes / (ms * 1e-3) / 1e9 / peak,
-            "call_wall_ms": 1e3 * wall / reps, "calls": reps}
+    gbs = nbytes / (kernel_ms * 1e-3) / 1e9
+    out = {"shape": "fp16 [32][1666][3][8][64], nheads=16", "ms": ms, "kernel_ms": kernel_ms,
+           "timing": "ms: CUDA events around the call, median (the records of earlier versions had events around the "
+                     "kernel alone); kernel_ms: device clock, first block to last, mean",
+           "algorithmic_bytes": nbytes, "kernel_achieved_gbs": gbs, "kernel_frac_of_measured_hbm": gbs / peak,
+           "call_wall_ms": 1e3 * wall / reps, "calls": reps}
     if cpu_too:
         # the reference's CPU routine on the same values widened to float32 (it works on float32),
         # all host cores (it caps its threads at the batch size, src/nn_cpu.c:95)
@@ -265,6 +275,14 @@ def timed_decodes(of, scores, state_len, steps, warmup=3):
     return med, float(res[0].sum())
 
 
+def parts_ms(ms):
+    """A decode's parts as GpuBuf.last_decode_ms times them, under names that hold for every batch size: a small
+    batch runs both scans before the beam search and only the posterior beside it, a large one the backward
+    scan before and the forward scan with the posterior beside.  The last part writes the results to the host."""
+    return {"scans_before_beam_search": ms["bwd_scan"], "beam_search": ms["beam_search"],
+            "beside_beam_search": ms["fwd_scan"], "sequence_and_results": ms["posterior_seq"]}
+
+
 def other_model(of, dev, state_len, t, n, seed, peak):
     """One more model/shape with the same kernels, scores resident: ms per decode, chunks/s and the
     whole-decode roofline on that shape's own algorithmic bytes."""
@@ -275,7 +293,7 @@ def other_model(of, dev, state_len, t, n, seed, peak):
     gbs = chunk_bytes(state_len, t) * n / (med["total"] * 1e-3) / 1e9
     return {"state_len": state_len, "T": t, "N": n, "ms_per_decode": med["total"],
             "chunks_per_sec": n / (med["total"] * 1e-3), "bases_per_sec": bases / (med["total"] * 1e-3),
-            "kernel_ms": {k: med[k] for k in ("bwd_scan", "fwd_scan", "beam_search", "posterior_seq", "d2h")},
+            "kernel_ms": parts_ms(med),
             "roofline_whole_decode": {"achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
                                       "algorithmic_bytes_per_chunk": chunk_bytes(state_len, t)}}
 
@@ -563,8 +581,8 @@ def main():
             "timing": "CUDA events recorded by the library on its own stream, summed over steps, max over ranks",
             "bases_per_sec": bases * args.steps / dev_s,
             "wall_ms_per_step": 1e3 * wall_s / args.steps,
-            "kernel_ms": {k: per[k] for k in ("bwd_scan", "fwd_scan", "beam_search", "posterior_seq", "d2h")},
-            "kernel_overlap": "fwd_scan (forward scan + posterior) runs on a second stream beside beam_search; the others are sequential",
+            "kernel_ms": parts_ms(per),
+            "kernel_overlap": "beside_beam_search runs on a second stream beside beam_search; the others are sequential",
             "roofline": {"bound": "hbm", "kernel": dom, "launches_per_decode": len(launches),
                          "avg_launch_ms": dom_ms, "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": ncu_traffic(dom), "peak_source": peak_src,
