@@ -121,8 +121,9 @@ float openfish_b200_last_rotary_ms(void);
 
 /* Self-check of the arithmetic the scans rely on.  Backward scores are made bit-identical to the
  * reference CPU decoder's by an fp32 evaluation that certifies its own result, with an exact FP64
- * routine behind it; the certificate rests on error bounds of two hardware approximations.  This
- * call measures them on the current GPU over their whole domains (about a second): err[0] = largest
+ * routine behind it; the certificate rests on error bounds of two hardware approximations (and, for
+ * the 256-state model's small and medium batches, on those of the first and of a table of logarithms that
+ * is computed on the host).  This call measures the two on the current GPU over their whole domains (about a second): err[0] = largest
  * relative error of ex2.approx.ftz.f32 on [-126, 0], err[1] = largest absolute error of
  * lg2.approx.ftz.f32 on [1, 8).  Returns OK when both are within the bounds below, ERR_ARITH when
  * not (results could then differ from the reference's in the last bit), ERR_CUDA/ERR_ALLOC on

@@ -33,8 +33,8 @@ namespace ofd {
 
 constexpr float kLseEps = 1.3487e-6f;  // 2^-19.5
 // The same with the logarithm out of a table (lse5_guess_pairs) instead of lg2.approx: the table's
-// error and the truncation after the third term, below 2^-26 each, take the place of the 1.96.
-// Sum 10.2; 11.2 = 2^-19.77.
+// error and the truncation after the third term, below 2^-26 each (tests/test_exact_math_host.py goes through
+// the floats), take the place of the 1.96.  Sum 10.2; 11.2 = 2^-19.77.
 constexpr float kGuessEps = 1.12e-6f;
 
 __device__ __forceinline__ float ex2_approx(float x) {

@@ -74,3 +74,31 @@ extern "C" void host_lse5_many(const float *v, const float *guess, int n, float 
         confirmed[i] = ofx::lse5_confirm(v + 5 * i, guess[i], tr);
     }
 }
+
+// The pairs (1/c, log c) behind the fp32 logarithm of fast_lse.cuh, and that logarithm with its roundings (the
+// device's packed multiply, subtract, add and fma round as the host's do).
+extern "C" int host_log_pairs(float *rcp, float *log_c) {
+    for (int i = 0; i < ofx::kLogTab; ++i) {
+        rcp[i] = tables()->rcp_f[i];
+        log_c[i] = tables()->log_f[i];
+    }
+    return ofx::kLogTab;
+}
+extern "C" double host_log_pair_worst(uint32_t first_bits, uint32_t last_bits, uint32_t step) {
+    double worst = 0.0;
+    for (uint64_t b = first_bits; b <= last_bits; b += step) {
+        const uint32_t bits = (uint32_t)b;
+        float s;
+        memcpy(&s, &bits, 4);
+        const uint32_t i = (bits >> 17) - (127u << 6);
+        const float u = fmaf(s, tables()->rcp_f[i], -1.0f);
+        const float third = u * (1.f / 3.f);
+        const float less = third - 0.5f;
+        const float w = fmaf(less, u, 1.0f);
+        const float l1p = u * w;
+        // (the sum with log c is left unrounded: the budget counts that rounding by itself)
+        const double off = fabs(((double)tables()->log_f[i] + (double)l1p) - log((double)s));
+        if (off > worst) worst = off;
+    }
+    return worst;
+}

@@ -114,6 +114,29 @@ def test_backward_scan_bit_exact_on_reference_golden(host, oracle_mod):
     assert np.array_equal(out, ref)
 
 
+def test_logarithm_pairs_keep_the_certificates_budget(host):
+    # fast_lse.cuh certifies floats of the scan that runs ahead with kGuessEps = 1.12e-6, in which the table and
+    # the truncation after the third term (with the terms' own roundings) count for 2^-26 each.  A certified state
+    # is never checked again, so the bound has to hold for every float: all edges of the 192 intervals and every
+    # 61st float of [1, 8) here (largest over all of them: 2^-25.92).
+    import ctypes
+    fp = np.ctypeslib.ndpointer(np.float32, flags="C_CONTIGUOUS")
+    host.host_log_pairs.argtypes = [fp, fp]
+    host.host_log_pair_worst.restype = C.c_double
+    host.host_log_pair_worst.argtypes = [ctypes.c_uint32] * 3
+    rcp, log_c = np.zeros(192, np.float32), np.zeros(192, np.float32)
+    assert host.host_log_pairs(rcp, log_c) == 192
+    # log c is a multiple of 2^-11, so that adding it to a score is exact from 2^-11 * 2^23 downwards
+    assert np.array_equal(np.rint(log_c.astype(np.float64) * 2048), log_c.astype(np.float64) * 2048)
+    assert np.abs(np.log(rcp.astype(np.float64)) + log_c).max() < 2.0 ** -26
+    one, eight, interval = 0x3F800000, 0x41000000, 1 << 17
+    worst = host.host_log_pair_worst(one, eight - 1, 61)
+    for first in range(one, eight, interval):
+        worst = max(worst, host.host_log_pair_worst(first, first + 64, 1),
+                    host.host_log_pair_worst(first + interval - 65, first + interval - 1, 1))
+    assert worst < 2.0 ** -25
+
+
 def test_second_tier_accuracy(host):
     from decimal import Decimal, getcontext
     getcontext().prec = 50
