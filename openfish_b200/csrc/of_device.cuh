@@ -32,10 +32,7 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
                  "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// The same by the threads whose flag is set, without a branch.
+// An arrival by the threads whose flag is set, without a branch.
 __device__ __forceinline__ void mbar_arrive_if(bool flag, uint64_t *bar) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%1];\n\t}"
                  ::"r"((int)flag), "r"(smem_u32(bar)) : "memory");

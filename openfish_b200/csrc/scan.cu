@@ -86,12 +86,13 @@ __device__ __forceinline__ void thread_store(float *smem_row, float *gmem_row, i
 // fwd is zero: the log partition function is the same for every row, so exponents stay in range).
 template <int NS>
 struct PosteriorRow {
+    static_assert(NS >= 128, "four states a lane and access");
     static constexpr int PERL = NS / 32;
-    static constexpr int VEC = PERL >= 4 ? 4 : PERL;
+    static constexpr int VEC = 4;
     static constexpr int NV = PERL / VEC;
     // two states in each arithmetic instruction: a 512-chunk decode of 256 states in 2.79 ms instead of 2.82, but
     // one of 256 chunks of 1024 states in 5.14 instead of 4.98
-    static constexpr bool kPacked = VEC > 1 && PERL <= 8;
+    static constexpr bool kPacked = PERL <= 8;
 
     __device__ static float row_max(const float *row, int lane) {
         float m = -3.0e38f;
@@ -99,15 +100,8 @@ struct PosteriorRow {
         return ofd::warp_max(m);
     }
     __device__ static void load(float *d, const float *p) {
-        if constexpr (VEC == 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(p);
-            d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-        } else if constexpr (VEC == 2) {
-            const float2 v = *reinterpret_cast<const float2 *>(p);
-            d[0] = v.x; d[1] = v.y;
-        } else {
-            d[0] = *p;
-        }
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
     __device__ static void emit(const float *fwd_row, const float *bwd_row, float *post_row, float m0, int lane) {
         const float kLog2e = 1.4426950408889634f;
@@ -142,7 +136,6 @@ struct PosteriorRow {
         const float inv = 1.0f / part;
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-            float *p = post_row + (q * 32 + lane) * VEC;
             float *x = e + q * VEC;
             if constexpr (kPacked) {
 #pragma unroll
@@ -152,12 +145,7 @@ struct PosteriorRow {
 #pragma unroll
                 for (int k = 0; k < VEC; ++k) x[k] *= inv;
             }
-            if constexpr (VEC == 4)
-                *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
-            else if constexpr (VEC == 2)
-                *reinterpret_cast<float2 *>(p) = make_float2(x[0], x[1]);
-            else
-                *p = x[0];
+            *reinterpret_cast<float4 *>(post_row + (q * 32 + lane) * VEC) = make_float4(x[0], x[1], x[2], x[3]);
         }
     }
 };
@@ -367,7 +355,7 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
         return;
     }
 
-    if (POST && warp == NW + 2) {
+    if constexpr (POST) if (warp == NW + 2) {
         // ------------------------------------------------------------------ posterior warp
         const float *bwd_chunk = bwd_in + (size_t)chunk * (size_t)(T + 1) * NS;
         const float m0 = PosteriorRow<NS>::row_max(bwd_chunk, lane);
@@ -624,7 +612,7 @@ scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__res
     spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, true, PACKED>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
 }
 
-// The kernels are described once, for loading (of_prepare_scans) and for launching.
+// The kernels are described once, for loading (of_load_scan) and for launching.
 template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
 struct Spec {
     static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB, PACKED>;

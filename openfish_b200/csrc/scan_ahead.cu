@@ -80,7 +80,8 @@ struct AheadSmem {
     static constexpr int H = E * (S + 1);  // rows kept: a row is overwritten only after it has gone out
     alignas(128) unsigned char ring[S][E][kRowBytes];
     alignas(16) float rows[H][NS];
-    alignas(8) ofd::LogPair log_f[ofd::kLogPairs];
+    static constexpr bool kLogTable = NS > 64;  // the logarithm out of a table (fast_lse.cuh)
+    alignas(8) ofd::LogPair log_f[kLogTable ? ofd::kLogPairs : 1];
     uint32_t mask[2][W][32];          // by group parity and scan thread: bit SPT*q + k, timestep q, state k
     int verdict[2][E];                // by group parity and timestep: a guess was wrong
     unsigned short marked[E][64];     // a timestep's marked states, when a lane has more than one
@@ -145,7 +146,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     for (int i = tid; i < ofx::kLogTab; i += NT) {
         sm.rcp_c[i] = tables->rcp_c[i];
         sm.log_c[i] = tables->log_c[i];
-        sm.log_f[i] = {tables->rcp_f[i], tables->log_f[i]};
+        if constexpr (Smem::kLogTable) sm.log_f[i] = {tables->rcp_f[i], tables->log_f[i]};
     }
     for (int i = tid; i < NS; i += NT) sm.rows[0][i] = 0.f;
     for (int i = tid; i < 2 * W * 32; i += NT) (&sm.mask[0][0][0])[i] = 0;
@@ -330,7 +331,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
                 } else {
                     float v[SPT][5];
                     thread_terms<Topo, SPT>(in, piece, j, k0, stay, v, res);
-                    bad |= ofd::lse5_guess_pairs<SPT, (NS > 64)>(v, res, sm.log_f) << (q * SPT);
+                    bad |= ofd::lse5_guess_pairs<SPT, Smem::kLogTable>(v, res, sm.log_f) << (q * SPT);
                 }
                 if (q == 0 && back) break;
                 // (timesteps past the end are taken like any other, on leftover scores: their rows lie

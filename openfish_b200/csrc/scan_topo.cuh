@@ -32,9 +32,9 @@ struct BwdTopo {
     // known only at run time: selects instead of strided shared-memory reads
     template <int SPT>
     __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
+        static_assert(SPT == 2 || SPT == 4, "two or four states a thread");
         if (SPT == 4) return half_of(w[2 * b + (k >> 1)], k & 1);
-        const uint32_t x = (k0 & 2) ? w[2 * b + 1] : w[2 * b];
-        return SPT == 2 ? half_of(x, k) : half_of(x, k0 & 1);
+        return half_of(k0 ? w[2 * b + 1] : w[2 * b], k);
     }
     __device__ static int j_of(int s) { return s % NJ; }
     __device__ static int k_of(int s) { return s / NJ; }
@@ -59,11 +59,10 @@ struct FwdTopo {
     __device__ static int half_index(int k, int b) { return 4 * k + b; }
     template <int SPT>
     __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
+        static_assert(SPT == 2 || SPT == 4, "two or four states a thread");
         const int c = b >> 1;
         if (SPT == 4) return half_of(w[2 * k + c], b & 1);
-        if (SPT == 2) return half_of(k0 ? w[4 + 2 * k + c] : w[2 * k + c], b & 1);
-        const uint32_t x = (k0 & 2) ? ((k0 & 1) ? w[6 + c] : w[4 + c]) : ((k0 & 1) ? w[2 + c] : w[c]);
-        return half_of(x, b & 1);
+        return half_of(k0 ? w[4 + 2 * k + c] : w[2 * k + c], b & 1);
     }
     __device__ static int j_of(int s) { return s >> 2; }
     __device__ static int k_of(int s) { return s & 3; }
