@@ -276,7 +276,12 @@ struct Seq {
     }
 };
 
-// 512 threads for many rounds of blocks: 4096 chunks 0.733 ms instead of 0.748.
+// 1024 threads shorten a chunk's chain of phases, 512 keep more chunks' gathers under way: many rounds of blocks
+// want the latter.  ms with 1024 / 512 threads: 256 states, T = 1666, 16 chunks 0.032 / 0.038, 296 0.098 / 0.102, 512
+// 0.131 / 0.139; T = 800, 600 chunks 0.091 / 0.085, 2072 0.236 / 0.211, 4096 0.427 / 0.382; 64 states, T = 800, 1036
+// chunks 0.090 / 0.088, 2072 0.152 / 0.145, 8000 0.500 / 0.467; 1024 states, T = 400, 600 chunks 0.062 / 0.057, 2072
+// 0.149 / 0.141, 4096 0.267 / 0.253.  From 4 chunks to the SM on 512 are the better, by at most 0.5 % of a
+// decode (25 us of 5.06 ms at 14), and the line lies at 14.
 template <int NS>
 cudaError_t launch_seq(const OfDecodeArgs &a, int sms, cudaStream_t stream) {
     return a.N > 14 * sms ? Seq<NS, 512>::launch(a, stream) : Seq<NS, 1024>::launch(a, stream);

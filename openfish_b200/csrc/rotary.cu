@@ -4,16 +4,18 @@
 // for every (batch, position, head) the pairs (i, i + rotary_half) of the head vector are
 // rotated by the angle whose cosine/sine sit at [position][i] of two fp32 tables:
 //   o0 = x0*cos - x1*sin,  o1 = x0*sin + x1*cos   (fp32 math, fp16 storage).
-// The op is pure HBM streaming (read + write of the rotated part of x; the encoder's tensor at the
-// rate of a copy), so a thread moves V halves per access: it rotates V consecutive pairs of two
+// The op is pure HBM streaming (read + write of the rotated part of x; the encoder's tensor at
+// 0.88 of a copy's rate), so a thread moves V halves per access: it rotates V consecutive pairs of two
 // heads with the same V angles, and a grid-stride loop over positions keeps every SM busy whatever
 // the shape.  V is 8 (16-byte accesses) where the sizes and pointers allow it, else 4 (8-byte ones:
 // a quarter of an 80-wide head); what allows neither takes a scalar kernel with the same arithmetic.
 //
-// A small call is bound by what surrounds the kernel.  The last block to finish writes the kernel's
+// A call is bound by what surrounds the kernel as well.  The last block to finish writes the kernel's
 // start and end times and the call's number to page-locked memory, where the caller looks for them:
 // 9 us for launch and wait together, against 18 with two timing events, a stream synchronisation
-// and the events' difference (64 positions of two sequences: 21.5 -> 13.6 us for the whole call).
+// and the events' difference (64 positions of two sequences: 21.5 -> 13.6 us for the whole call).  The report makes the
+// kernel itself longer, since each block waits for its own stores first: 38 us instead of 32 for the encoder's
+// tensor, whose call all the same takes 50 us instead of 55.
 #include <cuda_fp16.h>
 #include <stdint.h>
 
@@ -159,9 +161,10 @@ void launch_vec(const RotArgs &a, int sm_count, cudaStream_t stream) {
     const dim3 block(bx, 256 / bx);
     const long long positions = (long long)a.batch * a.seqlen;
     long long blocks = (positions + block.y - 1) / block.y;
-    // Eight blocks an SM stream a tensor that comes from HBM (32 x 1666 x 16 heads of 64: 38 us, 43 with
-    // four, 42 with 32); one that the L2 holds is over sooner with fewer blocks to start and to end
-    // (7 x 1201 x 10 heads of 80: 5.6 us with four, 7.4 with eight).
+    // Every block costs its start and its report, and many of them keep more loads under way.  The kernel with
+    // four / eight blocks to the SM, by the bytes that are rotated, in us: 13.6 MB 6.7 / 6.6, 17.1 MB 7.4 / 8.3,
+    // 20.5 MB 8.5 / 8.9, 27.3 MB 10.2 / 10.0, 34.1 MB 11.9 / 11.4, 54.6 MB 17.4 / 15.7, 109 MB 41.4 / 36.7 (42 with 32
+    // blocks); the same order with inputs that come from HBM.
     const long long bytes = 4LL * positions * a.nheads * a.rotary_half;
     const long long cap = (long long)sm_count * (bytes < (32LL << 20) ? 4 : 8);
     if (blocks > cap) blocks = cap;

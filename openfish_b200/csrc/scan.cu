@@ -657,12 +657,13 @@ cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bw
     const __half *s = static_cast<const __half *>(scores_fp16);
     if (T < 1) return cudaErrorInvalidValue;
     switch (state_len) {
-        // A block of 36 KB for batches that fit the GPU three and a half to the SM beside their beam
-        // searches; a larger batch takes one of 30 KB (fewer copies of a table), of which four go with
-        // four beam searches: 560 chunks of T = 800 in 1.64 ms instead of 1.96, 2048 of T = 1666 in 10.20
-        // instead of 10.31, but 512 in 3.00 instead of 2.96.  Six of them to the SM instead of five (64
-        // registers) when there are several rounds of blocks: 4096 chunks of T = 800 5.60 instead of 5.75 ms,
-        // 601 of T = 1201 1.65 instead of 1.63.
+        // Of blocks with 36 KB an SM holds seven together with beam searches (20 KB): four of either would need
+        // 512 bytes more than it has.  So a batch whose forward scans and beam searches are at most seven to the
+        // SM has them all resident, and a larger one takes blocks of 30 KB (fewer copies of a table).  This
+        // kernel beside the beam search, T = 800, large / small blocks: 500 chunks 0.796 / 0.815 ms, 518 0.797 /
+        // 0.812, 540 1.120 / 0.817, 592 1.130 / 0.822.  Six of them to the SM instead of five (64 registers)
+        // when there are several rounds of blocks, five / six: 1300 chunks 1.938 / 2.027 ms, 1480 2.130 / 2.088,
+        // 1600 2.409 / 2.292, 3000 4.244 / 4.169.
         case 4:
             if (2 * N <= 7 * sms) return SpecPosterior256::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
             if (N <= 10 * sms) return SpecPosterior256Many::launch(s, bwd, post, T, N, stay, tables, status, wait_ns, stream);
@@ -685,10 +686,11 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
         // all of 1024 forward scans found room beside their beam searches (3.06 ms a decode instead of 2.68)
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // Four blocks to the SM (128 registers) as long as that is room enough, else seven (72): what a
-        // block loses is less than what a half empty second round of blocks costs; eight (64) when there are
-        // several rounds anyway (4096 chunks of T = 800: 3.45 ms instead of 3.54, 601 of T = 1201: 1.09 instead of 1.06).  740 chunks of T = 1666:
-        // 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28; 2048: 3.55 instead of 4.20; 512: 1.16 with
-        // four, 1.24 with seven.
+        // block loses is less than what a half empty second round of blocks costs: 740 chunks of T = 1666
+        // 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28; 512: 1.16 with four, 1.24 with seven.  Eight (64)
+        // for many rounds; the line is the forward scan's, so that a batch has the thrifty blocks of both
+        // kernels or of neither.  T = 800, seven / eight: 1300 chunks 1.330 / 1.342 ms, 1480 1.470 / 1.498, 1600
+        // 1.499 / 1.568, 2072 1.865 / 1.839, 3000 2.689 / 2.616.
         case 4:
             if (N <= 4 * sms) return Spec256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             if (N > 10 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
