@@ -62,6 +62,14 @@ __device__ __forceinline__ float fold2_fast(float x, float y, bool &sure) {
     return adds ? lo : m;
 }
 
+// x plus an fp16, widened (exactly) and added with one rounding, in one instruction  (Alone no faster; beside the
+// forward scan of 1024 chunks of 64 states 1.13 ms instead of 1.15.)
+__device__ __forceinline__ float add_half(float x, __half h) {
+    float r;
+    asm("add.f32.f16 %0, %1, %2;" : "=f"(r) : "h"(__half_as_ushort(h)), "f"(x));
+    return r;
+}
+
 // CRC32C over two input bits, table form of src/beam_search.c:103-115:
 // crc' = (crc >> 2) ^ tab[(crc ^ bits) & 3], tab = {0, 0x417B1DBC, 0x82F63B78, 0xC38D26C4}.
 __device__ __forceinline__ uint32_t crc_tab2(uint32_t x) {
@@ -248,11 +256,13 @@ beam_search_kernel(const OfDecodeArgs a) {
         float c0, c1, c2, c3, c4;
         {
             // (float)score * score_scale, rounded before it is added (src/beam_search.c:233-234)
-            auto scaled = [&](__half h) { return SCALED ? __fmul_rn(__half2float(h), a.score_scale) : __half2float(h); };
-            c0 = __fadd_rn(__fadd_rn(score, scaled(s0)), bw.x);
-            c1 = __fadd_rn(__fadd_rn(score, scaled(s1)), bw.y);
-            c2 = __fadd_rn(__fadd_rn(score, scaled(s2)), bw.z);
-            c3 = __fadd_rn(__fadd_rn(score, scaled(s3)), bw.w);
+            auto plus = [&](float x, __half h) {
+                return SCALED ? __fadd_rn(x, __fmul_rn(__half2float(h), a.score_scale)) : add_half(x, h);
+            };
+            c0 = __fadd_rn(plus(score, s0), bw.x);
+            c1 = __fadd_rn(plus(score, s1), bw.y);
+            c2 = __fadd_rn(plus(score, s2), bw.z);
+            c3 = __fadd_rn(plus(score, s3), bw.w);
             c4 = __fadd_rn(__fadd_rn(score, a.stay), bs);
         }
         // pruning threshold (src/beam_search.c:320-381): best - ln(beam_cut); if more than 32

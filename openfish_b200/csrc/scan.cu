@@ -52,7 +52,7 @@ __device__ __forceinline__ void thread_terms(const float *in, const unsigned cha
     for (int k = 0; k < SPT; ++k) {
         v[k][0] = (own ? own[k] : in[Topo::state(j, k0 + k)]) + stay;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) v[k][b + 1] = x[b] + Topo::template score<SPT>(w, k0, k, b);
+        for (int b = 0; b < 4; ++b) v[k][b + 1] = Topo::template plus_score<SPT>(x[b], w, k0, k, b);
     }
 }
 

@@ -58,7 +58,7 @@ __device__ __forceinline__ void thread_terms(const float *in, const Piece &piece
     for (int k = 0; k < SPT; ++k) {
         v[k][0] = own[k] + stay;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) v[k][b + 1] = x[b] + Topo::template score<SPT>(piece.w, k0, k, b);
+        for (int b = 0; b < 4; ++b) v[k][b + 1] = Topo::template plus_score<SPT>(x[b], piece.w, k0, k, b);
     }
 }
 

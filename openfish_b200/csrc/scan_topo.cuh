@@ -5,11 +5,15 @@
 
 namespace scan_topo {
 
-// One fp16 out of a 32-bit word, widened.  Going through __half2 lets the conversion pick its
-// half of the register directly instead of shifting it out first.
-__device__ __forceinline__ float half_of(uint32_t word, int odd) {
-    const __half2 h = *reinterpret_cast<const __half2 *>(&word);
-    return odd ? __high2float(h) : __low2float(h);
+// x plus one fp16 out of a 32-bit word: widened (exactly) and added with one rounding, in one instruction (a
+// conversion and an addition before: a fifth of a state's instructions that are not exponentials.  256 states,
+// T = 1666, a decode of 592 chunks 2.762 ms instead of 2.808, of 1024 4.78 instead of 4.87; 64 states, 1024 chunks
+// 2.56 instead of 2.60).
+__device__ __forceinline__ float add_half(float x, uint32_t word, int odd) {
+    float r;
+    if (odd) asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %1;\n\tadd.f32.f16 %0, b, %2;\n\t}" : "=f"(r) : "r"(word), "f"(x));
+    else asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %1;\n\tadd.f32.f16 %0, a, %2;\n\t}" : "=f"(r) : "r"(word), "f"(x));
+    return r;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -31,10 +35,10 @@ struct BwdTopo {
     // the same out of the piece held as eight words, slot k0 + k with k0 (a multiple of SPT)
     // known only at run time: selects instead of strided shared-memory reads
     template <int SPT>
-    __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
+    __device__ static float plus_score(float x, const uint32_t (&w)[8], int k0, int k, int b) {
         static_assert(SPT == 2 || SPT == 4, "two or four states a thread");
-        if (SPT == 4) return half_of(w[2 * b + (k >> 1)], k & 1);
-        return half_of(k0 ? w[2 * b + 1] : w[2 * b], k);
+        if (SPT == 4) return add_half(x, w[2 * b + (k >> 1)], k & 1);
+        return add_half(x, k0 ? w[2 * b + 1] : w[2 * b], k);
     }
     __device__ static int j_of(int s) { return s % NJ; }
     __device__ static int k_of(int s) { return s / NJ; }
@@ -58,11 +62,11 @@ struct FwdTopo {
     }
     __device__ static int half_index(int k, int b) { return 4 * k + b; }
     template <int SPT>
-    __device__ static float score(const uint32_t (&w)[8], int k0, int k, int b) {
+    __device__ static float plus_score(float x, const uint32_t (&w)[8], int k0, int k, int b) {
         static_assert(SPT == 2 || SPT == 4, "two or four states a thread");
         const int c = b >> 1;
-        if (SPT == 4) return half_of(w[2 * k + c], b & 1);
-        return half_of(k0 ? w[4 + 2 * k + c] : w[2 * k + c], b & 1);
+        if (SPT == 4) return add_half(x, w[2 * k + c], b & 1);
+        return add_half(x, k0 ? w[4 + 2 * k + c] : w[2 * k + c], b & 1);
     }
     __device__ static int j_of(int s) { return s >> 2; }
     __device__ static int k_of(int s) { return s & 3; }
