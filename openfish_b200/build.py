@@ -17,7 +17,7 @@ CLI_SRC = os.path.join(HERE, "cli", "openfish_cli.c")
 CLI = os.path.join(HERE, "bin", "openfish")  # the command-line driver, linked against LIB
 CMP_SRC = os.path.join(HERE, "cli", "compare_blob.c")
 CMP = os.path.join(HERE, "bin", "compare_blob")  # tensor-file comparison in the reference's format
-CU = ["scan.cu", "scan_ahead.cu", "beam_search.cu", "posterior_seq.cu", "rotary.cu", "decode_b200.cu", "decode_static.cu",
+CU = ["scan.cu", "scan_ahead.cu", "scan_warp.cu", "beam_search.cu", "posterior_seq.cu", "rotary.cu", "decode_b200.cu", "decode_static.cu",
       "selfcheck.cu", "adaptor.cu"]
 CC = ["openfish_api.c"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -156,6 +156,7 @@ cudaError_t of_prepare_device() {
     for (int k = 0; k < kKernels && e == cudaSuccess; ++k) {
         e = of_load_scan(k);
         if (e == cudaSuccess) e = of_load_ahead(k);
+        if (e == cudaSuccess) e = of_load_warp(k);
         if (e == cudaSuccess) e = of_load_beam_search(k);
         if (e == cudaSuccess) e = of_load_posterior_seq(k);
     }

@@ -7,7 +7,7 @@ enum OfKernel : int {
     kFwd256, kBwd256, kBeam256, kFwd256Many, kFwd256Most, kSeq256, kBwd256Many, kBwd256Most, kAhead256,
     kPosterior256, kBeam256Scaled,
     kScan1024, kFwd1024, kFwd1024Many, kBeam1024, kSeq1024, kPosterior1024, kBeam1024Scaled, kScan1024Both, kScan1024Many,
-    kAhead64, kFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
+    kAhead64, kFwd64, kWarpBwd64, kWarpFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
     kSeq256Many, kSeq1024Many, kSeq64Many,
     kKernels
 };
@@ -22,6 +22,7 @@ cudaError_t of_load() {
 // Each loads the kernel if it is one of its file's, and else does nothing.
 cudaError_t of_load_scan(int kernel);           // scan.cu
 cudaError_t of_load_ahead(int kernel);          // scan_ahead.cu
+cudaError_t of_load_warp(int kernel);           // scan_warp.cu
 cudaError_t of_load_beam_search(int kernel);    // beam_search.cu
 cudaError_t of_load_posterior_seq(int kernel);  // posterior_seq.cu
 

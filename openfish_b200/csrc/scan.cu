@@ -12,7 +12,8 @@
 // backward scan first (the beam search waits for it) and the forward scan beside the beam search,
 // which leaves most issue slots free.  For the 256- and 1024-state models the forward scan also
 // forms the posterior (a warp of its own per block, see PosteriorRow) and its scores never leave the
-// chip; for the 64-state model they go to HBM for the kernel that forms the posterior.
+// chip; for the 64-state model they go to HBM for the kernel that forms the posterior (and batches of more
+// than three chunks to the SM have scan_warp.cu).
 //
 // Shape of a block.  In either direction the four states that share j also share their four
 // neighbour inputs, and their 16 transition scores are one contiguous 32-byte piece of the score
@@ -682,8 +683,7 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
                             uint64_t wait_ns, cudaStream_t stream) {
     const __half *s = static_cast<const __half *>(scores_fp16);
     switch (state_len) {
-        // two states a thread and few copies of a table: with one state a thread and 16 copies, not
-        // all of 1024 forward scans found room beside their beam searches (3.06 ms a decode instead of 2.68)
+        // (up to three chunks to the SM; scan_warp.cu has the kernel for more.)  Two states a thread
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // Four blocks to the SM (128 registers) as long as that is room enough, else seven (72): what a
         // block loses is less than what a half empty second round of blocks costs: 740 chunks of T = 1666

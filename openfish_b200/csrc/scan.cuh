@@ -14,7 +14,8 @@ namespace ofx { struct Tables; }
 enum class OfScanPlan {
     kTogether,           // both in one launch, the posterior by a kernel of its own
     kAheadThenForward,   // the backward one by of_launch_ahead, the forward one afterwards (beside the beam search)
-    kBackwardThenForward // both by scan.cu's kernels
+    kBackwardThenForward,// both by scan.cu's kernels
+    kWarps               // both by scan_warp.cu's kernels, a warp to a chunk (the 64-state model)
 };
 OfScanPlan of_scan_plan(int N, int state_len, int sms);
 
@@ -32,6 +33,12 @@ cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bw
 // model.  (scan_ahead.cu)
 cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, float stay,
                             const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream);
+
+// Backward scan, and forward scan with the posterior, of the 64-state model by one warp a chunk.  (scan_warp.cu)
+cudaError_t of_launch_warp_backward(const void *scores_fp16, float *bwd, int T, int N, float stay, const ofx::Tables *tables,
+                                    int *status, uint64_t wait_ns, cudaStream_t stream);
+cudaError_t of_launch_warp_forward_posterior(const void *scores_fp16, const float *bwd, float *post, int T, int N, float stay,
+                                             const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream);
 
 // post holds the forward rows and gets softmax_s(fwd + bwd) in their place.  (scan_ahead.cu)
 cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int state_len, cudaStream_t stream);

@@ -29,50 +29,11 @@
 #include "of_device.cuh"
 #include "prepare.cuh"
 #include "scan.cuh"
-#include "scan_topo.cuh"
+#include "scan_piece.cuh"
 
 namespace {
 
 using namespace scan_topo;
-
-// The 16 scores of the four states that share j: 32 consecutive bytes of the score row.
-struct Piece {
-    uint32_t w[8];
-    __device__ __forceinline__ Piece(const unsigned char *row, int j) { load(row, j); }
-    __device__ __forceinline__ void load(const unsigned char *row, int j) {
-        const uint4 lo = *reinterpret_cast<const uint4 *>(row + 32 * j);
-        const uint4 hi = *reinterpret_cast<const uint4 *>(row + 32 * j + 16);
-        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
-        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
-    }
-};
-
-// Terms of the SPT states (j, k0 .. k0+SPT-1) of one thread; `own` holds those states of row `in`
-// (what the thread computed a timestep ago).
-template <class Topo, int SPT>
-__device__ __forceinline__ void thread_terms(const float *in, const Piece &piece, int j, int k0, float stay,
-                                             float (*v)[5], const float *own) {
-    float x[4];
-    Topo::shared_inputs(in, j, x);
-#pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-        v[k][0] = own[k] + stay;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) v[k][b + 1] = Topo::template plus_score<SPT>(x[b], piece.w, k0, k, b);
-    }
-}
-
-template <class Topo, int SPT>
-__device__ __forceinline__ void thread_store(float *dst, int j, int k0, const float *res) {
-    if constexpr (Topo::kForward && SPT == 4) {
-        *reinterpret_cast<float4 *>(dst + 4 * j) = make_float4(res[0], res[1], res[2], res[3]);
-    } else if constexpr (Topo::kForward && SPT == 2) {
-        *reinterpret_cast<float2 *>(dst + 4 * j + k0) = make_float2(res[0], res[1]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) dst[Topo::state(j, k0 + k)] = res[k];
-    }
-}
 
 template <int NS, int W, int E, int S>
 struct AheadSmem {
@@ -94,30 +55,6 @@ struct AheadSmem {
     alignas(8) uint64_t empty[S];     // those rows gone out
     int abort_flag;
 };
-
-// Scores from which on guesses are made: one in twelve states is then marked, one in a thousand wrong.
-constexpr float kGuessFrom = 512.f;
-
-// Every state by the exact routine, judged by one of a row's scores: too small, or no finite number (then none of
-// the row's states is certified, every group would be gone back to, and a batch with one infinite score took 1.4
-// times what the kernel that lists its states takes: 300 chunks of T = 1000 3.70 ms instead of 2.43).
-__device__ __forceinline__ bool exact_for_all(float score) {
-    const uint32_t from = __float_as_uint(kGuessFrom), infinity = 0x7f800000u;
-    return (__float_as_uint(score) & 0x7fffffffu) - from >= infinity - from;
-}
-
-// All states of a thread by the exact routine; out of line (the first hundred timesteps and redone
-// ones come here), so everything is passed in registers.
-template <class Topo, int SPT>
-__device__ __noinline__ float4 exact_step(const float *in, const unsigned char *row, int j, int k0, float stay,
-                                          float4 own, const double *exp2_j, const double *rcp_c, const double *log_c) {
-    float v[SPT][5], out[SPT];
-    const float o[4] = {own.x, own.y, own.z, own.w};
-    thread_terms<Topo, SPT>(in, Piece(row, j), j, k0, stay, v, o);
-    const ofx::TabRef tr = {exp2_j, 1, rcp_c, log_c};
-    ofx::lse5_batch_exact<SPT>(v, out, tr);
-    return make_float4(out[0], SPT > 1 ? out[1 % SPT] : 0.f, SPT > 2 ? out[2 % SPT] : 0.f, SPT > 2 ? out[3 % SPT] : 0.f);
-}
 
 template <int ID, int THREADS>
 __device__ __forceinline__ void named_sync() {
@@ -496,7 +433,9 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 // Where the lines lie (decodes of T = 800, ms, by plan: together / ahead then forward / backward then forward):
 //   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;
 //                at T = 1666 440: - / 2.59 / 2.65;  512: - / 2.92 / 2.82
-//   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;  592: 1.16 / 1.01 / 1.05
+//   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;
+//                ahead then forward / a warp to a chunk: 200 0.79 / 0.87;  444 0.896 / 0.906;  592 0.98 / 0.92;
+//                1500 2.18 / 1.61;  at T = 1666 1024 2.58 / 2.22;  4096 9.21 / 6.92
 //   1024 states: 74 chunks 1.42 /  -   / 1.81;  222: 2.69 /  -   / 2.79;  240: 2.98 /  -   / 2.80
 // Two directions on one SM are in each other's way beyond their number (their code is more than an
 // instruction cache holds), which is why "together" ends where every block has an SM to itself, except for
@@ -504,13 +443,14 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 OfScanPlan of_scan_plan(int N, int state_len, int sms) {
     if (state_len == 5) return 2 * N <= 3 * sms ? OfScanPlan::kTogether : OfScanPlan::kBackwardThenForward;
     if (2 * N <= sms) return OfScanPlan::kTogether;
-    if (state_len == 3 || N <= 3 * sms) return OfScanPlan::kAheadThenForward;
-    return OfScanPlan::kBackwardThenForward;
+    if (N <= 3 * sms) return OfScanPlan::kAheadThenForward;
+    return state_len == 3 ? OfScanPlan::kWarps : OfScanPlan::kBackwardThenForward;
 }
 
 cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bwd, float *post, int T, int N,
                                   int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                   uint64_t wait_ns, cudaStream_t stream) {
+    if (plan == OfScanPlan::kWarps) return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
     if (plan == OfScanPlan::kBackwardThenForward || state_len == 5)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
@@ -520,6 +460,8 @@ cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bw
 cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, const float *bwd, float *post, int T,
                                         int N, int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                         uint64_t wait_ns, cudaStream_t stream) {
+    if (plan == OfScanPlan::kWarps)
+        return of_launch_warp_forward_posterior(scores, bwd, post, T, N, stay, tables, status, wait_ns, stream);
     if (plan != OfScanPlan::kTogether) {
         // (a row of the 64-state model is too little work for a warp-wide reduction per chunk and timestep)
         if (state_len != 3)

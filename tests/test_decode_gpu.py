@@ -171,6 +171,30 @@ def test_an_infinite_score_is_taken_alike_by_every_scan_kernel_and_at_a_bearable
     assert few < 2.2 * scans(sc)[0]
 
 
+@pytest.mark.parametrize("T,N", [(1, 445), (7, 445), (8, 446), (9, 447), (16, 445), (23, 1000), (400, 445)])
+def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod, T, N):
+    # 64 states, more than three chunks to the multiprocessor: groups of eight timesteps, whole and ragged, T long
+    # enough for guesses to be made and to be wrong
+    from openfish_b200 import synth
+    check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 500 + T, p_step=0.6), 3, min_identical=1.0)
+
+
+@pytest.mark.parametrize("infinite", [False, True])
+def test_a_warp_each_leaves_the_bits_that_small_batches_get(native_lib, infinite):
+    # backward scores, posterior (whose sums are added up in one order everywhere) and what follows from them, up to
+    # 56 chunks to the multiprocessor; with an infinite score no state is certified from there on
+    import torch
+    from openfish_b200 import synth
+    sc = synth.make_scores(331, 5, 3, 77, p_step=0.5)
+    if infinite:
+        sc[160, :, 7] = np.inf
+    few = gpu_decode(native_lib, sc, 3)
+    for copies in (90, 1640):
+        many = gpu_decode(native_lib, np.tile(sc, (1, copies, 1)), 3)
+        for k in few:
+            assert np.array_equal(few[k].view(np.uint8), many[k][-5:].view(np.uint8)), (k, copies)
+
+
 @pytest.mark.parametrize("sl,T,N", [(3, 511, 3), (3, 512, 2), (4, 513, 2), (5, 1025, 2), (3, 16384, 1),
                                     (3, 256, 2073), (3, 257, 2080)])
 def test_windows_of_the_traceback(native_lib, oracle_mod, sl, T, N):
