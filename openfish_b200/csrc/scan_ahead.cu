@@ -10,10 +10,11 @@
 // scores have grown) needs the value-exact routine, a chain of some 450 cycles on its own.  The scan
 // warps never wait for it: such a state gets the likelier of its two candidate floats, a bit in its
 // thread's mask says so, and the scan goes on.  Timesteps come in groups of E; while the scan warps work
-// on a group, E checker warps recompute the marked states of the group before, a timestep each, and
-// their verdict is looked at in the group after.  Was a guess wrong (one timestep in sixty), the scan
-// goes back to the group it was made in, takes that timestep with the exact routine for every state and
-// carries on from there.  What reaches HBM is what the exact routine alone would have produced.  While
+// on a group, E checker warps recompute the marked states of the group before, a timestep each, put those
+// whose guess was wrong right in their row, and their verdict is looked at in the group after.  Was a guess
+// wrong (one timestep in sixty), the scan goes back and carries on behind the first such timestep; the rows
+// behind it, which followed from the wrong value, and whatever has been put right in them are written
+// again.  What reaches HBM is what the exact routine alone would have produced.  While
 // the scores are small and the float grid fine, guesses are too many and too often wrong: every state
 // goes through the exact routine until the scores have passed kGuessFrom.
 //
@@ -174,7 +175,8 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             if (g < 0 || g >= groups) m = 0;
             const int g0 = g < 0 ? 0 : g;
             const int h0 = (g0 * E + q) % H;
-            const float *in = sm.rows[h0], *res = sm.rows[h0 + 1 == H ? 0 : h0 + 1];
+            const float *in = sm.rows[h0];
+            float *out_row = sm.rows[h0 + 1 == H ? 0 : h0 + 1];
             const unsigned char *row = sm.ring[g0 % S][q];
             bool wrong = false;
             // bit `bit` of lane l's marks
@@ -183,31 +185,34 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
                 const int s = Topo::state(t % Topo::NJ, (t / Topo::NJ) * SPT + bit % SPT);
                 float v[5];
                 terms_of<Topo>(s, in, row, stay, v);
-                const float guess = res[s];
+                const float guess = out_row[s];
                 const float x = ofx::lse5_exact(v, tr);
-                wrong = wrong || (mine && __float_as_uint(x) != __float_as_uint(guess));
+                // (Nobody else writes this row before the next group's end.  Where an earlier timestep turns out
+                // wrong too, or the scan is going back right now, the row is taken again.)
+                if (mine && __float_as_uint(x) != __float_as_uint(guess)) {
+                    wrong = true;
+                    out_row[s] = x;
+                }
             };
             uint32_t owners = __ballot_sync(0xffffffffu, m != 0);
             if (owners) {
                 if (__any_sync(0xffffffffu, (m & (m - 1u)) != 0)) {
-                    int n = 0;
                     do {
-                        const int to = n + __popc(owners & lt_mask);
-                        if (m && to < 64) sm.marked[q][to] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
-                        n += __popc(owners);
-                        m &= m - 1u;
-                        owners = __ballot_sync(0xffffffffu, m != 0);
-                    } while (owners);
-                    __syncwarp();
-                    if (n > 64) {
-                        wrong = true;  // (not worth checking: exactly for all states, then)
-                    } else {
+                        int n = 0;
+                        do {
+                            if (m) sm.marked[q][n + __popc(owners & lt_mask)] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
+                            n += __popc(owners);
+                            m &= m - 1u;
+                            owners = __ballot_sync(0xffffffffu, m != 0);
+                        } while (owners && n + __popc(owners) <= 64);
+                        __syncwarp();
                         for (int first = 0; first < n; first += 32) {
                             const bool mine = first + lane < n;
                             const int e = sm.marked[q][mine ? first + lane : 0];
                             check(mine, e & 31, e >> 5);
                         }
-                    }
+                        __syncwarp();
+                    } while (owners);
                 } else {
                     check(m != 0, lane, m ? __ffs(m) - 1 : 0);
                 }
@@ -227,10 +232,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     int g = 0, stage = 0;
     uint32_t parity = 0;
     int ignore = 2;  // verdicts to come that are about nothing
-    // timesteps of group `exact_of` that go through the exact routine for all states: those found wrong
-    // so far (they add up, or two wrong guesses in one group would take turns for ever)
-    uint32_t exact = 0;
-    int exact_of = -1;
+    int from = 0;    // the group's first timestep to be taken: behind a corrected one when the scan has gone back
     bool all = true;  // what exact_for_all said a group ago
     ofd::mbar_wait_bounded(&sm.full[0], 0u, &sm.abort_flag, status, wait_ns);
     Piece piece(ring, j);
@@ -246,7 +248,6 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         const uint32_t next_parity = next ? parity : parity ^ 1u;
         const unsigned char *ring_next = next ? ring + E * Smem::kRowBytes : sm.ring[0][0];
         const float probe = rows[0];
-        const uint32_t how = all ? ~0u : (g == exact_of ? exact : 0u);
         const int n = T - g * E;  // timesteps left
         const bool ready = g + 1 >= groups || ofd::mbar_try_wait(&sm.full[next], next_parity);
         const bool back = ignore == 0 && wrong != 0;
@@ -254,9 +255,10 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         if (g < groups) {
 #pragma unroll
             for (int q = 0; q < E; ++q) {
+                if (q < from) continue;
                 const float *in = rows + q * NS;
                 float *nxt = q + 1 < E ? rows + (q + 1) * NS : rows_next;
-                if (__builtin_expect((how >> q) & 1u, 0)) {
+                if (__builtin_expect(all, 0)) {
                     const float4 own = make_float4(res[0], res[1], SPT > 2 ? res[2 % SPT] : 0.f, SPT > 2 ? res[3 % SPT] : 0.f);
                     const float4 x = exact_step<Topo, SPT>(in, ring + q * Smem::kRowBytes, j, k0, stay, own, sm.exp2_j, sm.rcp_c, sm.log_c);
                     res[0] = x.x;
@@ -281,11 +283,10 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             }
         }
         if (__builtin_expect(back, 0)) {
-            // back to the group before the last (only the first wrong timestep is known to be wrong for
-            // certain: what follows it followed from it)
+            // back to the group before the last, behind its first wrong timestep, which the checker has put right
+            // (what follows it followed from it)
             g -= 2;
-            exact = (g == exact_of ? exact : 0u) | (wrong & (0u - wrong));
-            exact_of = g;
+            from = __ffs(wrong);
             ignore = 2;
             par ^= 1;  // (no barrier has been passed)
             if (tid == 0) *(volatile int *)&sm.back = sm.back + 2;
@@ -295,9 +296,9 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             parity = (uint32_t)(g / S) & 1u;
             ring = sm.ring[stage][0];
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) res[k] = rows[Topo::state(j, k0 + k)];
-            piece.load(ring, j);
-            all = exact_for_all(rows[0]);
+            for (int k = 0; k < SPT; ++k) res[k] = (from < E ? rows + from * NS : rows_next)[Topo::state(j, k0 + k)];
+            piece.load(ring + (from < E ? from : 0) * Smem::kRowBytes, j);
+            all = exact_for_all<NS>(rows[0]);
             continue;
         }
         // the group before the last is verified
@@ -307,9 +308,10 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         sm.mask[par][warp][lane] = bad;
         if (!ready) ofd::mbar_wait_slow(&sm.full[next], next_parity, &sm.abort_flag, status, wait_ns);
         piece.load(ring_next, j);
-        all = exact_for_all(probe);
+        all = exact_for_all<NS>(probe);
         named_sync<2, kSync>();
         ++g;
+        from = 0;
         stage = next;
         parity = next_parity;
         ring = ring_next;
@@ -341,8 +343,14 @@ struct Ahead {
         return cudaGetLastError();
     }
 };
-using Ahead64 = Ahead<64, 1, 2, 6, 8>;
-using Ahead256 = Ahead<256, 4, 2, 6, 3>;
+// Groups of four: what a group costs besides its timesteps (250 cycles) is paid half as often as with two, and going
+// back, rare and short, loses less than that.  Both scans with groups of two / three / four / six: one chunk of
+// 64 states, T = 1000, 0.306 / 0.292 / 0.285 / 0.279 ms, 40 chunks of T = 120 0.074 / 0.069 / 0.066 / 0.068; 14 chunks of 256
+// states, T = 1666, 0.640 / 0.593 / 0.572 / -, and the backward scan of 300 chunks 0.948 / 0.885 / 0.872 / -.  (Before values
+// were put right in place: one chunk of 64 states 0.342, 14 of 256 0.640 with two.)  Five stages, so that three
+// blocks of 256 states fit an SM; four come too late (14 chunks 0.844).
+using Ahead64 = Ahead<64, 1, 4, 6, 5>;
+using Ahead256 = Ahead<256, 4, 4, 5, 3>;
 
 // ------------------------------------------------------------------------------------------
 // post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,
@@ -450,7 +458,10 @@ OfScanPlan of_scan_plan(int N, int state_len, int sms) {
 cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bwd, float *post, int T, int N,
                                   int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                   uint64_t wait_ns, cudaStream_t stream) {
-    if (plan == OfScanPlan::kWarps) return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
+    // (the backward scan of 592 chunks of T = 800 0.300 ms by the kernel that runs ahead and 0.354 by a warp each, of 740
+    // 0.376 and 0.395, of 1024 of T = 1666 0.79 and 0.74)
+    if (plan == OfScanPlan::kWarps && N > 5 * sms)
+        return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
     if (plan == OfScanPlan::kBackwardThenForward || state_len == 5)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);

@@ -149,7 +149,7 @@ scan_warp_kernel(const __half *__restrict__ scores, float *__restrict__ out, con
             const float *in = sm.rows[wrap(at + q)];
             const unsigned char *row = sm.ring[stage][q];
             float *gmem_out = out_chunk + (ptrdiff_t)Topo::out_row(g * K + q, T) * NS;
-            const bool all = exact_for_all(in[0]);
+            const bool all = exact_for_all<NS>(in[0]);
             uint32_t mask = 0;  // bit SPT*q + k: state k of timestep q is a guess
             Piece piece(row, j);
 #pragma unroll 1
