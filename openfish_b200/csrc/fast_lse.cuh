@@ -83,35 +83,6 @@ __device__ __forceinline__ bool lse5_try_fast(const float v[5], float &out) {
 
 namespace ofd {
 
-// K fast evaluations stage by stage.  out[k] is the certified result where ok[k], and otherwise
-// the better of the two candidate floats (the one nearest to max + log(sum) as estimated), to be
-// confirmed or corrected by the value-exact routine.
-template <int K>
-__device__ __forceinline__ void lse5_fast_guess(const float (*v)[5], float *out, bool *ok) {
-    const float kLog2e = 1.4426950408889634f;
-    float m[K], e[K][5], s[K], l[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        m[k] = max5(v[k]);
-#pragma unroll
-    for (int i = 0; i < 5; ++i)
-#pragma unroll
-        for (int k = 0; k < K; ++k) e[k][i] = ex2_approx((v[k][i] - m[k]) * kLog2e);
-#pragma unroll
-    for (int k = 0; k < K; ++k) s[k] = ((e[k][0] + e[k][1]) + (e[k][2] + e[k][3])) + e[k][4];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        l[k] = ln_1to8(s[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const float lo = m[k] + (l[k] - kLseEps);
-        const float hi = m[k] + (l[k] + kLseEps);
-        out[k] = m[k] + l[k];
-        ok[k] = lo == hi;  // (a NaN sum makes both ends NaN: never accepted)
-    }
-}
-
 // Two floats in a register pair, for the packed additions and multiplications of sm_100 (each half is
 // an ordinary rounded operation; a pair costs one issue slot).
 typedef unsigned long long f32x2;

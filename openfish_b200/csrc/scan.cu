@@ -189,12 +189,18 @@ struct SpecSmem {
     // the state's number (32 bytes), so that the checker's chain starts with one round trip to
     // shared memory instead of three dependent ones (list, then state, then the state's inputs).
     alignas(16) float4 listed[2][NW][kPerWarp][2];  // {v0 v1 v2 v3} {v4 guess state -}
-    int n_listed[2][NW];
+    alignas(NW % 4 == 0 ? 16 : 4) int n_listed[2][NW];
     unsigned short wrong_state[NW * kPerWarp];
     float wrong_value[NW * kPerWarp];
     // settle-now path: a warp's uncertified states, dealt out to its lanes, and their exact values
     unsigned short redo_state[NW][32 * SPT];
     float redo_value[NW][32 * SPT];
+    // The logarithm out of a table (fast_lse.cuh) where a row has so many states that one timestep in six had a wrong
+    // guess: backward scan of 40 chunks of 1024 states, T = 300, both directions, 0.398 ms instead of 0.433, 256 chunks of
+    // T = 1666 1.96 instead of 1.97 and with the posterior, beside the beam search, 2.80 instead of 2.84; for 256
+    // states the look-up costs more than it saves (512 chunks 1.175 instead of 1.146).
+    static constexpr bool kTable = NS == 1024;
+    alignas(8) ofd::LogPair log_f[kTable ? ofd::kLogPairs : 1];
     int abort_flag;
 };
 
@@ -280,11 +286,9 @@ __device__ __noinline__ int crowded_step(SpecSmem<NS, SPT, RING, COPIES, POST> &
 // final after the barrier that ends timestep r (its guesses have been checked by then) and its
 // buffer is written again during timestep r+2, so the posterior warp takes it during timestep
 // r+1; the last two rows are taken after the scan.
-// PACKED: two states in each arithmetic instruction, roles by a warp number that the compiler knows to be the
-// same for a warp.  Fewer instructions, and faster (256 states, 1024 chunks: 5.01 ms a decode instead of 5.11;
-// 1024 states, 32 chunks: 2.34 instead of 2.42) except for the 1024-state model's blocks of ten warps when two
-// of them fill an SM (256 chunks: backward scan 2.02 ms instead of 1.97).
-template <class Topo, int NS, int SPT, int RING, int COPIES, bool POST, bool PACKED>
+// Two states in each arithmetic instruction, roles by a warp number that the compiler knows to be the same for a warp:
+// fewer instructions (256 states, 1024 chunks: 5.01 ms a decode instead of 5.11).
+template <class Topo, int NS, int SPT, int RING, int COPIES, bool POST>
 __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, const __half *scores,
                                           float *out, const float *bwd_in, int T, int N, float stay,
                                           const ofx::Tables *tables, int *status, uint64_t wait_ns) {
@@ -298,12 +302,13 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
     const int tid = threadIdx.x, lane = tid & 31;
-    const int warp = PACKED ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     for (int i = tid; i < ofx::kExpTab * kExpCopies; i += blockDim.x)
         sm.exp2_rep[i] = tables->exp2_j[i / kExpCopies];
     for (int i = tid; i < ofx::kLogTab; i += blockDim.x) {
         sm.rcp_c[i] = tables->rcp_c[i];
         sm.log_c[i] = tables->log_c[i];
+        if constexpr (Smem::kTable) sm.log_f[i] = {tables->rcp_f[i], tables->log_f[i]};
     }
     for (int i = tid; i < 2 * NW; i += blockDim.x) (&sm.n_listed[0][0])[i] = 0;
     for (int i = tid; i < NS; i += blockDim.x) sm.alpha[0][i] = 0.f;
@@ -407,7 +412,7 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
                     }
                     return differs;
                 };
-                if (NW * PER <= 32) {
+                if constexpr (NW * PER <= 32) {
                     // a lane per slot: nothing to look up before the entry can be fetched
                     const int w = lane / PER, k = lane % PER;
                     const float4 a = sm.listed[par][w < NW ? w : 0][k][0], b = sm.listed[par][w < NW ? w : 0][k][1];
@@ -428,21 +433,23 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
                     // more slots than lanes: the filled ones are taken 32 at a time
                     int cnt[NW], total = 0;
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        cnt[w] = sm.n_listed[par][w];
-                        total += cnt[w];
+                    for (int w = 0; w < NW; w += 4) {
+                        const int4 c = *reinterpret_cast<const int4 *>(&sm.n_listed[par][w]);
+                        cnt[w] = c.x; cnt[w + 1] = c.y; cnt[w + 2] = c.z; cnt[w + 3] = c.w;
                     }
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) total += cnt[w];
                     for (int base = 0; base < total; base += 32) {
                         const int e = base + lane;
-                        int at_w = 0, at_k = 0, acc = 0;
+                        // the list that entry e is on: the last that starts at or before it
+                        int at_w = 0, start = 0, acc = 0;
 #pragma unroll
-                        for (int w = 0; w < NW; ++w) {
-                            if (e >= acc && e < acc + cnt[w]) {
-                                at_w = w;
-                                at_k = e - acc;
-                            }
-                            acc += cnt[w];
+                        for (int w = 1; w < NW; ++w) {
+                            acc += cnt[w - 1];
+                            at_w += e >= acc;
+                            start = e >= acc ? acc : start;
                         }
+                        const int at_k = e < total ? e - start : 0;
                         const float4 a = sm.listed[par][at_w][at_k][0], b = sm.listed[par][at_w][at_k][1];
                         const float v[5] = {a.x, a.y, a.z, a.w, b.x};
                         const float x = ofx::lse5_exact(v, tr, e < total);
@@ -519,16 +526,9 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
         float v[SPT][5];
         bool ok[SPT];
         thread_terms<Topo, SPT>(in, row, j, k0, stay, v, res);
-        uint32_t bad = 0;  // bit k: state k is uncertified
-        if constexpr (PACKED && SPT > 1) {
-            bad = ofd::lse5_guess_pairs<SPT, false>(v, res, nullptr);
+        const uint32_t bad = ofd::lse5_guess_pairs<SPT, Smem::kTable>(v, res, sm.log_f);  // bit k: state k is uncertified
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) ok[k] = !((bad >> k) & 1u);
-        } else {
-            ofd::lse5_fast_guess<SPT>(v, res, ok);
-#pragma unroll
-            for (int k = 0; k < SPT; ++k) bad |= ok[k] ? 0u : 1u << k;
-        }
+        for (int k = 0; k < SPT; ++k) ok[k] = !((bad >> k) & 1u);
         // out they go at once (certified values and guesses alike), so that the stores issue in the
         // shadow of the vote below; the two routes that settle states here and now store again
         thread_store<Topo, SPT>(nxt, gmem_out, j, k0, res, !POST);
@@ -589,34 +589,34 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
 // One grid for either or both directions: the first n_bwd_blocks blocks scan backwards, the
 // rest forwards.
 
-template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
+template <int NS, int SPT, int RING, int COPIES, int MINB>
 __global__ void __launch_bounds__(NS / SPT + 64, MINB)
 scan_spec_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd,
                  int T, int N, int n_bwd_blocks, float stay, const ofx::Tables *__restrict__ tables,
                  int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     if ((int)blockIdx.x < n_bwd_blocks)
-        spec_body<BwdTopo<NS>, NS, SPT, RING, COPIES, false, PACKED>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
+        spec_body<BwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
                                                      status, wait_ns);
     else
-        spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, false, PACKED>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
+        spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
                                                      stay, tables, status, wait_ns);
 }
 
 // Forward scan with the posterior on top: one block per chunk, reads the finished backward scores.
-template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
+template <int NS, int SPT, int RING, int COPIES, int MINB>
 __global__ void __launch_bounds__(NS / SPT + 96, MINB)
 scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__restrict__ bwd,
                            float *__restrict__ post, int T, int N, float stay,
                            const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, true, PACKED>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
+    spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, true>(smem_raw, blockIdx.x, scores, post, bwd, T, N, stay, tables, status, wait_ns);
 }
 
 // The kernels are described once, for loading (of_load_scan) and for launching.
-template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
+template <int NS, int SPT, int RING, int COPIES, int MINB>
 struct Spec {
-    static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB, PACKED>;
+    static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB>;
     static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, false>);
     static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
@@ -626,9 +626,9 @@ struct Spec {
     }
 };
 
-template <int NS, int SPT, int RING, int COPIES, int MINB, bool PACKED>
+template <int NS, int SPT, int RING, int COPIES, int MINB>
 struct SpecPosterior {
-    static constexpr auto kern = scan_spec_posterior_kernel<NS, SPT, RING, COPIES, MINB, PACKED>;
+    static constexpr auto kern = scan_spec_posterior_kernel<NS, SPT, RING, COPIES, MINB>;
     static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, true>);
     static cudaError_t launch(const __half *scores, const float *bwd, float *post, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
@@ -637,18 +637,17 @@ struct SpecPosterior {
     }
 };
 
-using Spec64 = Spec<64, 2, 8, 4, 12, true>;
-using Spec256 = Spec<256, 4, 6, 16, 4, true>;
-using Spec256Many = Spec<256, 4, 6, 4, 7, true>;
-using Spec256Most = Spec<256, 4, 6, 4, 8, true>;
-using Spec1024 = Spec<1024, 4, 6, 16, 2, false>;
-using Spec1024Both = Spec<1024, 4, 6, 16, 2, true>;
-using Spec1024Many = Spec<1024, 4, 4, 4, 3, false>;
-using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, 5, true>;
-using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, 5, true>;
-using SpecPosterior256Most = SpecPosterior<256, 4, 6, 4, 6, true>;
-using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 16, 2, false>;
-using SpecPosterior1024Many = SpecPosterior<1024, 4, 3, 4, 3, false>;
+using Spec64 = Spec<64, 2, 8, 4, 12>;
+using Spec256 = Spec<256, 4, 6, 16, 4>;
+using Spec256Many = Spec<256, 4, 6, 4, 7>;
+using Spec256Most = Spec<256, 4, 6, 4, 8>;
+using Spec1024 = Spec<1024, 4, 6, 16, 2>;
+using Spec1024Many = Spec<1024, 4, 4, 4, 3>;
+using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, 5>;
+using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, 5>;
+using SpecPosterior256Most = SpecPosterior<256, 4, 6, 4, 6>;
+using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 8, 2>;
+using SpecPosterior1024Many = SpecPosterior<1024, 4, 3, 4, 3>;
 
 }  // namespace
 
@@ -695,11 +694,10 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
             if (N <= 4 * sms) return Spec256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             if (N > 10 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Spec256Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        // (both directions: a batch that leaves the GPU room; three blocks to the SM, with a smaller ring, when
-        // two are not room enough: 444 chunks of T = 800 1.54 ms instead of 1.91)
+        // (three blocks to the SM, with a smaller ring, when two are not room enough: 444 chunks of T = 800 1.54 ms
+        // instead of 1.91)
         case 5:
             if ((bwd && fwd ? 2 : 1) * N > 2 * sms) return Spec1024Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-            if (bwd && fwd) return Spec1024Both::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Spec1024::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
     }
@@ -714,7 +712,6 @@ cudaError_t of_load_scan(int kernel) {
         case kFwd256Most: return of_load<SpecPosterior256Most>();
         case kBwd256Most: return of_load<Spec256Most>();
         case kScan1024: return of_load<Spec1024>();
-        case kScan1024Both: return of_load<Spec1024Both>();
         case kScan1024Many: return of_load<Spec1024Many>();
         case kFwd1024Many: return of_load<SpecPosterior1024Many>();
         case kFwd1024: return of_load<SpecPosterior1024>();
