@@ -477,7 +477,14 @@ cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, con
         // (a row of the 64-state model is too little work for a warp-wide reduction per chunk and timestep)
         if (state_len != 3)
             return of_launch_forward_posterior(scores, bwd, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
-        const cudaError_t e = of_launch_scans(scores, nullptr, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
+        // With two chunks to some SMs scan.cu's kernel ends after the beam search, unless T is large (its first hundred
+        // timesteps are what takes long), and the one that runs ahead before it; with one or three to the SM that is in
+        // the beam search's way.  Decodes with scan.cu's kernel / the other, ms: T = 800 100 chunks 0.655 / 0.660, 160 0.704 /
+        // 0.678, 296 0.747 / 0.722, 370 of T = 300 0.407 / 0.397; T = 300 200 0.358 / 0.334; T = 1666 200 1.294 / 1.299, 370 1.448 / 1.481
+        const bool ahead = N > sms && N <= 2 * sms && T <= 1400;
+        const cudaError_t e =
+            ahead ? of_launch_ahead(scores, nullptr, post, T, N, state_len, stay, tables, status, wait_ns, stream)
+                  : of_launch_scans(scores, nullptr, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
         if (e != cudaSuccess) return e;
     }
     return of_launch_posterior(bwd, post, T, N, state_len, stream);

@@ -179,6 +179,13 @@ def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod,
     check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 500 + T, p_step=0.6), 3, min_identical=1.0)
 
 
+@pytest.mark.parametrize("T,N", [(5, 149), (300, 150), (4, 296), (3, 297)])
+def test_forward_scan_of_two_chunks_to_the_multiprocessor(native_lib, oracle_mod, T, N):
+    # 64 states: between one and two chunks to the multiprocessor both scans run ahead of their checks
+    from openfish_b200 import synth
+    check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 800 + T, p_step=0.6), 3, min_identical=1.0)
+
+
 @pytest.mark.parametrize("infinite", [False, True])
 def test_a_warp_each_leaves_the_bits_that_small_batches_get(native_lib, infinite):
     # backward scores, posterior (whose sums are added up in one order everywhere) and what follows from them, up to
