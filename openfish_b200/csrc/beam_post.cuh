@@ -32,6 +32,6 @@ struct OfDecodeArgs {
 };
 
 // needs scores, bwd; writes bp, init_kmers
-cudaError_t of_launch_beam_search(const OfDecodeArgs &a, cudaStream_t stream);
+cudaError_t of_launch_beam_search(const OfDecodeArgs &a, int sms, cudaStream_t stream);
 // needs post, bp, init_kmers; writes every output
 cudaError_t of_launch_posterior_seq(const OfDecodeArgs &a, int sms, cudaStream_t stream);

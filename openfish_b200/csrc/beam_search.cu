@@ -434,20 +434,35 @@ struct Beam {
 template <bool SCALED> using Beam64 = Beam<64, 2, 4, SCALED>;
 template <bool SCALED> using Beam256 = Beam<256, 2, 2, SCALED>;
 template <bool SCALED> using Beam1024 = Beam<1024, 4, 1, SCALED>;
+// For a batch that has an SM to a beam search (no forward scan beside it): longer groups, since a group's end (arrival, wait,
+// the next slot's address) is on the chain and costs as much as a tenth of a timestep.  The kernel with groups of
+// 4 / 6 / 8 / 12 / 16 timesteps: 64 states, T = 1000, 0.432 / 0.426 / 0.426 / 0.422 / 0.422 ms; 256 states, T = 1666, 0.702 /
+// 0.694 / 0.688 / 0.678 / 0.684 (0.735 with two); 1024 states, 74 chunks of T = 800, with 1 / 2 / 5 / 6 / 8: 0.469 / 0.487 / 0.422
+// / 0.426 / 0.446.  Beside forward scans the larger blocks push those together on fewer SMs: 148 chunks of 256 states, T =
+// 1666, 2.70 ms a decode instead of 1.52.
+template <bool SCALED> using BeamFew64 = Beam<64, 2, 12, SCALED>;
+template <bool SCALED> using BeamFew256 = Beam<256, 2, 12, SCALED>;
+template <bool SCALED> using BeamFew1024 = Beam<1024, 2, 5, SCALED>;
 
 // (a scale of one leaves every score as it is: no multiplication then)
 template <template <bool> class B>
-cudaError_t launch_beam(const OfDecodeArgs &a, cudaStream_t stream) {
+cudaError_t launch_beam_of(const OfDecodeArgs &a, cudaStream_t stream) {
     return a.score_scale == 1.0f ? B<false>::launch(a, stream) : B<true>::launch(a, stream);
+}
+template <template <bool> class B, template <bool> class FEW>
+cudaError_t launch_beam(const OfDecodeArgs &a, int sms, cudaStream_t stream) {
+    // (the batches whose scans are both done when the beam search starts, see of_scan_plan)
+    const bool few = a.state_len == 5 ? a.N <= sms : 2 * a.N <= sms;
+    return few ? launch_beam_of<FEW>(a, stream) : launch_beam_of<B>(a, stream);
 }
 
 }  // namespace
 
-cudaError_t of_launch_beam_search(const OfDecodeArgs &a, cudaStream_t stream) {
+cudaError_t of_launch_beam_search(const OfDecodeArgs &a, int sms, cudaStream_t stream) {
     switch (a.state_len) {
-        case 3: return launch_beam<Beam64>(a, stream);
-        case 4: return launch_beam<Beam256>(a, stream);
-        case 5: return launch_beam<Beam1024>(a, stream);
+        case 3: return launch_beam<Beam64, BeamFew64>(a, sms, stream);
+        case 4: return launch_beam<Beam256, BeamFew256>(a, sms, stream);
+        case 5: return launch_beam<Beam1024, BeamFew1024>(a, sms, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -460,6 +475,12 @@ cudaError_t of_load_beam_search(int kernel) {
         case kBeam64Scaled: return of_load<Beam64<true>>();
         case kBeam256Scaled: return of_load<Beam256<true>>();
         case kBeam1024Scaled: return of_load<Beam1024<true>>();
+        case kBeamFew64: return of_load<BeamFew64<false>>();
+        case kBeamFew256: return of_load<BeamFew256<false>>();
+        case kBeamFew1024: return of_load<BeamFew1024<false>>();
+        case kBeamFew64Scaled: return of_load<BeamFew64<true>>();
+        case kBeamFew256Scaled: return of_load<BeamFew256<true>>();
+        case kBeamFew1024Scaled: return of_load<BeamFew1024<true>>();
         default: return cudaSuccess;
     }
 }

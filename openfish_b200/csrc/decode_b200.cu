@@ -331,7 +331,7 @@ extern "C" int ofb_decode_submit(int T, int N, int C, const void *scores, int st
     CU(of_launch_rest_of_posterior(plan, scores, g->pub.bwd_NTC, g->pub.post_NTC, T, N, state_len, g->sms, blank_score,
                                    g->d_tables, g->d_status, g->wait_ns, g->stream2));
     CU(cudaEventRecord(ev[5], g->stream2));
-    CU(of_launch_beam_search(a, g->stream));
+    CU(of_launch_beam_search(a, g->sms, g->stream));
     CU(cudaEventRecord(ev[2], g->stream));
     CU(cudaStreamWaitEvent(g->stream, ev[5], 0));
     CU(of_launch_posterior_seq(a, g->sms, g->stream));

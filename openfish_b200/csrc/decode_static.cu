@@ -176,7 +176,7 @@ extern "C" int openfish_b200_decode_static(int T, int N, int C, const void *scor
         a.q_shift = options->q_shift;
         a.q_scale = options->q_scale;
         a.score_scale = options->temperature;
-        e = of_launch_beam_search(a, stream);
+        e = of_launch_beam_search(a, sms, stream);
         if (e == cudaSuccess) e = of_launch_posterior_seq(a, sms, stream);
     }
     int dev_status = 0;

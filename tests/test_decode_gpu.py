@@ -186,6 +186,16 @@ def test_forward_scan_of_two_chunks_to_the_multiprocessor(native_lib, oracle_mod
     check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 800 + T, p_step=0.6), 3, min_identical=1.0)
 
 
+@pytest.mark.parametrize("sl,T", [(3, 11), (3, 12), (4, 13), (4, 24), (4, 25), (3, 37), (5, 4), (5, 5), (5, 6), (5, 11)])
+def test_groups_of_the_beam_search_that_has_an_sm_to_itself(native_lib, oracle_mod, sl, T):
+    # rows arrive 12 (1024 states: 5) timesteps at a time: a group less, exactly and more than whole ones; with a
+    # scale, the other instance of the kernel
+    from openfish_b200 import synth
+    sc = synth.make_scores(T, 3, sl, 900 + T, p_step=0.6)
+    check(native_lib, oracle_mod, sc, sl, min_identical=1.0)
+    check(native_lib, oracle_mod, sc, sl, dict(temperature=0.8), min_identical=1.0)
+
+
 @pytest.mark.parametrize("infinite", [False, True])
 def test_a_warp_each_leaves_the_bits_that_small_batches_get(native_lib, infinite):
     # backward scores, posterior (whose sums are added up in one order everywhere) and what follows from them, up to
