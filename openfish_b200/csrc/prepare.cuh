@@ -4,12 +4,12 @@
 
 // The decode's kernels, in the order in which they are loaded.
 enum OfKernel : int {
-    kFwd256, kBwd256, kBeam256, kFwd256Many, kFwd256Most, kSeq256, kBwd256Many, kBwd256Most, kAhead256,
+    kFwd256, kBeam256, kFwd256Many, kFwd256Most, kSeq256, kBwd256Many, kBwd256Most, kAhead256,
     kPosterior256, kBeam256Scaled,
     kScan1024, kFwd1024, kFwd1024Many, kBeam1024, kSeq1024, kPosterior1024, kBeam1024Scaled, kScan1024Many,
     kAhead64, kFwd64, kWarpBwd64, kWarpFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
     kSeq256Many, kSeq1024Many, kSeq64Many,
-    kBeamFew256, kBeamFew64, kBeamFew1024, kBeamFew256Scaled, kBeamFew64Scaled, kBeamFew1024Scaled,
+    kBeamFew256, kBeamFew64, kBeamFew1024, kBeamFew256Scaled, kBeamFew64Scaled, kBeamFew1024Scaled, kAhead256Mid, kAhead64Mid,
     kKernels
 };
 

@@ -638,7 +638,6 @@ struct SpecPosterior {
 };
 
 using Spec64 = Spec<64, 2, 8, 4, 12>;
-using Spec256 = Spec<256, 4, 6, 16, 4>;
 using Spec256Many = Spec<256, 4, 6, 4, 7>;
 using Spec256Most = Spec<256, 4, 6, 4, 8>;
 using Spec1024 = Spec<1024, 4, 6, 16, 2>;
@@ -684,14 +683,12 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
     switch (state_len) {
         // (up to three chunks to the SM; scan_warp.cu has the kernel for more.)  Two states a thread
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        // Four blocks to the SM (128 registers) as long as that is room enough, else seven (72): what a
-        // block loses is less than what a half empty second round of blocks costs: 740 chunks of T = 1666
-        // 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28; 512: 1.16 with four, 1.24 with seven.  Eight (64)
-        // for many rounds; the line is the forward scan's, so that a batch has the thrifty blocks of both
+        // (more than four chunks to the SM; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
+        // registers) rather than four: what a block loses is less than what a half empty second round of blocks
+        // costs: 740 chunks of T = 1666 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28.  Eight (64) for many rounds; the line is the forward scan's, so that a batch has the thrifty blocks of both
         // kernels or of neither.  T = 800, seven / eight: 1300 chunks 1.330 / 1.342 ms, 1480 1.470 / 1.498, 1600
         // 1.499 / 1.568, 2072 1.865 / 1.839, 3000 2.689 / 2.616.
         case 4:
-            if (N <= 4 * sms) return Spec256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             if (N > 10 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Spec256Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // (three blocks to the SM, with a smaller ring, when two are not room enough: 444 chunks of T = 800 1.54 ms
@@ -705,7 +702,6 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
 
 cudaError_t of_load_scan(int kernel) {
     switch (kernel) {
-        case kBwd256: return of_load<Spec256>();
         case kFwd256: return of_load<SpecPosterior256>();
         case kBwd256Many: return of_load<Spec256Many>();
         case kFwd256Many: return of_load<SpecPosterior256Many>();

@@ -31,7 +31,7 @@ cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bw
 
 // One or both scans by the kernel for batches that leave the GPU room, for the 64- and the 256-state
 // model.  (scan_ahead.cu)
-cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, float stay,
+cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, int sms, float stay,
                             const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream);
 
 // Backward scan, and forward scan with the posterior, of the 64-state model by one warp a chunk.  (scan_warp.cu)

@@ -10,8 +10,8 @@
 // scores have grown) needs the value-exact routine, a chain of some 450 cycles on its own.  The scan
 // warps never wait for it: such a state gets the likelier of its two candidate floats, a bit in its
 // thread's mask says so, and the scan goes on.  Timesteps come in groups of E; while the scan warps work
-// on a group, E checker warps recompute the marked states of the group before, a timestep each, put those
-// whose guess was wrong right in their row, and their verdict is looked at in the group after.  Was a guess
+// on a group, a checker warp recomputes the marked states of the group before, 32 at a time, puts those
+// whose guess was wrong right in their row, and its verdict is looked at in the group after.  Was a guess
 // wrong (one timestep in sixty), the scan goes back and carries on behind the first such timestep; the rows
 // behind it, which followed from the wrong value, and whatever has been put right in them are written
 // again.  What reaches HBM is what the exact routine alone would have produced.  While
@@ -45,8 +45,8 @@ struct AheadSmem {
     static constexpr bool kLogTable = NS > 64;  // the logarithm out of a table (fast_lse.cuh)
     alignas(8) ofd::LogPair log_f[kLogTable ? ofd::kLogPairs : 1];
     uint32_t mask[2][W][32];          // by group parity and scan thread: bit SPT*q + k, timestep q, state k
-    int verdict[2][E];                // by group parity and timestep: a guess was wrong
-    unsigned short marked[E][64];     // a timestep's marked states, when a lane has more than one
+    uint32_t verdict[2];              // by group parity: bit q, a guess of timestep q was wrong
+    unsigned short marked[64];        // marked states of a group, dealt out to the checker's lanes
     int back;                         // barriers minus groups: two more for every time the scan has gone back
     double exp2_j[ofx::kExpTab];
     double rcp_c[ofx::kLogTab];
@@ -63,7 +63,7 @@ __device__ __forceinline__ void named_sync() {
     else asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
 }
 
-// One direction of one chunk by one block: W scan warps, E checker warps, a copy warp and an output warp.
+// One direction of one chunk by one block: W scan warps, a checker warp, a copy warp and an output warp.
 // `out` gets the T+1 rows of the chunk.
 template <class Topo, int NS, int W, int E, int S>
 __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, const __half *scores, float *out,
@@ -71,9 +71,9 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
                                            uint64_t wait_ns) {
     constexpr int SPT = NS / (32 * W);  // states per scan thread
     static_assert(SPT == 2 || SPT == 4, "a thread's states share one j");
-    static_assert(E * SPT <= 32 && E >= 2 && S >= 4, "a mask word per group; three groups are under way");
-    constexpr int NT = 32 * (W + E + 2);
-    constexpr int kSync = 32 * (W + E);  // threads at a group's end
+    static_assert(W * E * SPT <= 32 && E >= 2 && S >= 4, "a mask word per group; three groups are under way");
+    constexpr int NT = 32 * (W + 3);
+    constexpr int kSync = 32 * (W + 1);  // threads at a group's end
     using Smem = AheadSmem<NS, W, E, S>;
     constexpr int H = Smem::H;
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
@@ -88,7 +88,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     }
     for (int i = tid; i < NS; i += NT) sm.rows[0][i] = 0.f;
     for (int i = tid; i < 2 * W * 32; i += NT) (&sm.mask[0][0][0])[i] = 0;
-    if (tid < 2 * E) (&sm.verdict[0][0])[tid] = 0;
+    if (tid < 2) sm.verdict[tid] = 0;
     if (tid == 0) {
         sm.abort_flag = 0;
         sm.back = 0;
@@ -104,7 +104,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     float *out_chunk = out + (size_t)chunk * (size_t)(T + 1) * NS;
     const int groups = (T + E - 1) / E;
 
-    if (warp == W + E) {
+    if (warp == W + 1) {
         // ------------------------------------------------------------------ copy warp
         if (lane == 0) {
             const size_t t_stride = (size_t)N * NS * 4;
@@ -122,7 +122,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         return;
     }
 
-    if (warp == W + E + 1) {
+    if (warp == W + 2) {
         // ------------------------------------------------------------------ output warp
         // rows of a group leave once the group is verified; row T at the end
         constexpr int PERL = NS / 32, V = PERL >= 4 ? 4 : PERL;  // floats per lane, per access
@@ -156,11 +156,9 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         return;
     }
 
-    if (warp >= W) {
-        // ------------------------------------------------------------------ checker warps
-        // checker q takes timestep q of every group
+    if (warp == W) {
+        // ------------------------------------------------------------------ checker warp
         const ofx::TabRef tr = {sm.exp2_j, 1, sm.rcp_c, sm.log_c};
-        const int q = warp - W;
         const uint32_t lt_mask = (1u << lane) - 1u;
         for (int at = 0;; ++at) {
             named_sync<2, kSync>();
@@ -169,56 +167,48 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             const int g = at - *(volatile int *)&sm.back;
             if (g > groups) return;
             const int par = at & 1;
-            uint32_t m = 0;  // marks of this lane's W scan threads, SPT bits each
+            uint32_t m = 0;  // marks of this lane's W scan threads, E*SPT bits each
 #pragma unroll
-            for (int w = 0; w < W; ++w) m |= ((sm.mask[par][w][lane] >> (q * SPT)) & ((1u << SPT) - 1u)) << (w * SPT);
+            for (int w = 0; w < W; ++w) m |= sm.mask[par][w][lane] << (w * E * SPT);
             if (g < 0 || g >= groups) m = 0;
             const int g0 = g < 0 ? 0 : g;
-            const int h0 = (g0 * E + q) % H;
-            const float *in = sm.rows[h0];
-            float *out_row = sm.rows[h0 + 1 == H ? 0 : h0 + 1];
-            const unsigned char *row = sm.ring[g0 % S][q];
-            bool wrong = false;
-            // bit `bit` of lane l's marks
-            auto check = [&](bool mine, int l, int bit) {
-                const int t = (bit / SPT) * 32 + l;  // the scan thread
-                const int s = Topo::state(t % Topo::NJ, (t / Topo::NJ) * SPT + bit % SPT);
-                float v[5];
-                terms_of<Topo>(s, in, row, stay, v);
-                const float guess = out_row[s];
-                const float x = ofx::lse5_exact(v, tr);
-                // (Nobody else writes this row before the next group's end.  Where an earlier timestep turns out
-                // wrong too, or the scan is going back right now, the row is taken again.)
-                if (mine && __float_as_uint(x) != __float_as_uint(guess)) {
-                    wrong = true;
-                    out_row[s] = x;
-                }
-            };
-            uint32_t owners = __ballot_sync(0xffffffffu, m != 0);
-            if (owners) {
-                if (__any_sync(0xffffffffu, (m & (m - 1u)) != 0)) {
-                    do {
-                        int n = 0;
-                        do {
-                            if (m) sm.marked[q][n + __popc(owners & lt_mask)] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
-                            n += __popc(owners);
-                            m &= m - 1u;
-                            owners = __ballot_sync(0xffffffffu, m != 0);
-                        } while (owners && n + __popc(owners) <= 64);
-                        __syncwarp();
-                        for (int first = 0; first < n; first += 32) {
-                            const bool mine = first + lane < n;
-                            const int e = sm.marked[q][mine ? first + lane : 0];
-                            check(mine, e & 31, e >> 5);
-                        }
-                        __syncwarp();
-                    } while (owners);
-                } else {
-                    check(m != 0, lane, m ? __ffs(m) - 1 : 0);
+            const int h0 = (g0 * E) % H;
+            const unsigned char *ring0 = sm.ring[g0 % S][0];
+            uint32_t wrong = 0;
+            // The marked states, 32 at a time.  A value put right here may be one that a later entry reads, or that was
+            // itself worked out from a wrong one: both lie behind the first wrong timestep, from which on all is
+            // taken again.  (Nobody else writes these rows before the next group's end.)
+            for (uint32_t owners = __ballot_sync(0xffffffffu, m != 0); owners;) {
+                int n = 0;
+                do {
+                    if (m) sm.marked[n + __popc(owners & lt_mask)] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
+                    n += __popc(owners);
+                    m &= m - 1u;
+                    owners = __ballot_sync(0xffffffffu, m != 0);
+                } while (owners && n + __popc(owners) <= 64);
+                __syncwarp();
+                for (int first = 0; first < n; first += 32) {
+                    const bool mine = first + lane < n;
+                    const int e = sm.marked[mine ? first + lane : 0];
+                    const int bit = e >> 5, q = (bit / SPT) % E;
+                    const int t = bit / (E * SPT) * 32 + (e & 31);  // the scan thread
+                    const int s = Topo::state(t % Topo::NJ, (t / Topo::NJ) * SPT + bit % SPT);
+                    const int h = h0 + q < H ? h0 + q : h0 + q - H;
+                    float *const guess = &sm.rows[h + 1 == H ? 0 : h + 1][s];
+                    float v[5];
+                    terms_of<Topo>(s, sm.rows[h], ring0 + q * Smem::kRowBytes, stay, v);
+                    const float was = *guess;
+                    const float x = ofx::lse5_exact(v, tr);
+                    __syncwarp();  // (every lane has its terms)
+                    if (mine && __float_as_uint(x) != __float_as_uint(was)) {
+                        wrong |= 1u << q;
+                        *guess = x;
+                    }
+                    __syncwarp();
                 }
             }
-            wrong = __any_sync(0xffffffffu, wrong);
-            if (lane == 0) sm.verdict[par][q] = wrong;
+            wrong = __reduce_or_sync(0xffffffffu, wrong);
+            if (lane == 0) sm.verdict[par] = wrong;
         }
     }
 
@@ -236,14 +226,12 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     bool all = true;  // what exact_for_all said a group ago
     ofd::mbar_wait_bounded(&sm.full[0], 0u, &sm.abort_flag, status, wait_ns);
     Piece piece(ring, j);
-    // (one group past the end for the last verdict, one more for the checkers to leave)
+    // (one group past the end for the last verdict, one more for the checker to leave)
     for (int par = 0; g <= groups + 1; par ^= 1) {
         // The verdict on the group before the last was handed over at the barrier just passed (it stays
         // until the check of this group).  Nothing waits for it here: it is looked at when the first
         // timestep of this group has been computed.
-        uint32_t wrong = 0;
-#pragma unroll
-        for (int q = 0; q < E; ++q) wrong |= *(volatile int *)&sm.verdict[par][q] ? 1u << q : 0u;
+        const uint32_t wrong = *(volatile uint32_t *)&sm.verdict[par];
         const int next = stage + 1 == S ? 0 : stage + 1;
         const uint32_t next_parity = next ? parity : parity ^ 1u;
         const unsigned char *ring_next = next ? ring + E * Smem::kRowBytes : sm.ring[0][0];
@@ -322,7 +310,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
 
 // The first n_bwd blocks scan backwards, the others forwards.
 template <int NS, int W, int E, int S, int MINB>
-__global__ void __launch_bounds__(32 * (W + E + 2), MINB)
+__global__ void __launch_bounds__(32 * (W + 3), MINB)
 scan_ahead_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd, int T, int N,
                   int n_bwd, float stay, const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -339,18 +327,26 @@ struct Ahead {
     static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
         const int n_bwd = bwd ? N : 0, n_fwd = fwd ? N : 0;
-        kern<<<n_bwd + n_fwd, 32 * (W + E + 2), bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
+        kern<<<n_bwd + n_fwd, 32 * (W + 3), bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
         return cudaGetLastError();
     }
 };
-// Groups of four: what a group costs besides its timesteps (250 cycles) is paid half as often as with two, and going
-// back, rare and short, loses less than that.  Both scans with groups of two / three / four / six: one chunk of
-// 64 states, T = 1000, 0.306 / 0.292 / 0.285 / 0.279 ms, 40 chunks of T = 120 0.074 / 0.069 / 0.066 / 0.068; 14 chunks of 256
-// states, T = 1666, 0.640 / 0.593 / 0.572 / -, and the backward scan of 300 chunks 0.948 / 0.885 / 0.872 / -.  (Before values
-// were put right in place: one chunk of 64 states 0.342, 14 of 256 0.640 with two.)  Five stages, so that three
-// blocks of 256 states fit an SM; four come too late (14 chunks 0.844).
-using Ahead64 = Ahead<64, 1, 4, 6, 5>;
+// Longer groups: what a group costs besides its timesteps (250 cycles, and the checker's pass) is paid less often, and
+// going back, rare and short, loses less than that.  One checker for a group instead of one for each of its
+// timesteps, whose lists were nearly empty: both scans of one chunk of 64 states, T = 1000, 0.256 ms instead of 0.280
+// (groups of four), 0.246 with groups of six; of 14 chunks of 256 states, T = 1666, 0.560 instead of 0.572; the backward
+// scan of 300 chunks 0.766 instead of 0.874.  (Groups of two with a checker for each timestep, and wrong guesses
+// gone back to and taken again instead of put right: 0.345, 0.642, 0.979.)  Five stages of 256 states, so that three
+// blocks fit an SM; four come too late (14 chunks 0.844).
+// For more than three chunks of 256 states to the SM two scan warps of four states a thread, and blocks that fit four
+// times: backward scan of 512 chunks 0.970 ms, 1.009 with four warps, 1.146 with scan.cu's kernel; of 601 chunks of T = 1201,
+// which do not all fit, 1.132 with these and 1.030 with scan.cu's.  For more than five chunks of 64 states blocks that
+// fit eight times (T = 800: 760 chunks 0.310 instead of 0.395 by a warp a chunk; 1300, which do not all fit, 0.511
+// and 0.462).
+using Ahead64 = Ahead<64, 1, 6, 6, 5>;
+using Ahead64Mid = Ahead<64, 1, 4, 6, 8>;
 using Ahead256 = Ahead<256, 4, 4, 5, 3>;
+using Ahead256Mid = Ahead<256, 2, 3, 5, 4>;
 
 // ------------------------------------------------------------------------------------------
 // post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,
@@ -411,13 +407,17 @@ struct Posterior {
 
 }  // namespace
 
-cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, float stay,
+cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, int sms, float stay,
                             const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
     const __half *s = static_cast<const __half *>(scores_fp16);
     if (T < 1) return cudaErrorInvalidValue;
     switch (state_len) {
-        case 3: return Ahead64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        case 4: return Ahead256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        case 3:
+            if (N > 5 * sms) return Ahead64Mid::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+            return Ahead64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+        case 4:
+            if (N > 3 * sms) return Ahead256Mid::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+            return Ahead256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -440,7 +440,7 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 
 // Where the lines lie (decodes of T = 800, ms, by plan: together / ahead then forward / backward then forward):
 //   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;
-//                at T = 1666 440: - / 2.59 / 2.65;  512: - / 2.92 / 2.82
+//                at T = 1666 512: - / 2.56 / 2.73;  at T = 1201 601: - / 2.85 / 2.74
 //   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;
 //                ahead then forward / a warp to a chunk: 200 0.79 / 0.87;  444 0.896 / 0.906;  592 0.98 / 0.92;
 //                1500 2.18 / 1.61;  at T = 1666 1024 2.58 / 2.22;  4096 9.21 / 6.92
@@ -451,21 +451,20 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 OfScanPlan of_scan_plan(int N, int state_len, int sms) {
     if (state_len == 5) return 2 * N <= 3 * sms ? OfScanPlan::kTogether : OfScanPlan::kBackwardThenForward;
     if (2 * N <= sms) return OfScanPlan::kTogether;
-    if (N <= 3 * sms) return OfScanPlan::kAheadThenForward;
+    if (N <= (state_len == 3 ? 3 : 4) * sms) return OfScanPlan::kAheadThenForward;
     return state_len == 3 ? OfScanPlan::kWarps : OfScanPlan::kBackwardThenForward;
 }
 
 cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bwd, float *post, int T, int N,
                                   int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                   uint64_t wait_ns, cudaStream_t stream) {
-    // (the backward scan of 592 chunks of T = 800 0.300 ms by the kernel that runs ahead and 0.354 by a warp each, of 740
-    // 0.376 and 0.395, of 1024 of T = 1666 0.79 and 0.74)
-    if (plan == OfScanPlan::kWarps && N > 5 * sms)
+    // (the backward scan of 1024 chunks of T = 1666 0.597 ms by the kernel that runs ahead and 0.742 by a warp each)
+    if (plan == OfScanPlan::kWarps && N > 8 * sms)
         return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
     if (plan == OfScanPlan::kBackwardThenForward || state_len == 5)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
-    return of_launch_ahead(scores, bwd, fwd, T, N, state_len, stay, tables, status, wait_ns, stream);
+    return of_launch_ahead(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
 }
 
 cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, const float *bwd, float *post, int T,
@@ -474,16 +473,21 @@ cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, con
     if (plan == OfScanPlan::kWarps)
         return of_launch_warp_forward_posterior(scores, bwd, post, T, N, stay, tables, status, wait_ns, stream);
     if (plan != OfScanPlan::kTogether) {
+        // The forward scan beside the beam search: scan.cu's kernel is in its way least, the one that runs ahead
+        // (followed by the posterior's kernel) has the shorter chain, above all of the first hundred timesteps.  So
+        // the latter where the former would end after the beam search.  Decodes of 256 states with the former / the
+        // latter, ms: 100 chunks T = 300 0.424 / 0.366, 600 0.664 / 0.618, 1000 0.961 / 0.956, 1666 1.467 / 1.524; 148 chunks 600 0.666 /
+        // 0.648, 1000 0.970 / 1.006; 200 chunks T = 300 0.513 / 0.447, 1000 1.207 / 1.136, 1666 1.821 / 1.794; 250 chunks 1000 1.211 /
+        // 1.177, 1666 1.841 / 1.852; 296 chunks 1000 1.229 / 1.212, 1666 1.882 / 1.934; 330 chunks T = 300 0.602 / 0.629.  64 states: 200
+        // chunks T = 300 0.358 / 0.334, 1666 1.256 / 1.273; 310 chunks T = 800 0.765 / 0.733; 440 0.805 / 0.768, 1666 1.424 / 1.409.
+        bool ahead = false;
+        if (state_len == 3) ahead = N > 2 * sms || T <= 1400;
+        if (state_len == 4 && N <= 2 * sms) ahead = N <= sms ? T <= 700 : 2 * N <= 3 * sms || T <= 1100;
         // (a row of the 64-state model is too little work for a warp-wide reduction per chunk and timestep)
-        if (state_len != 3)
+        if (!ahead && state_len != 3)
             return of_launch_forward_posterior(scores, bwd, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
-        // With two chunks to some SMs scan.cu's kernel ends after the beam search, unless T is large (its first hundred
-        // timesteps are what takes long), and the one that runs ahead before it; with one or three to the SM that is in
-        // the beam search's way.  Decodes with scan.cu's kernel / the other, ms: T = 800 100 chunks 0.655 / 0.660, 160 0.704 /
-        // 0.678, 296 0.747 / 0.722, 370 of T = 300 0.407 / 0.397; T = 300 200 0.358 / 0.334; T = 1666 200 1.294 / 1.299, 370 1.448 / 1.481
-        const bool ahead = N > sms && N <= 2 * sms && T <= 1400;
         const cudaError_t e =
-            ahead ? of_launch_ahead(scores, nullptr, post, T, N, state_len, stay, tables, status, wait_ns, stream)
+            ahead ? of_launch_ahead(scores, nullptr, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream)
                   : of_launch_scans(scores, nullptr, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
         if (e != cudaSuccess) return e;
     }
@@ -493,6 +497,8 @@ cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, con
 cudaError_t of_load_ahead(int kernel) {
     switch (kernel) {
         case kAhead256: return of_load<Ahead256>();
+        case kAhead64Mid: return of_load<Ahead64Mid>();
+        case kAhead256Mid: return of_load<Ahead256Mid>();
         case kAhead64: return of_load<Ahead64>();
         case kPosterior64: return of_load<Posterior<64>>();
         case kPosterior256: return of_load<Posterior<256>>();

@@ -52,7 +52,7 @@ __device__ __forceinline__ void thread_store(float *dst, int j, int k0, const fl
 template <int NS> constexpr float kGuessFrom = NS == 64 ? 256.f : 512.f;
 
 // Every state by the exact routine, judged by one of a row's scores: too small, or no finite number (then none of
-// the row's states is certified and all would go through the checkers; a batch of 300 chunks of T = 1000 with one infinite
+// the row's states is certified and all would go through the checker; a batch of 300 chunks of T = 1000 with one infinite
 // score took 3.70 ms instead of 2.43).
 template <int NS>
 __device__ __forceinline__ bool exact_for_all(float score) {

@@ -179,11 +179,14 @@ def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod,
     check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 500 + T, p_step=0.6), 3, min_identical=1.0)
 
 
-@pytest.mark.parametrize("T,N", [(5, 149), (300, 150), (4, 296), (3, 297)])
-def test_forward_scan_of_two_chunks_to_the_multiprocessor(native_lib, oracle_mod, T, N):
-    # 64 states: between one and two chunks to the multiprocessor both scans run ahead of their checks
+@pytest.mark.parametrize("sl,T,N", [(3, 5, 149), (3, 300, 150), (3, 4, 296), (3, 3, 297), (3, 1401, 76), (3, 6, 741), (3, 200, 760),
+                                    (3, 13, 1184), (3, 9, 1185), (3, 120, 1186), (4, 5, 76), (4, 300, 148), (4, 701, 75), (4, 13, 222),
+                                    (4, 1101, 223), (4, 9, 296), (4, 4, 446), (4, 300, 448), (4, 7, 592)])
+def test_scans_that_run_ahead_by_chunks_to_the_multiprocessor(native_lib, oracle_mod, sl, T, N):
+    # which scans of a batch run ahead of their checks, and with what blocks, hangs on the chunks to the
+    # multiprocessor and on T; T whole and ragged in groups of three, four and six timesteps
     from openfish_b200 import synth
-    check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 800 + T, p_step=0.6), 3, min_identical=1.0)
+    check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 800 + T, p_step=0.6), sl, min_identical=1.0)
 
 
 @pytest.mark.parametrize("sl,T", [(3, 11), (3, 12), (4, 13), (4, 24), (4, 25), (3, 37), (5, 4), (5, 5), (5, 6), (5, 11)])
