@@ -9,7 +9,7 @@ enum OfKernel : int {
     kScan1024, kFwd1024, kFwd1024Many, kBeam1024, kSeq1024, kPosterior1024, kBeam1024Scaled, kScan1024Many,
     kAhead64, kFwd64, kWarpBwd64, kWarpFwd64, kBeam64, kPosterior64, kSeq64, kBeam64Scaled,
     kSeq256Many, kSeq1024Many, kSeq64Many,
-    kBeamFew256, kBeamFew64, kBeamFew1024, kBeamFew256Scaled, kBeamFew64Scaled, kBeamFew1024Scaled, kAhead256Mid, kAhead64Mid,
+    kBeamFew256, kBeamFew64, kBeamFew1024, kBeamFew256Scaled, kBeamFew64Scaled, kBeamFew1024Scaled, kAhead256Mid, kAhead256Five, kAhead64Mid,
     kKernels
 };
 

@@ -683,7 +683,7 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
     switch (state_len) {
         // (up to three chunks to the SM; scan_warp.cu has the kernel for more.)  Two states a thread
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        // (more than four chunks to the SM; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
+        // (more than five chunks to the SM; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
         // registers) rather than four: what a block loses is less than what a half empty second round of blocks
         // costs: 740 chunks of T = 1666 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28.  Eight (64) for many rounds; the line is the forward scan's, so that a batch has the thrifty blocks of both
         // kernels or of neither.  T = 800, seven / eight: 1300 chunks 1.330 / 1.342 ms, 1480 1.470 / 1.498, 1600

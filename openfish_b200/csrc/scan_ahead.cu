@@ -340,13 +340,15 @@ struct Ahead {
 // blocks fit an SM; four come too late (14 chunks 0.844).
 // For more than three chunks of 256 states to the SM two scan warps of four states a thread, and blocks that fit four
 // times: backward scan of 512 chunks 0.970 ms, 1.009 with four warps, 1.146 with scan.cu's kernel; of 601 chunks of T = 1201,
-// which do not all fit, 1.132 with these and 1.030 with scan.cu's.  For more than five chunks of 64 states blocks that
+// which do not all fit, 1.132 with these, 1.030 with scan.cu's, and 0.989 with shorter groups, which fit five times.
+// (Seven to the SM, with four stages of two timesteps: 1024 chunks 3.12 instead of scan.cu's 1.79.)  For more than five chunks of 64 states blocks that
 // fit eight times (T = 800: 760 chunks 0.310 instead of 0.395 by a warp a chunk; 1300, which do not all fit, 0.511
 // and 0.462).
 using Ahead64 = Ahead<64, 1, 6, 6, 5>;
 using Ahead64Mid = Ahead<64, 1, 4, 6, 8>;
 using Ahead256 = Ahead<256, 4, 4, 5, 3>;
 using Ahead256Mid = Ahead<256, 2, 3, 5, 4>;
+using Ahead256Five = Ahead<256, 2, 2, 5, 5>;
 
 // ------------------------------------------------------------------------------------------
 // post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,
@@ -416,6 +418,7 @@ cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int
             if (N > 5 * sms) return Ahead64Mid::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Ahead64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         case 4:
+            if (N > 4 * sms) return Ahead256Five::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             if (N > 3 * sms) return Ahead256Mid::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Ahead256::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         default: return cudaErrorInvalidValue;
@@ -440,7 +443,7 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 
 // Where the lines lie (decodes of T = 800, ms, by plan: together / ahead then forward / backward then forward):
 //   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;
-//                at T = 1666 512: - / 2.56 / 2.73;  at T = 1201 601: - / 2.85 / 2.74
+//                at T = 1666 512: - / 2.56 / 2.73;  1024: - / 5.10 / 4.77;  at T = 1201 601: - / 2.69 / 2.73
 //   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;
 //                ahead then forward / a warp to a chunk: 200 0.79 / 0.87;  444 0.896 / 0.906;  592 0.98 / 0.92;
 //                1500 2.18 / 1.61;  at T = 1666 1024 2.58 / 2.22;  4096 9.21 / 6.92
@@ -451,7 +454,7 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 OfScanPlan of_scan_plan(int N, int state_len, int sms) {
     if (state_len == 5) return 2 * N <= 3 * sms ? OfScanPlan::kTogether : OfScanPlan::kBackwardThenForward;
     if (2 * N <= sms) return OfScanPlan::kTogether;
-    if (N <= (state_len == 3 ? 3 : 4) * sms) return OfScanPlan::kAheadThenForward;
+    if (N <= (state_len == 3 ? 3 : 5) * sms) return OfScanPlan::kAheadThenForward;
     return state_len == 3 ? OfScanPlan::kWarps : OfScanPlan::kBackwardThenForward;
 }
 
@@ -462,7 +465,10 @@ cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bw
     if (plan == OfScanPlan::kWarps && N > 8 * sms)
         return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
-    if (plan == OfScanPlan::kBackwardThenForward || state_len == 5)
+    // (five chunks of 256 states to the SM: the shorter groups pay once the first timesteps are a small part; 620 chunks of
+    // T = 300 0.358 ms against scan.cu's 0.352, 594 of T = 800 0.699 against 0.735)
+    const bool early = state_len == 4 && N > 4 * sms && T < 500;
+    if (plan == OfScanPlan::kBackwardThenForward || state_len == 5 || early)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
     return of_launch_ahead(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
 }
@@ -499,6 +505,7 @@ cudaError_t of_load_ahead(int kernel) {
         case kAhead256: return of_load<Ahead256>();
         case kAhead64Mid: return of_load<Ahead64Mid>();
         case kAhead256Mid: return of_load<Ahead256Mid>();
+        case kAhead256Five: return of_load<Ahead256Five>();
         case kAhead64: return of_load<Ahead64>();
         case kPosterior64: return of_load<Posterior<64>>();
         case kPosterior256: return of_load<Posterior<256>>();
