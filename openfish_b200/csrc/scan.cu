@@ -685,11 +685,11 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // (more than five chunks to the SM; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
         // registers) rather than four: what a block loses is less than what a half empty second round of blocks
-        // costs: 740 chunks of T = 1666 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28.  Eight (64) for many rounds; the line is the forward scan's, so that a batch has the thrifty blocks of both
-        // kernels or of neither.  T = 800, seven / eight: 1300 chunks 1.330 / 1.342 ms, 1480 1.470 / 1.498, 1600
-        // 1.499 / 1.568, 2072 1.865 / 1.839, 3000 2.689 / 2.616.
+        // costs: 740 chunks of T = 1666 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28.  Eight (64)
+        // for many rounds.  Seven / eight, T = 800: 1490 chunks 1.453 / 1.495 ms, 1600 1.469 / 1.550, 1900 1.701 / 1.685, 2050 1.817 /
+        // 1.807, 2200 1.996 / 1.913; T = 300: 1700 0.727 / 0.753.
         case 4:
-            if (N > 10 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
+            if (N > 12 * sms) return Spec256Most::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
             return Spec256Many::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
         // (three blocks to the SM, with a smaller ring, when two are not room enough: 444 chunks of T = 800 1.54 ms
         // instead of 1.91)
