@@ -144,8 +144,8 @@ int openfish_b200_selfcheck_arith(double err[2]);
  * the reference, whose kernels do not wait. */
 int openfish_b200_selfcheck_wait(const openfish_gpubuf_t *gpubuf, unsigned limit_us);
 
-/* Number of kernels one decode call launches (for benchmark bookkeeping; the 64-state model's larger
- * batches launch one more). */
+/* Number of kernels one decode call launches (for benchmark bookkeeping; batches whose forward scan
+ * leaves the posterior to a kernel of its own beside the beam search launch one more). */
 int openfish_b200_kernels_per_decode(void);
 
 /* Decode without allocating anything, for callers that cannot let a library allocate once they
