@@ -27,6 +27,7 @@
 
 #include "exact_math.cuh"
 #include "fast_lse.cuh"
+#include "group_order.h"
 #include "of_device.cuh"
 #include "prepare.cuh"
 #include "scan.cuh"
@@ -47,7 +48,7 @@ struct AheadSmem {
     uint32_t mask[2][W][32];          // by group parity and scan thread: bit SPT*q + k, timestep q, state k
     uint32_t verdict[2];              // by group parity: bit q, a guess of timestep q was wrong
     unsigned short marked[64];        // marked states of a group, dealt out to the checker's lanes
-    int back;                         // barriers minus groups: two more for every time the scan has gone back
+    int ended[2];                     // by barrier parity: the group that ended there (group_order.h)
     double exp2_j[ofx::kExpTab];
     double rcp_c[ofx::kLogTab];
     double log_c[ofx::kLogTab];
@@ -91,7 +92,6 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     if (tid < 2) sm.verdict[tid] = 0;
     if (tid == 0) {
         sm.abort_flag = 0;
-        sm.back = 0;
         for (int r = 0; r < S; ++r) {
             ofd::mbar_init(&sm.full[r], 1);
             ofd::mbar_init(&sm.done[r], 1);
@@ -162,18 +162,15 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         const uint32_t lt_mask = (1u << lane) - 1u;
         for (int at = 0;; ++at) {
             named_sync<2, kSync>();
-            // the group that has just ended (when the scan is going back right now, `back` may show it
-            // already or not: this check is void either way)
-            const int g = at - *(volatile int *)&sm.back;
+            const int g = group_told(sm.ended, at);  // has just ended
             if (g > groups) return;
             const int par = at & 1;
             uint32_t m = 0;  // marks of this lane's W scan threads, E*SPT bits each
 #pragma unroll
             for (int w = 0; w < W; ++w) m |= sm.mask[par][w][lane] << (w * E * SPT);
-            if (g < 0 || g >= groups) m = 0;
-            const int g0 = g < 0 ? 0 : g;
-            const int h0 = (g0 * E) % H;
-            const unsigned char *ring0 = sm.ring[g0 % S][0];
+            if (g >= groups) m = 0;
+            const int h0 = (g * E) % H;
+            const unsigned char *ring0 = sm.ring[g % S][0];
             uint32_t wrong = 0;
             // The marked states, 32 at a time.  A value put right here may be one that a later entry reads, or that was
             // itself worked out from a wrong one: both lie behind the first wrong timestep, from which on all is
@@ -219,31 +216,30 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
     for (int k = 0; k < SPT; ++k) res[k] = 0.f;
     float *rows = sm.rows[0], *rows_next = sm.rows[E % H];  // row g*E, row (g+1)*E
     const unsigned char *ring = sm.ring[0][0];
-    int g = 0, stage = 0;
+    GroupOrder at;
+    int stage = 0;
     uint32_t parity = 0;
-    int ignore = 2;  // verdicts to come that are about nothing
-    int from = 0;    // the group's first timestep to be taken: behind a corrected one when the scan has gone back
     bool all = true;  // what exact_for_all said a group ago
     ofd::mbar_wait_bounded(&sm.full[0], 0u, &sm.abort_flag, status, wait_ns);
     Piece piece(ring, j);
     // (one group past the end for the last verdict, one more for the checker to leave)
-    for (int par = 0; g <= groups + 1; par ^= 1) {
+    while (at.g <= groups + 1) {
         // The verdict on the group before the last was handed over at the barrier just passed (it stays
         // until the check of this group).  Nothing waits for it here: it is looked at when the first
         // timestep of this group has been computed.
-        const uint32_t wrong = *(volatile uint32_t *)&sm.verdict[par];
+        const uint32_t wrong = *(volatile uint32_t *)&sm.verdict[at.par];
         const int next = stage + 1 == S ? 0 : stage + 1;
         const uint32_t next_parity = next ? parity : parity ^ 1u;
         const unsigned char *ring_next = next ? ring + E * Smem::kRowBytes : sm.ring[0][0];
         const float probe = rows[0];
-        const int n = T - g * E;  // timesteps left
-        const bool ready = g + 1 >= groups || ofd::mbar_try_wait(&sm.full[next], next_parity);
-        const bool back = ignore == 0 && wrong != 0;
+        const int n = T - at.g * E;  // timesteps left
+        const bool ready = at.g + 1 >= groups || ofd::mbar_try_wait(&sm.full[next], next_parity);
+        const bool back = at.goes_back(wrong);
         uint32_t bad = 0;
-        if (g < groups) {
+        if (at.g < groups) {
 #pragma unroll
             for (int q = 0; q < E; ++q) {
-                if (q < from) continue;
+                if (q < at.from) continue;
                 const float *in = rows + q * NS;
                 float *nxt = q + 1 < E ? rows + (q + 1) * NS : rows_next;
                 if (__builtin_expect(all, 0)) {
@@ -273,33 +269,28 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         if (__builtin_expect(back, 0)) {
             // back to the group before the last, behind its first wrong timestep, which the checker has put right
             // (what follows it followed from it)
-            g -= 2;
-            from = __ffs(wrong);
-            ignore = 2;
-            par ^= 1;  // (no barrier has been passed)
-            if (tid == 0) *(volatile int *)&sm.back = sm.back + 2;
-            rows = sm.rows[(g * E) % H];
-            rows_next = sm.rows[(g * E + E) % H];
-            stage = g % S;
-            parity = (uint32_t)(g / S) & 1u;
+            at.go_back(wrong);
+            rows = sm.rows[(at.g * E) % H];
+            rows_next = sm.rows[(at.g * E + E) % H];
+            stage = at.g % S;
+            parity = (uint32_t)(at.g / S) & 1u;
             ring = sm.ring[stage][0];
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) res[k] = (from < E ? rows + from * NS : rows_next)[Topo::state(j, k0 + k)];
-            piece.load(ring + (from < E ? from : 0) * Smem::kRowBytes, j);
+            for (int k = 0; k < SPT; ++k) res[k] = (at.from < E ? rows + at.from * NS : rows_next)[Topo::state(j, k0 + k)];
+            piece.load(ring + (at.from < E ? at.from : 0) * Smem::kRowBytes, j);
             all = exact_for_all<NS>(rows[0]);
             continue;
         }
         // the group before the last is verified
-        ofd::mbar_arrive_if(tid == 0 && ignore == 0 && g <= groups + 1, &sm.done[stage >= 2 ? stage - 2 : stage - 2 + S]);
-        ignore -= ignore > 0;
+        ofd::mbar_arrive_if(tid == 0 && at.verified(), &sm.done[stage >= 2 ? stage - 2 : stage - 2 + S]);
         if (n < E) bad &= n > 0 ? (1u << (n * SPT)) - 1u : 0u;
-        sm.mask[par][warp][lane] = bad;
+        sm.mask[at.par][warp][lane] = bad;
+        if (tid == 0) at.tell(sm.ended);
         if (!ready) ofd::mbar_wait_slow(&sm.full[next], next_parity, &sm.abort_flag, status, wait_ns);
         piece.load(ring_next, j);
         all = exact_for_all<NS>(probe);
         named_sync<2, kSync>();
-        ++g;
-        from = 0;
+        at.next();
         stage = next;
         parity = next_parity;
         ring = ring_next;
