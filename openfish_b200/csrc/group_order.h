@@ -31,11 +31,12 @@ struct GroupOrder {
     }
     // the verdict just looked at was about group g-2 and found it right: its input rows are final
     OF_HD bool verified() const { return ignore == 0; }
-    // By one thread, at the end of a group, before the barrier.  The checker writes into the rows of the group that it
-    // is told, so it must be one that is still to be verified, whenever it gets round to reading which: a check that the
-    // scan goes back beside is of the group in between, all of whose rows are taken again.  Hence a note for each
-    // parity, which stays as it is until the barrier after the next; a single count that the scan changed on
-    // going back could send a late checker to a group whose rows were final and whose scores were gone.
+    // By one thread, when the scan takes up a group (or goes back to it), for the barrier that ends it.  The checker writes
+    // into the rows of the group that it is told, so it must be one that is still to be verified, whenever it gets round to
+    // reading which: a check that the scan goes back beside is of the group in between, all of whose rows are taken
+    // again.  Hence a note for each parity, which stays as it is from its barrier to the next; a single count that the
+    // scan changed on going back could send a late checker to a group whose rows were final and whose scores were
+    // gone.
     OF_HD void tell(volatile int *ended) const { ended[par] = g; }
     OF_HD void next() {
         ++g;

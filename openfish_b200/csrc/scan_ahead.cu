@@ -228,6 +228,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         // until the check of this group).  Nothing waits for it here: it is looked at when the first
         // timestep of this group has been computed.
         const uint32_t wrong = *(volatile uint32_t *)&sm.verdict[at.par];
+        if (tid == 0) at.tell(sm.ended);
         const int next = stage + 1 == S ? 0 : stage + 1;
         const uint32_t next_parity = next ? parity : parity ^ 1u;
         const unsigned char *ring_next = next ? ring + E * Smem::kRowBytes : sm.ring[0][0];
@@ -285,7 +286,6 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         ofd::mbar_arrive_if(tid == 0 && at.verified(), &sm.done[stage >= 2 ? stage - 2 : stage - 2 + S]);
         if (n < E) bad &= n > 0 ? (1u << (n * SPT)) - 1u : 0u;
         sm.mask[at.par][warp][lane] = bad;
-        if (tid == 0) at.tell(sm.ended);
         if (!ready) ofd::mbar_wait_slow(&sm.full[next], next_parity, &sm.abort_flag, status, wait_ns);
         piece.load(ring_next, j);
         all = exact_for_all<NS>(probe);

@@ -67,6 +67,7 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
 
     while (at.g <= groups + 1) {
         const uint32_t seen = verdict[at.par];
+        at.tell(ended);
         const bool back = at.goes_back(seen);
         uint32_t guesses = 0;
         meanwhile();
@@ -94,7 +95,6 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
         }
         if (at.verified() && verified < groups) ++verified;
         mask[at.par] = guesses;
-        at.tell(ended);
         meanwhile();
         while (at.g + 1 < groups && holds[(at.g + 1) % S] != at.g + 1) {
             if (left == verified) return -3;  // nothing could ever bring those scores
