@@ -9,6 +9,8 @@
 #define OF_HD inline
 #endif
 
+constexpr uint32_t kAllAnew = 1u << 31;  // a verdict: too many guesses to check, the scan takes the whole group exactly
+
 // The scan warps' side; a barrier that scan warps and checker pass together ends every group.  While the scan takes
 // a group, the checker looks at the one that ended at the last barrier and puts its wrong guesses right; the
 // verdict (bit q: a guess of timestep q was wrong) is looked at in the group after.
@@ -19,13 +21,14 @@ struct GroupOrder {
     int par = 0;     // parity of the barriers passed
 
     OF_HD bool goes_back(uint32_t verdict) const { return ignore == 0 && verdict != 0; }
-    // to the group before the last, behind its first wrong timestep; no barrier is passed for it
+    // to the group before the last, behind its first wrong timestep or, with kAllAnew, to its start; no barrier is
+    // passed for it
     OF_HD void go_back(uint32_t verdict) {
         g -= 2;
 #ifdef __CUDA_ARCH__
-        from = __ffs((int)verdict);
+        from = verdict & kAllAnew ? 0 : __ffs((int)verdict);
 #else
-        from = __builtin_ffs((int)verdict);
+        from = verdict & kAllAnew ? 0 : __builtin_ffs((int)verdict);
 #endif
         ignore = 2;
     }

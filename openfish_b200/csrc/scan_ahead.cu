@@ -58,6 +58,11 @@ struct AheadSmem {
     int abort_flag;
 };
 
+// Rounds of up to 64 marked states that a group's check goes through; with more the group is taken again exactly by
+// the scan warps, which is 32 times as many hands.  Ordinary groups stay below two (a state in fourteen when guesses
+// begin); it is for rows that turn infinite, whose first state, by which exact_for_all judges, is still finite.
+constexpr int kRounds = 5;
+
 template <int ID, int THREADS>
 __device__ __forceinline__ void named_sync() {
     if constexpr (THREADS == 32) __syncwarp();
@@ -172,10 +177,15 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
             const int h0 = (g * E) % H;
             const unsigned char *ring0 = sm.ring[g % S][0];
             uint32_t wrong = 0;
+            int rounds = 0;
             // The marked states, 32 at a time.  A value put right here may be one that a later entry reads, or that was
             // itself worked out from a wrong one: both lie behind the first wrong timestep, from which on all is
             // taken again.  (Nobody else writes these rows before the next group's end.)
             for (uint32_t owners = __ballot_sync(0xffffffffu, m != 0); owners;) {
+                if (NS > 64 && rounds++ == kRounds) {
+                    wrong = kAllAnew;
+                    break;
+                }
                 int n = 0;
                 do {
                     if (m) sm.marked[n + __popc(owners & lt_mask)] = (unsigned short)(lane | (__ffs(m) - 1) << 5);
@@ -269,7 +279,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         }
         if (__builtin_expect(back, 0)) {
             // back to the group before the last, behind its first wrong timestep, which the checker has put right
-            // (what follows it followed from it)
+            // (what follows it followed from it), or to its start, to take it exactly
             at.go_back(wrong);
             rows = sm.rows[(at.g * E) % H];
             rows_next = sm.rows[(at.g * E + E) % H];
@@ -279,7 +289,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
 #pragma unroll
             for (int k = 0; k < SPT; ++k) res[k] = (at.from < E ? rows + at.from * NS : rows_next)[Topo::state(j, k0 + k)];
             piece.load(ring + (at.from < E ? at.from : 0) * Smem::kRowBytes, j);
-            all = exact_for_all<NS>(rows[0]);
+            all = (wrong & kAllAnew) || exact_for_all<NS>(rows[0]);
             continue;
         }
         // the group before the last is verified

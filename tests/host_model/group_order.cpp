@@ -13,10 +13,10 @@ static uint32_t next_row(uint32_t row, uint32_t score) {
 }
 
 // Scans T timesteps in groups of E through a ring of S groups.  marked, wrong: percentages of timesteps whose value
-// is a guess, and of guesses that are wrong.  Returns how many of the T+1 rows left with a wrong value; *backs the times the
+// is a guess, and of guesses that are wrong; many: guesses that are too many for a check.  Returns how many of the T+1 rows left with a wrong value; *backs the times the
 // scan has gone back, *late the checks that ran after the scan had gone back beside them; negative: -1 a row that
 // has not left is written over, -2 a group checked that is not there.
-extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned seed, int *backs, int *late) {
+extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, int many, unsigned seed, int *backs, int *late) {
     std::mt19937 rng(seed);
     auto percent = [&](int p) { return (int)(rng() % 100) < p; };
     const int groups = (T + E - 1) / E, H = E * (S + 1);
@@ -35,7 +35,7 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
     int ended[2] = {0, 0};
     uint32_t mask[2] = {0, 0}, verdict[2] = {0, 0};
     int barrier = -1;          // the last one passed
-    bool check_due = false, went_back = false;
+    bool check_due = false, went_back = false, exactly = false;
     int verified = 0, left = 0;  // groups
 
     auto check = [&]() {
@@ -44,8 +44,13 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
         uint32_t m = g < groups ? mask[barrier & 1] : 0, v = 0;
         if (g < 0 || g > groups + 1) bad = -2;
         if (went_back && m) ++*late;
+        int checked = 0;
         for (int q = 0; q < E; ++q) {
             if (!(m >> q & 1)) continue;
+            if (++checked == many) {
+                v = kAllAnew;
+                break;
+            }
             const int h = (g * E + q) % H;
             const uint32_t x = next_row(rows[h], ring[g % S * E + q]);
             if (x != rows[(h + 1) % H]) {
@@ -76,7 +81,7 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
                 if (q < at.from) continue;
                 const int t = at.g * E + q;
                 uint32_t x = next_row(rows[t % H], ring[at.g % S * E + q]);
-                if (percent(marked)) {
+                if (!exactly && percent(marked)) {
                     if (t < T) guesses |= 1u << q;
                     if (percent(wrong)) x ^= 1u;
                 }
@@ -88,6 +93,7 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
         }
         if (back) {
             at.go_back(seen);
+            exactly = seen & kAllAnew;
             went_back = true;
             ++*backs;
             meanwhile();
@@ -104,6 +110,7 @@ extern "C" int wrong_rows(int T, int E, int S, int marked, int wrong, unsigned s
         ++barrier;
         check_due = true;
         went_back = false;
+        exactly = false;
         at.next();
     }
     while (left < verified) group_leaves();

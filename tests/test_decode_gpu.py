@@ -171,6 +171,30 @@ def test_an_infinite_score_is_taken_alike_by_every_scan_kernel_and_at_a_bearable
     assert few < 2.2 * scans(sc)[0]
 
 
+def test_rows_that_turn_infinite_are_taken_again_at_once(native_lib):
+    # a group in which the rows turn infinite has more guesses than its check can be about; the scans of 14 chunks take
+    # 1.47 times as long as with ordinary scores (half of the timesteps by the exact routine), 1.85 times while every one of
+    # those guesses was checked, and the group gone back to, a timestep at a time
+    import torch
+    from openfish_b200 import synth
+    of = native_lib
+    T, N = 1000, 14
+    sc = torch.from_numpy(synth.make_scores(T, N, 4, 95)).cuda()
+    gb = of.gpubuf_init(T, N, 4)
+
+    def scans():
+        ms = []
+        for _ in range(7):
+            of.decode_gpu(sc, 4, gpubuf=gb)
+            ms.append(gb.last_decode_ms()["bwd_scan"])
+        return min(ms)
+
+    ordinary = scans()
+    sc[T // 2, :, 7] = float("inf")
+    assert scans() < 1.6 * ordinary
+    gb.free()
+
+
 @pytest.mark.parametrize("T,N", [(1, 445), (7, 445), (8, 446), (9, 447), (16, 445), (23, 1000), (400, 445)])
 def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod, T, N):
     # 64 states, more than three chunks to the multiprocessor: groups of eight timesteps, whole and ragged, T long

@@ -18,14 +18,16 @@ def host(tmp_path_factory):
 
 @pytest.mark.parametrize("E,S", [(6, 6), (4, 6), (4, 5), (3, 5), (2, 5), (2, 4)])
 def test_every_row_that_leaves_is_right(host, E, S):
-    # the kernels' groups and stages; nearly all timesteps guessed and half of them wrong, ordinary ones, none
+    # the kernels' groups and stages; nearly all timesteps guessed and half of them wrong, ordinary ones, none; with
+    # guesses too many for a check at times
     backs, late = C.c_int(), C.c_int()
     seen = [0, 0]
-    for marked, wrong in ((95, 50), (70, 10), (30, 60), (5, 100), (100, 0)):
+    for marked, wrong, many in ((95, 50, 99), (70, 10, 99), (30, 60, 99), (5, 100, 99), (100, 0, 99), (95, 50, 2), (60, 30, 3),
+                                (100, 0, 1)):
         for T in list(range(1, 3 * E + 2)) + [E * S, 257, 800]:
             for seed in range(12):
-                n = host.wrong_rows(T, E, S, marked, wrong, 1 + seed, C.byref(backs), C.byref(late))
-                assert n == 0, (marked, wrong, T, seed, n, backs.value)
+                n = host.wrong_rows(T, E, S, marked, wrong, many, 1 + seed, C.byref(backs), C.byref(late))
+                assert n == 0, (marked, wrong, many, T, seed, n, backs.value)
                 seen[0] += backs.value
                 seen[1] += late.value
     assert seen[0] > 1000 and seen[1] > 100  # (that the scan goes back, and a check is late beside it, does occur)
