@@ -446,8 +446,9 @@ cudaError_t of_launch_posterior(const float *bwd, float *post, int T, int N, int
 //   256 states:  74 chunks 0.79 / 0.87 / 0.98;  111: 0.98 / 0.88 / 0.98;  296: 1.42 / 1.20 / 1.28;
 //                at T = 1666 512: - / 2.56 / 2.73;  1024: - / 5.10 / 4.77;  at T = 1201 601: - / 2.69 / 2.73
 //   64 states:   74 chunks 0.69 / 0.69 / 0.72;  296: 0.95 / 0.79 / 0.83;
-//                ahead then forward / a warp to a chunk: 200 0.79 / 0.87;  444 0.896 / 0.906;  592 0.98 / 0.92;
-//                1500 2.18 / 1.61;  at T = 1666 1024 2.58 / 2.22;  4096 9.21 / 6.92
+//                ahead then forward / a warp to a chunk (their forward scan): 445 0.755 / 0.761, 500 0.781 / 0.774, 592 0.795 /
+//                0.786, 700 1.086 / 0.919;  at T = 300 445 0.361 / 0.374, 592 0.379 / 0.380;  at T = 1666 445 1.406 / 1.404, 592
+//                1.482 / 1.447, 1024 2.45 / 2.03
 //   1024 states: 74 chunks 1.42 /  -   / 1.81;  222: 2.69 /  -   / 2.79;  240: 2.98 /  -   / 2.80
 // Two directions on one SM are in each other's way beyond their number (their code is more than an
 // instruction cache holds), which is why "together" ends where every block has an SM to itself, except for
@@ -482,14 +483,18 @@ cudaError_t of_launch_rest_of_posterior(OfScanPlan plan, const void *scores, con
     if (plan != OfScanPlan::kTogether) {
         // The forward scan beside the beam search: scan.cu's kernel is in its way least, the one that runs ahead
         // (followed by the posterior's kernel) has the shorter chain, above all of the first hundred timesteps.  So
-        // the latter where the former would end after the beam search.  Decodes of 256 states with the former / the
-        // latter, ms: 100 chunks T = 300 0.424 / 0.366, 600 0.664 / 0.618, 1000 0.961 / 0.956, 1666 1.467 / 1.524; 148 chunks 600 0.666 /
-        // 0.648, 1000 0.970 / 1.006; 200 chunks T = 300 0.513 / 0.447, 1000 1.207 / 1.136, 1666 1.821 / 1.794; 250 chunks 1000 1.211 /
-        // 1.177, 1666 1.841 / 1.852; 296 chunks 1000 1.229 / 1.212, 1666 1.882 / 1.934; 330 chunks T = 300 0.602 / 0.629.  64 states: 200
-        // chunks T = 300 0.358 / 0.334, 1666 1.256 / 1.273; 310 chunks T = 800 0.765 / 0.733; 440 0.805 / 0.768, 1666 1.424 / 1.409.
+        // the latter where the former would end after the beam search: in short and in small batches, up to two chunks to the
+        // SM (three of 64 states).  Decodes with the former / the latter, ms, by chunks and T:
+        //   256 states, a chunk to the SM:  75: 700 0.707 / 0.663, 1400 1.240 / 1.235;  100: 700 0.712 / 0.704, 1000 0.931 / 0.950;
+        //   148: 500 0.572 / 0.552, 700 0.716 / 0.731.  Two:  149: 1666 1.729 / 1.678, 2000 2.084 / 2.064, 3000 3.17 / 3.27;  222: 1000
+        //   1.176 / 1.152, 1400 1.541 / 1.541, 2000 2.162 / 2.248;  296: 700 0.921 / 0.898, 1000 1.202 / 1.207, 1666 1.810 / 1.891.
+        //   Three:  297: 300 0.545 / 0.570, 1666 2.174 / 2.257.
+        //   64 states:  75 to 148 within 1 % for every T (300 to 2000);  200: 300 0.330 / 0.321, 700 0.609 / 0.600, 1000 0.809 /
+        //   0.820;  296: 300 0.339 / 0.337, 700 0.628 / 0.636, 1400 1.110 / 1.148.  Three:  310 of T = 800 0.765 / 0.733; 440 0.805 / 0.768.
+        const long long steps = (long long)T * N;
         bool ahead = false;
-        if (state_len == 3) ahead = N > 2 * sms || T <= 1400;
-        if (state_len == 4 && N <= 2 * sms) ahead = N <= sms ? T <= 700 : 2 * N <= 3 * sms || T <= 1100;
+        if (state_len == 3) ahead = N <= sms || N > 2 * sms || steps <= 1000ll * sms;
+        if (state_len == 4) ahead = steps <= (N <= sms ? 600ll : 2000ll) * sms && N <= 2 * sms;
         // (a row of the 64-state model is too little work for a warp-wide reduction per chunk and timestep)
         if (!ahead && state_len != 3)
             return of_launch_forward_posterior(scores, bwd, post, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
