@@ -8,12 +8,12 @@
 //   fwd[n][0][s] = 0,  fwd[n][t+1][s] = LSE5( fwd[n][t][s] + stay,   fwd[n][t][j + b*ns/4] + score[t][n][4s + b] )
 //                                       for s = 4j + k                         (b = 0..3 in both)
 // The two recursions do not depend on each other (only the posterior needs both).  This file's kernels
-// are for batches that fill the GPU (scan_ahead.cu has one for small batches): the decode runs the
+// are for batches that fill the GPU (scan_ahead.cu has one for smaller ones): the decode runs the
 // backward scan first (the beam search waits for it) and the forward scan beside the beam search,
 // which leaves most issue slots free.  For the 256- and 1024-state models the forward scan also
 // forms the posterior (a warp of its own per block, see PosteriorRow) and its scores never leave the
-// chip; for the 64-state model they go to HBM for the kernel that forms the posterior (and batches of more
-// than three chunks to the SM have scan_warp.cu).
+// chip.  Of the 64-state model only the forward scan of a few batches is left to this file (scan_ahead.cu says which);
+// its rows go to HBM for the kernel that forms the posterior.
 //
 // Shape of a block.  In either direction the four states that share j also share their four
 // neighbour inputs, and their 16 transition scores are one contiguous 32-byte piece of the score
@@ -586,21 +586,25 @@ __device__ __forceinline__ void spec_body(unsigned char *smem_raw, int chunk, co
 }
 
 // ------------------------------------------------------------------------------------------
-// One grid for either or both directions: the first n_bwd_blocks blocks scan backwards, the
+// One grid for the directions DIRS (kBackward, kForward or both): the first n_bwd_blocks blocks scan backwards, the
 // rest forwards.
+enum : int { kBackward = 1, kForward = 2 };
 
-template <int NS, int SPT, int RING, int COPIES, int MINB>
+template <int NS, int SPT, int RING, int COPIES, int MINB, int DIRS>
 __global__ void __launch_bounds__(NS / SPT + 64, MINB)
 scan_spec_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd,
                  int T, int N, int n_bwd_blocks, float stay, const ofx::Tables *__restrict__ tables,
                  int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    if ((int)blockIdx.x < n_bwd_blocks)
-        spec_body<BwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
-                                                     status, wait_ns);
-    else
-        spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
-                                                     stay, tables, status, wait_ns);
+    const bool backward = DIRS == kBackward || (DIRS != kForward && (int)blockIdx.x < n_bwd_blocks);
+    if constexpr (DIRS & kBackward)
+        if (backward)
+            spec_body<BwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x, scores, bwd, nullptr, T, N, stay, tables,
+                                                                 status, wait_ns);
+    if constexpr (DIRS & kForward)
+        if (!backward)
+            spec_body<FwdTopo<NS>, NS, SPT, RING, COPIES, false>(smem_raw, blockIdx.x - n_bwd_blocks, scores, fwd, nullptr, T, N,
+                                                                 stay, tables, status, wait_ns);
 }
 
 // Forward scan with the posterior on top: one block per chunk, reads the finished backward scores.
@@ -614,13 +618,14 @@ scan_spec_posterior_kernel(const __half *__restrict__ scores, const float *__res
 }
 
 // The kernels are described once, for loading (of_load_scan) and for launching.
-template <int NS, int SPT, int RING, int COPIES, int MINB>
+template <int NS, int SPT, int RING, int COPIES, int MINB, int DIRS>
 struct Spec {
-    static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB>;
+    static constexpr auto kern = scan_spec_kernel<NS, SPT, RING, COPIES, MINB, DIRS>;
     static constexpr size_t bytes = sizeof(SpecSmem<NS, SPT, RING, COPIES, false>);
     static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
         const int n_bwd = bwd ? N : 0, n_fwd = fwd ? N : 0;
+        if ((bwd && !(DIRS & kBackward)) || (fwd && !(DIRS & kForward))) return cudaErrorInvalidValue;
         kern<<<n_bwd + n_fwd, NS / SPT + 64, bytes, stream>>>(scores, bwd, fwd, T, N, n_bwd, stay, tables, status, wait_ns);
         return cudaGetLastError();
     }
@@ -637,11 +642,13 @@ struct SpecPosterior {
     }
 };
 
-using Spec64 = Spec<64, 2, 8, 4, 12>;
-using Spec256Many = Spec<256, 4, 6, 4, 7>;
-using Spec256Most = Spec<256, 4, 6, 4, 8>;
-using Spec1024 = Spec<1024, 4, 6, 16, 2>;
-using Spec1024Many = Spec<1024, 4, 4, 4, 3>;
+using Spec64 = Spec<64, 2, 8, 4, 12, kForward>;
+// (Nothing launches the forward half of this one.  Without it the backward half takes 1.5 % longer, 1024 chunks of T =
+// 1666 1.826 ms instead of 1.796, with the same registers: where the code comes to lie.)
+using Spec256Many = Spec<256, 4, 6, 4, 7, kBackward | kForward>;
+using Spec256Most = Spec<256, 4, 6, 4, 8, kBackward>;
+using Spec1024 = Spec<1024, 4, 6, 16, 2, kBackward | kForward>;
+using Spec1024Many = Spec<1024, 4, 4, 4, 3, kBackward | kForward>;
 using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, 5>;
 using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, 5>;
 using SpecPosterior256Most = SpecPosterior<256, 4, 6, 4, 6>;
@@ -681,9 +688,10 @@ cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int
                             uint64_t wait_ns, cudaStream_t stream) {
     const __half *s = static_cast<const __half *>(scores_fp16);
     switch (state_len) {
-        // (up to three chunks to the SM; scan_warp.cu has the kernel for more.)  Two states a thread
+        // (the forward scan of one to two chunks to the SM with many timesteps; all else of this model is scan_ahead.cu's and
+        // scan_warp.cu's)
         case 3: return Spec64::launch(s, bwd, fwd, T, N, stay, tables, status, wait_ns, stream);
-        // (more than five chunks to the SM; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
+        // (more than five chunks to the SM, four if T is small; scan_ahead.cu has the kernel for fewer)  Seven blocks to the SM (72
         // registers) rather than four: what a block loses is less than what a half empty second round of blocks
         // costs: 740 chunks of T = 1666 1.43 ms instead of 1.86; 1024: 1.90 instead of 2.28.  Eight (64)
         // for many rounds.  Seven / eight, T = 800: 1490 chunks 1.453 / 1.495 ms, 1600 1.469 / 1.550, 1900 1.701 / 1.685, 2050 1.817 /
