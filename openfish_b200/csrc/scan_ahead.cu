@@ -467,9 +467,10 @@ cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bw
     if (plan == OfScanPlan::kWarps && N > 8 * sms)
         return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
-    // (five chunks of 256 states to the SM: the shorter groups pay once the first timesteps are a small part; 620 chunks of
-    // T = 300 0.358 ms against scan.cu's 0.352, 594 of T = 800 0.699 against 0.735)
-    const bool early = state_len == 4 && N > 4 * sms && T < 500;
+    // (five chunks of 256 states to the SM: the shorter groups pay once the first timesteps are a small part.  Decodes with
+    // this kernel / scan.cu's: T = 100, 593 chunks 0.426 / 0.409 ms; 200, 680 chunks 0.719 / 0.710; 300 0.941 / 0.947; 400
+    // 1.154 / 1.173)
+    const bool early = state_len == 4 && N > 4 * sms && T < 250;
     if (plan == OfScanPlan::kBackwardThenForward || state_len == 5 || early)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
     return of_launch_ahead(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
