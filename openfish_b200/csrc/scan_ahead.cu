@@ -16,7 +16,7 @@
 // behind it, which followed from the wrong value, and whatever has been put right in them are written
 // again.  What reaches HBM is what the exact routine alone would have produced.  While
 // the scores are small and the float grid fine, guesses are too many and too often wrong: every state
-// goes through the exact routine until the scores have passed kGuessFrom.
+// goes through the exact routine until the scores have passed FROM.
 //
 // What bounds it: the instructions of one timestep in one scan warp, issued two to three cycles apart.
 // So a thread has two states (four warps for 256 states; with four states a thread a timestep takes a
@@ -71,7 +71,7 @@ __device__ __forceinline__ void named_sync() {
 
 // One direction of one chunk by one block: W scan warps, a checker warp, a copy warp and an output warp.
 // `out` gets the T+1 rows of the chunk.
-template <class Topo, int NS, int W, int E, int S>
+template <class Topo, int NS, int W, int E, int S, int FROM>
 __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, const __half *scores, float *out,
                                            int T, int N, float stay, const ofx::Tables *tables, int *status,
                                            uint64_t wait_ns) {
@@ -289,7 +289,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
 #pragma unroll
             for (int k = 0; k < SPT; ++k) res[k] = (at.from < E ? rows + at.from * NS : rows_next)[Topo::state(j, k0 + k)];
             piece.load(ring + (at.from < E ? at.from : 0) * Smem::kRowBytes, j);
-            all = (wrong & kAllAnew) || exact_for_all<NS>(rows[0]);
+            all = (wrong & kAllAnew) || exact_for_all<FROM>(rows[0]);
             continue;
         }
         // the group before the last is verified
@@ -298,7 +298,7 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
         sm.mask[at.par][warp][lane] = bad;
         if (!ready) ofd::mbar_wait_slow(&sm.full[next], next_parity, &sm.abort_flag, status, wait_ns);
         piece.load(ring_next, j);
-        all = exact_for_all<NS>(probe);
+        all = exact_for_all<FROM>(probe);
         named_sync<2, kSync>();
         at.next();
         stage = next;
@@ -310,20 +310,20 @@ __device__ __forceinline__ void scan_chunk(unsigned char *smem_raw, int chunk, c
 }
 
 // The first n_bwd blocks scan backwards, the others forwards.
-template <int NS, int W, int E, int S, int MINB>
+template <int NS, int W, int E, int S, int MINB, int FROM>
 __global__ void __launch_bounds__(32 * (W + 3), MINB)
 scan_ahead_kernel(const __half *__restrict__ scores, float *__restrict__ bwd, float *__restrict__ fwd, int T, int N,
                   int n_bwd, float stay, const ofx::Tables *__restrict__ tables, int *status, uint64_t wait_ns) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     if ((int)blockIdx.x < n_bwd)
-        scan_chunk<BwdTopo<NS>, NS, W, E, S>(smem_raw, blockIdx.x, scores, bwd, T, N, stay, tables, status, wait_ns);
+        scan_chunk<BwdTopo<NS>, NS, W, E, S, FROM>(smem_raw, blockIdx.x, scores, bwd, T, N, stay, tables, status, wait_ns);
     else
-        scan_chunk<FwdTopo<NS>, NS, W, E, S>(smem_raw, blockIdx.x - n_bwd, scores, fwd, T, N, stay, tables, status, wait_ns);
+        scan_chunk<FwdTopo<NS>, NS, W, E, S, FROM>(smem_raw, blockIdx.x - n_bwd, scores, fwd, T, N, stay, tables, status, wait_ns);
 }
 
-template <int NS, int W, int E, int S, int MINB>
+template <int NS, int W, int E, int S, int MINB, int FROM>
 struct Ahead {
-    static constexpr auto kern = scan_ahead_kernel<NS, W, E, S, MINB>;
+    static constexpr auto kern = scan_ahead_kernel<NS, W, E, S, MINB, FROM>;
     static constexpr size_t bytes = sizeof(AheadSmem<NS, W, E, S>);
     static cudaError_t launch(const __half *scores, float *bwd, float *fwd, int T, int N, float stay,
                               const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream) {
@@ -345,11 +345,17 @@ struct Ahead {
 // (Seven to the SM, with four stages of two timesteps: 1024 chunks 3.12 instead of scan.cu's 1.79.)  For more than five chunks of 64 states blocks that
 // fit eight times (T = 800: 760 chunks 0.310 instead of 0.395 by a warp a chunk; 1300, which do not all fit, 0.511
 // and 0.462).
-using Ahead64 = Ahead<64, 1, 6, 6, 5>;
-using Ahead64Mid = Ahead<64, 1, 4, 6, 8>;
-using Ahead256 = Ahead<256, 4, 4, 5, 3>;
-using Ahead256Mid = Ahead<256, 2, 3, 5, 4>;
-using Ahead256Five = Ahead<256, 2, 2, 5, 5>;
+// FROM, the score from which on guesses are made: at 512 one state in fourteen is marked, at 256 one in seven, and the fewer
+// states there are, the fewer to go wrong.  Both scans of 40 chunks of T = 120, from 512 / 256 / 128: 64 states 0.069 / 0.065 /
+// 0.067 ms, 256 states 0.076 / 0.085 / 0.094.  With two scan warps the exact routine is dearer, and so the more chunks there
+// are to an SM: backward scan of T = 300, 512 chunks 0.256 / 0.259 / 0.279, 600 0.339 / 0.316 / 0.319; where scores grow slowly (by two a
+// timestep, as stays do) 0.326 / 0.283 / 0.300 and 0.472 / 0.385 / 0.371, where all states are equal 0.317 / 0.229 / 0.184 and 0.468 /
+// 0.326 / 0.255.
+using Ahead64 = Ahead<64, 1, 6, 6, 5, 256>;
+using Ahead64Mid = Ahead<64, 1, 4, 6, 8, 256>;
+using Ahead256 = Ahead<256, 4, 4, 5, 3, 512>;
+using Ahead256Mid = Ahead<256, 2, 3, 5, 4, 256>;
+using Ahead256Five = Ahead<256, 2, 2, 5, 5, 128>;
 
 // ------------------------------------------------------------------------------------------
 // post (in: forward rows) = softmax over states of forward + backward, row by row: rows are independent,

@@ -46,17 +46,12 @@ __device__ __forceinline__ void thread_store(float *dst, int j, int k0, const fl
     }
 }
 
-// Scores from which on guesses are made: one state in fourteen (256 states) or in seven (64, of which there are
-// fewer to go wrong) is then marked.  Both scans of 40 chunks of T = 120, from 512 / 256 / 128: 64 states 0.069 / 0.065 /
-// 0.067 ms, 256 states 0.076 / 0.085 / 0.094.
-template <int NS> constexpr float kGuessFrom = NS == 64 ? 256.f : 512.f;
-
-// Every state by the exact routine, judged by one of a row's scores: too small, or no finite number (then none of
+// Every state by the exact routine, judged by one of a row's scores: below FROM, or no finite number (then none of
 // the row's states is certified and all would go through the checker; a batch of 300 chunks of T = 1000 with one infinite
 // score took 3.70 ms instead of 2.43).
-template <int NS>
+template <int FROM>
 __device__ __forceinline__ bool exact_for_all(float score) {
-    const uint32_t from = __float_as_uint(kGuessFrom<NS>), infinity = 0x7f800000u;
+    const uint32_t from = __float_as_uint((float)FROM), infinity = 0x7f800000u;
     return (__float_as_uint(score) & 0x7fffffffu) - from >= infinity - from;
 }
 

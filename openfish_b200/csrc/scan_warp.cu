@@ -34,6 +34,7 @@ constexpr int K = 8;            // timesteps to a group
 constexpr int STAGES = 2;       // groups of score rows kept
 constexpr int H = K + 1;        // rows kept: a group's input row and the K behind it
 constexpr int SPT = 2;          // states to a lane
+constexpr int kGuessFrom = 256; // score from which on guesses are made
 constexpr int kRowBytes = NS * 4 * 2;
 static_assert(SPT * K <= 32, "a mask word holds a group's marks");
 
@@ -149,7 +150,7 @@ scan_warp_kernel(const __half *__restrict__ scores, float *__restrict__ out, con
             const float *in = sm.rows[wrap(at + q)];
             const unsigned char *row = sm.ring[stage][q];
             float *gmem_out = out_chunk + (ptrdiff_t)Topo::out_row(g * K + q, T) * NS;
-            const bool all = exact_for_all<NS>(in[0]);
+            const bool all = exact_for_all<kGuessFrom>(in[0]);
             uint32_t mask = 0;  // bit SPT*q + k: state k of timestep q is a guess
             Piece piece(row, j);
 #pragma unroll 1

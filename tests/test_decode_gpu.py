@@ -195,6 +195,28 @@ def test_rows_that_turn_infinite_are_taken_again_at_once(native_lib):
     gb.free()
 
 
+def test_scores_that_grow_slowly_cost_little_more(native_lib):
+    # paths that mostly stay gain two a timestep, and most of 300 timesteps have scores too small for guesses in blocks
+    # that begin with them late: backward scan of 600 chunks 1.40 times that of ordinary scores when they began at 512, 1.18
+    # from 128 on
+    import torch
+    from openfish_b200 import synth
+    of = native_lib
+    T, N = 300, 600
+    sc = torch.from_numpy(synth.make_scores(T, 24, 4, 96)).cuda().repeat(1, N // 24, 1).contiguous()
+    gb = of.gpubuf_init(T, N, 4)
+
+    def scan(scores):
+        ms = []
+        for _ in range(9):
+            of.decode_gpu(scores, 4, gpubuf=gb)
+            ms.append(gb.last_decode_ms()["bwd_scan"])
+        return min(ms)
+
+    assert scan((sc * 0.3 - 3.0).contiguous()) < 1.29 * scan(sc)
+    gb.free()
+
+
 @pytest.mark.parametrize("T,N", [(1, 445), (7, 445), (8, 446), (9, 447), (16, 445), (23, 1000), (400, 445)])
 def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod, T, N):
     # 64 states, more than three chunks to the multiprocessor: groups of eight timesteps, whole and ragged, T long
