@@ -473,10 +473,10 @@ cudaError_t of_launch_first_scans(OfScanPlan plan, const void *scores, float *bw
     if (plan == OfScanPlan::kWarps && N > 8 * sms)
         return of_launch_warp_backward(scores, bwd, T, N, stay, tables, status, wait_ns, stream);
     float *fwd = plan == OfScanPlan::kTogether ? post : nullptr;
-    // (five chunks of 256 states to the SM: the shorter groups pay once the first timesteps are a small part.  Decodes with
-    // this kernel / scan.cu's: T = 100, 593 chunks 0.426 / 0.409 ms; 200, 680 chunks 0.719 / 0.710; 300 0.941 / 0.947; 400
-    // 1.154 / 1.173)
-    const bool early = state_len == 4 && N > 4 * sms && T < 250;
+    // (five chunks of 256 states to the SM, a few timesteps: all of them by the exact routine, at which scan.cu's kernel is no
+    // slower.  Decodes with this file's kernel / scan.cu's, 593 and 740 chunks: T = 60 0.287 / 0.288 and 0.321 / 0.313 ms; 100
+    // 0.406 / 0.412 and 0.446 / 0.446; 200 0.637 / 0.672 and 0.710 / 0.726)
+    const bool early = state_len == 4 && N > 4 * sms && T < 100;
     if (plan == OfScanPlan::kBackwardThenForward || state_len == 5 || early)
         return of_launch_scans(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);
     return of_launch_ahead(scores, bwd, fwd, T, N, state_len, sms, stay, tables, status, wait_ns, stream);

@@ -229,7 +229,7 @@ def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod,
                                     (3, 13, 1184), (3, 9, 1185), (3, 120, 1186), (4, 5, 76), (4, 300, 148), (4, 701, 75), (4, 13, 222),
                                     (4, 1101, 223), (4, 9, 296), (4, 4, 446), (4, 300, 448), (4, 7, 592), (4, 300, 594), (4, 3, 740), (4, 5, 741), (4, 5, 1776), (4, 4, 1777),
                                     (3, 993, 149), (3, 994, 149), (3, 501, 296), (4, 600, 148), (4, 601, 148), (4, 1186, 75), (4, 1333, 222),
-                                    (4, 1334, 222), (4, 1001, 296), (4, 249, 593), (4, 250, 593)])
+                                    (4, 1334, 222), (4, 1001, 296), (4, 99, 593), (4, 100, 593)])
 def test_scans_that_run_ahead_by_chunks_to_the_multiprocessor(native_lib, oracle_mod, sl, T, N):
     # which scans of a batch run ahead of their checks, and with what blocks, hangs on the chunks to the
     # multiprocessor and on T; T whole and ragged in groups of three, four and six timesteps
