@@ -171,6 +171,27 @@ def test_an_infinite_score_is_taken_alike_by_every_scan_kernel_and_at_a_bearable
     assert few < 2.2 * scans(sc)[0]
 
 
+@pytest.mark.parametrize("sl,T,many", [(3, 1500, 160), (3, 300, 760), (3, 300, 1200), (4, 300, 600), (4, 300, 800), (4, 300, 1800),
+                                       (5, 200, 120), (5, 200, 232), (5, 200, 300)])
+def test_an_infinite_score_leaves_the_same_bits_in_every_block_shape(native_lib, sl, T, many):
+    # few chunks against batches that go to the other kernels and to the other shapes of their blocks
+    import torch
+    from openfish_b200 import synth
+    of = native_lib
+    sc = torch.from_numpy(synth.make_scores(T, 4, sl, 93)).cuda()
+    sc[T // 2, :, 7] = float("inf")
+
+    def bits(scores):
+        gb = of.gpubuf_init(T, scores.shape[1], sl)
+        of.decode_gpu(scores, sl, gpubuf=gb)
+        got = [gb.tensor(n)[-4:].contiguous().view(torch.int32).cpu().numpy() for n in ("bwd_NTC", "post_NTC")]
+        gb.free()
+        return got
+
+    few, tiled = bits(sc), bits(sc.repeat(1, many // 4, 1).contiguous())
+    assert all(np.array_equal(a, b) for a, b in zip(few, tiled))
+
+
 def test_rows_that_turn_infinite_are_taken_again_at_once(native_lib):
     # a group in which the rows turn infinite has more guesses than its check can be about; the scans of 14 chunks take
     # 1.47 times as long as with ordinary scores (half of the timesteps by the exact routine), 1.85 times while every one of
@@ -219,8 +240,8 @@ def test_scores_that_grow_slowly_cost_little_more(native_lib):
 
 @pytest.mark.parametrize("T,N", [(1, 445), (7, 445), (8, 446), (9, 447), (16, 445), (23, 1000), (400, 445)])
 def test_batches_whose_chunks_are_scanned_by_a_warp_each(native_lib, oracle_mod, T, N):
-    # 64 states, more than three chunks to the multiprocessor: groups of eight timesteps, whole and ragged, T long
-    # enough for guesses to be made and to be wrong
+    # 64 states, more than three chunks to the multiprocessor (up to eight: the forward scan only): groups of eight
+    # timesteps, whole and ragged, T long enough for guesses to be made and to be wrong
     from openfish_b200 import synth
     check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 500 + T, p_step=0.6), 3, min_identical=1.0)
 
@@ -235,6 +256,49 @@ def test_scans_that_run_ahead_by_chunks_to_the_multiprocessor(native_lib, oracle
     # multiprocessor and on T; T whole and ragged in groups of three, four and six timesteps
     from openfish_b200 import synth
     check(native_lib, oracle_mod, synth.make_scores(T, N, sl, 800 + T, p_step=0.6), sl, min_identical=1.0)
+
+
+# (scale, shift, p_step, options): ordinary scores; paths that grow slowly, so that guesses are many for most of the
+# timesteps and often wrong, several to a group; large scores; falling ones; tiny ones, never out of the exact routine
+SCORE_KINDS = [(1.0, 0.0, 0.6, dict(blank_score=0.7)), (0.3, -3.0, 0.3, dict()), (2.0, -1.0, 0.5, dict(blank_score=3.5, beam_cut=20.0)),
+               (8.0, 0.0, 1.0, dict()), (1.0, -12.0, 0.6, dict(temperature=0.9)), (0.05, 0.0, 0.6, dict(blank_score=-0.5))]
+
+
+@pytest.mark.parametrize("sl,T,N", [(3, 300, 150), (3, 300, 300), (3, 260, 450), (3, 260, 760), (3, 300, 1200), (4, 260, 90), (4, 260, 190),
+                                    (4, 260, 310), (4, 300, 460), (4, 300, 610), (4, 260, 760), (4, 260, 1790), (5, 150, 120),
+                                    (5, 150, 230), (5, 150, 300)])
+def test_kinds_of_scores_in_every_block_shape(native_lib, oracle_mod, sl, T, N):
+    # a batch of ten chunks (four of 1024 states) over and over: every copy's backward scores are the oracle's, the
+    # first and the last in full
+    import torch
+    from openfish_b200 import synth
+    of, oracle = native_lib, oracle_mod
+    flags = oracle.SCAN_STAY_FROM_OPTIONS | oracle.TEMPERATURE_SCALES_SCORES
+    few = 10 if sl < 5 else 4
+    for kind, (scale, shift, p_step, okw) in enumerate(SCORE_KINDS):
+        sc = (synth.make_scores(T, few, sl, 700 + 10 * kind + sl, p_step=p_step).astype(np.float32) * scale + shift).astype(np.float16)
+        ref = oracle.decode(sc.astype(np.float32), sl, oracle.decoder_init(**okw), nthreads=10, tensors=True, flags=flags)
+        copies = -(-N // few)
+        gb = of.gpubuf_init(T, few * copies, sl)
+        out = of.decode_gpu(torch.from_numpy(sc).cuda().repeat(1, copies, 1).contiguous(), sl, options=of.decoder_init(**okw), gpubuf=gb)
+        want = torch.from_numpy(ref["bwd"]).cuda()
+        bwd = gb.tensor("bwd_NTC").view(copies, few, T + 1, 4 ** sl)
+        differ = [i for i in range(copies) if not torch.equal(bwd[i], want)]
+        assert not differ, (kind, differ)
+        names = (("bwd", "bwd_NTC"), ("post", "post_NTC"), ("qual", "qual_data"), ("states", "states"),
+                 ("base_probs", "base_probs"), ("total_probs", "total_probs"))
+        for part in (slice(0, few), slice(-few, None)):
+            got = {k: out[k][part] for k in ("moves", "sequence", "qstring")}
+            got.update({k: gb.tensor(n)[part].cpu().numpy() for k, n in names})
+            assert_parity(compare(got, ref), min_identical=1.0)
+        gb.free()
+
+
+@pytest.mark.parametrize("T,N", [(1, 1185), (7, 1186), (8, 1185), (16, 1187), (17, 1185), (23, 1200)])
+def test_backward_scans_by_a_warp_each(native_lib, oracle_mod, T, N):
+    # more than eight chunks of 64 states to the multiprocessor: groups of eight timesteps, whole and ragged
+    from openfish_b200 import synth
+    check(native_lib, oracle_mod, synth.make_scores(T, N, 3, 520 + T, p_step=0.6), 3, min_identical=1.0)
 
 
 @pytest.mark.parametrize("sl,T", [(3, 11), (3, 12), (4, 13), (4, 24), (4, 25), (3, 37), (5, 4), (5, 5), (5, 6), (5, 11)])
