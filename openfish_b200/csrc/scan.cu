@@ -652,7 +652,7 @@ using Spec1024Many = Spec<1024, 4, 4, 4, 3, kBackward | kForward>;
 using SpecPosterior256 = SpecPosterior<256, 4, 6, 16, 5>;
 using SpecPosterior256Many = SpecPosterior<256, 4, 6, 4, 5>;
 using SpecPosterior256Most = SpecPosterior<256, 4, 6, 4, 6>;
-using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 8, 2>;
+using SpecPosterior1024 = SpecPosterior<1024, 4, 6, 8, 2>;  // (16 copies of the table: no difference)
 using SpecPosterior1024Many = SpecPosterior<1024, 4, 3, 4, 3>;
 
 }  // namespace

@@ -13,13 +13,16 @@ namespace ofx { struct Tables; }
 // How the scans of a batch are best run.
 enum class OfScanPlan {
     kTogether,           // both in one launch, the posterior by a kernel of its own
-    kAheadThenForward,   // the backward one by of_launch_ahead, the forward one afterwards (beside the beam search)
+    kAheadThenForward,   // the backward one by of_launch_ahead (with few timesteps, of five chunks to the multiprocessor, by
+                         // scan.cu's kernel), the forward one afterwards, beside the beam search, by either file's
     kBackwardThenForward,// both by scan.cu's kernels
-    kWarps               // both by scan_warp.cu's kernels, a warp to a chunk (the 64-state model)
+    kWarps               // the 64-state model: the forward one by scan_warp.cu's kernel, a warp to a chunk; the backward one by
+                         // of_launch_ahead, and in batches of more than eight chunks to the multiprocessor by a warp to a chunk
 };
 OfScanPlan of_scan_plan(int N, int state_len, int sms);
 
-// One or both scans (bwd or fwd null: not that direction) by the kernel for batches that fill the GPU.  (scan.cu)
+// One or both scans (bwd or fwd null: not that direction) by the kernel for batches that fill the GPU: 64 states
+// forwards only, 256 states backwards only.  (scan.cu)
 cudaError_t of_launch_scans(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, int sms,
                             float stay, const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream);
 
@@ -29,8 +32,7 @@ cudaError_t of_launch_forward_posterior(const void *scores_fp16, const float *bw
                                         int state_len, int sms, float stay, const ofx::Tables *tables, int *status,
                                         uint64_t wait_ns, cudaStream_t stream);
 
-// One or both scans by the kernel for batches that leave the GPU room, for the 64- and the 256-state
-// model.  (scan_ahead.cu)
+// One or both scans by the kernel that runs ahead of its checks, for the 64- and the 256-state model.  (scan_ahead.cu)
 cudaError_t of_launch_ahead(const void *scores_fp16, float *bwd, float *fwd, int T, int N, int state_len, int sms, float stay,
                             const ofx::Tables *tables, int *status, uint64_t wait_ns, cudaStream_t stream);
 

@@ -1,10 +1,11 @@
-// scan_ahead.cu -- the two scans of a small batch, side by side, for sm_100a.
+// scan_ahead.cu -- scans that run ahead of their checks, for the 64- and the 256-state model, for sm_100a.
 //
-// Same recursions and, value for value, the same results as scan.cu (src/decode_cpu.c:13-52, 54-119),
-// arranged for the case in which a GPU has fewer chunks than it could hold and a batch lasts as long as
-// one chunk's chain of T dependent timesteps.  One launch takes both directions (a block each for the
-// backward and the forward scan of a chunk; they do not depend on each other), the forward rows go to
-// HBM, and the posterior is formed by a kernel of its own while the beam search runs.
+// Same recursions and, value for value, the same results as scan.cu (src/decode_cpu.c:13-52, 54-119), for batches
+// that last as long as a chunk's chain of T dependent timesteps: up to five chunks of 256 states and eight of 64 to
+// the SM.  While blocks have SMs to themselves one launch takes both directions (a block each for the backward and
+// the forward scan of a chunk; they do not depend on each other); in larger batches it takes the backward scan,
+// and in some of them the forward scan beside the beam search.  The forward rows go to HBM, and the posterior is formed by
+// a kernel of its own.
 //
 // A state whose rounding the fp32 evaluation cannot certify (two or three of a row's 256, once the
 // scores have grown) needs the value-exact routine, a chain of some 450 cycles on its own.  The scan
@@ -59,8 +60,10 @@ struct AheadSmem {
 };
 
 // Rounds of up to 64 marked states that a group's check goes through; with more the group is taken again exactly by
-// the scan warps, which is 32 times as many hands.  Ordinary groups stay below two (a state in fourteen when guesses
-// begin); it is for rows that turn infinite, whose first state, by which exact_for_all judges, is still finite.
+// the scan warps, which have a lane to two or four states.  Ordinary groups stay below four (FROM, below, says how many
+// states are marked when guesses begin); it is for rows that turn infinite, whose first state, by which
+// exact_for_all judges, is still finite: scans of 14 chunks of 256 states, T = 1000, infinite half way, 0.489 ms instead
+// of 0.610.
 constexpr int kRounds = 5;
 
 template <int ID, int THREADS>

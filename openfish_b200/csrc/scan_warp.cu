@@ -13,10 +13,11 @@
 // What bounds it: in a batch that fills the GPU, instructions.  Gone is what the kernels for fewer chunks spend so
 // that a timestep is short: a checker's pass over a nearly empty list every timestep or two (one pass for eight
 // here), barriers and votes, a copy warp's polling, and for the posterior a forward row that goes to HBM and back
-// and a reduction over 32 lanes (four lanes to a row here).  A chunk alone takes longer than with those.  Decodes
-// of T = 1666: 1024 chunks 2.22 ms instead of 2.58 (backward scan 0.74 instead of 0.86, forward scan and posterior
-// beside the beam search 1.29 instead of 1.54), 4096 chunks 6.9 instead of 9.2.  K = 8: with 4 there are twice the
-// passes (4096 chunks: backward scan 2.17 ms instead of 1.84); with 16 a block takes twice the shared memory (forward
+// and a reduction over 32 lanes (four lanes to a row here).  A chunk alone takes longer than with those, and the
+// backward scan does up to eight chunks to the SM (scan_ahead.cu: 1024 chunks of T = 1666 0.57 ms instead of 0.74).  Beside
+// the beam search, with the posterior, T = 1666: 1024 chunks 1.31 ms instead of scan_ahead.cu's 1.72, 4096 4.71; backward scan of
+// 4096 chunks 1.83 ms.  (The kernel before it, scan.cu's with a posterior kernel: 1.54 for 1024.)  K = 8: with 4 there are
+// twice the passes (4096 chunks: backward scan 2.17 ms instead of 1.84); with 16 a block takes twice the shared memory (forward
 // scan of 4096 chunks beside the beam search 5.4 ms instead of 4.7).
 #include "exact_math.cuh"
 #include "fast_lse.cuh"
@@ -176,7 +177,8 @@ scan_warp_kernel(const __half *__restrict__ scores, float *__restrict__ out, con
             }
             // The marked states, 32 at a time.  A value put right here may be one that a later entry reads, or that
             // was itself worked out from a wrong one: both lie behind the first wrong timestep, from which on all
-            // is taken again.
+            // is taken again.  (scan_ahead.cu's checker deals its marks out the same way.  As a function that both call the
+            // compiler lays 64-state scan_ahead's code out so that 300 to 444 chunks take 5 % longer.)
             int first_wrong = K;
             for (uint32_t owners = __ballot_sync(0xffffffffu, mask != 0); owners;) {
                 int count = 0;
