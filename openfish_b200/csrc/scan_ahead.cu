@@ -338,7 +338,7 @@ struct Ahead {
 // Longer groups: what a group costs besides its timesteps (250 cycles, and the checker's pass) is paid less often, and
 // going back, rare and short, loses less than that.  One checker for a group instead of one for each of its
 // timesteps, whose lists were nearly empty: both scans of one chunk of 64 states, T = 1000, 0.256 ms instead of 0.280
-// (groups of four), 0.246 with groups of six; of 14 chunks of 256 states, T = 1666, 0.560 instead of 0.572; the backward
+// (groups of four), 0.246 with groups of six (0.236 by now); of 14 chunks of 256 states, T = 1666, 0.560 instead of 0.572 (0.51 by now); the backward
 // scan of 300 chunks 0.766 instead of 0.874.  (Groups of two with a checker for each timestep, and wrong guesses
 // gone back to and taken again instead of put right: 0.345, 0.642, 0.979.)  Five stages of 256 states, so that three
 // blocks fit an SM; four come too late (14 chunks 0.844).

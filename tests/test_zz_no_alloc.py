@@ -35,6 +35,16 @@ def test_static_scratch_decode_matches_regular_decode_twice_in_a_row(native_lib)
             assert np.array_equal(want[k], got[k]), (sl, T, N, k)
 
 
+@pytest.mark.parametrize("sl,T,N", [(3, 40, 150), (3, 40, 500), (3, 33, 1200), (4, 40, 150), (4, 40, 460), (4, 28, 610), (4, 25, 760)])
+def test_static_scratch_decode_of_batches_that_take_the_other_kernels(native_lib, sl, T, N):
+    # scores of 40 to 120 a timestep, so that guesses are made within these few
+    from openfish_b200 import synth
+    sc = (synth.make_scores(T, N, sl, 30 + N, p_step=0.7).astype(np.float32) * 8 + 30).astype(np.float16)
+    want, got = both_ways(native_lib, sc, sl, {})
+    for k in want:
+        assert np.array_equal(want[k], got[k]), k
+
+
 def test_static_scratch_decode_against_the_oracle_and_without_allocating(native_lib, oracle_mod):
     import torch
     from openfish_b200 import synth
